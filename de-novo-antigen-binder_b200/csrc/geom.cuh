@@ -206,7 +206,7 @@ __device__ __forceinline__ bool cg_term(const CgB& b, const float4 apq, const fl
 // compute_forces_with_grid for one body: the 27 cells in the reference's order,
 // one sequential f32 sum.
 template <bool COUNT = false>
-__device__ __forceinline__ void cg_force(const AgView& A, const CgB& b, float& fx, float& fy, float& fz,
+__device__ __noinline__ void cg_force(const AgView& A, const CgB& b, float& fx, float& fy, float& fz,
                                          int* n_pairs = nullptr) {
     const GridView& g = A.ca_grid;
     const int cx = cell_coord(b.x, g.inv), cy = cell_coord(b.y, g.inv), cz = cell_coord(b.z, g.inv);

@@ -4,33 +4,48 @@
 //
 // Per step, in the reference's order:
 //  1. Langevin: coarse-grained force, restraint, noise, 2 A clamp, rigid
-//     translation (diffusion.rs:306-339).  A residue's force comes from its Verlet
-//     list (8 lanes per residue, 16 in the 16-warp instance), whose in-cutoff
-//     entries in list order are the reference's pairs in its order; its lane 0
-//     adds their terms in that order, which is the reference's sequential sum.
-//     Candidates too long for lists: eight lanes per residue split the 27 probe
-//     cells (reference order) into consecutive runs and lane 0 adds the runs'
-//     terms lane by lane.
-//  2. Interface mask: any antigen Calpha within sqrt(iface_cutoff_sq) (:343-351).
-//  3. Mutation / rotamer sweep (:354-399).  A move at residue r changes only
+//     translation (diffusion.rs:306-339), then the interface test (any antigen
+//     Calpha within sqrt(iface_cutoff_sq), :343-351) and the residue's mutation /
+//     rotamer draw, all by one group of GL lanes per residue.  The force comes from
+//     the residue's Verlet list: its in-cutoff entries in list order are the
+//     reference's pairs in its order; the group compacts them, evaluates one pair per
+//     lane and folds the terms in that order by shuffles -- the reference's
+//     sequential sum, held by every lane.  Meanwhile idle warps draw the backbone
+//     moves.
+//  2. Mutation / rotamer sweep (:354-399).  A move at residue r changes only
 //     residue r's atoms, and the Calpha-level energy of r depends only on r's
 //     Calpha and amino acid; residues interact only through the disulfide term.
-//     So every residue's proposal, its rejection rebuild and both Calpha energies
-//     are computed in parallel (builds on one half of the warps, energies on the
-//     other); one thread takes the decisions that involve a Cys in residue order,
-//     updating the disulfide energy, and records the disulfide energy current at
-//     every other move's turn; those moves, which leave it unchanged, are then
-//     decided in parallel — the reference's sequential sweep, exactly.
-//  4. Backbone phi/psi sweep (:403-418): sequential over the attempted moves;
-//     per move the Calpha energies of residues r..n are evaluated by warps, the
-//     downstream atoms rotated by all threads (Rodrigues, allatom.rs:397-479), and
-//     the decision broadcast; a rejected move is undone by the opposite rotation,
-//     as in the reference.
-// Calpha energies are cached per residue and recomputed whenever the Calpha moved.
+//     So every proposal, its rejection rebuild and both Calpha energies are computed
+//     in parallel (builds on the last warps, energies on the others, together with
+//     the energies the first backbone move starts from); then warp 0 decides: the
+//     moves that involve a Cys in residue order, updating the disulfide energy, the
+//     others -- which leave it unchanged -- each by a lane with the disulfide energy
+//     of its turn: the reference's sequential sweep, exactly.
+//  3. Backbone phi/psi sweep (:403-418): sequential over the attempted moves;
+//     per move the downstream atoms rotated by all threads (Rodrigues,
+//     allatom.rs:397-479), the Calpha energies of residues r+1..n by all warps, the
+//     decision by warp 0; a rejected move is undone by the opposite rotation, as in
+//     the reference, and the energies it disturbed are recomputed only if another
+//     move follows in the same step.
 //
-// Accumulation: ACC = float reproduces the reference's f32 sums bit for bit; ACC =
-// double sums the same f32 pair terms in double and takes the Metropolis test on
-// the double energy difference.
+// What bounds it: the chain of dependent latencies of a step (one candidate's work is
+// tiny), so every phase is arranged to be short and few (three barriers a step, four
+// more per backbone move) and many candidates share an SM.  64 x 20 residues, 300-residue
+// antigen, 600 steps: 13.4 ms before (42 k cycles a step: lane-0 FP64 folds of every
+// energy, one thread scanning for Cys pairs, side chains built from divergent constant
+// tables and local memory, nine barriers), 9.5 ms now; 1024 x 20 residues, 60 steps:
+// 7.9 ms before, 4.2 ms now.  What is left is about 6.5 cycles per dependent instruction
+// (2.5 of fixed latency, 1 of shared memory, 0.8 of branches, 0.6-0.9 of instruction
+// fetch): the code is kept small -- one copy of each exponential, pair term and scan, no
+// unrolling (178 -> 122 KB) -- because several warps in different phases of unrolled code
+// waited for instructions more than for anything else (a 1024-candidate launch 5.5 -> 4.3 ms).
+//
+// Accumulation: ACC = float reproduces the reference's f32 sums bit for bit (terms
+// staged and added in antigen order by one lane); ACC = double sums the same f32 pair
+// terms in double over the lanes of a group and a fixed butterfly, and takes the
+// Metropolis test on the double energy difference.
+#include <type_traits>
+
 #include "cg_list.cuh"
 #include "geom.cuh"
 #include "kernels.h"
@@ -49,145 +64,88 @@ cudaError_t anneal_init_mlp_table(const float* t) {
 
 constexpr int AN_WARPS = 8;
 constexpr int AN_THREADS = AN_WARPS * 32;
-constexpr int CG_LANES = 8;                          // lanes per residue in the Langevin probe
-constexpr int CG_RES_PER_PASS = AN_THREADS / CG_LANES;
-constexpr int CG_SLOTS = 16;                         // in-cutoff terms a lane holds
-static_assert(CG_IN_MAX * (16 + 4) <= CG_LANES * CG_SLOTS * 16, "list scratch must fit a group's term slots");
-constexpr int STAGE_CAP = 64;                        // staged in-cutoff terms per warp
+constexpr int STAGE_CAP = 64;                        // staged in-cutoff terms per warp (ACC = float)
+constexpr int HIT_CAP = 96;                          // in-cutoff entries a warp's scan holds (ACC = double)
+constexpr int EL = 8;                                // lanes per Calpha energy (ACC = double)
+constexpr int MASK_WORDS = ANNEAL_MAX_RES / 32;      // residue bit masks of a candidate
+constexpr int AN_IN = 32;                            // in-cutoff entries of the force a residue holds per round
+constexpr int SC_MAX = 9;                            // side-chain atoms of a residue program
 constexpr int AG_STAGE_MAX = 1024;                   // antigen Calphas staged in shared memory
 constexpr int CELL_STAGE_MAX = 4096;                 // Calpha-grid cells staged in shared memory
 enum : int { MV_NONE = 0, MV_ROT = 1, MV_MUT = 2 };
-enum : int { SEL_KEEP = 0, SEL_PROP = 1, SEL_REJ = 2 };
-enum : int { IS_DVALID = 0, IS_DECISION = 1, IS_NCYS = 2, IS_LASTCYS = 3, IS_NMV = 4, IS_NTASK = 5 };
+enum : int { SEL_KEEP = 0, SEL_PROP = 1, SEL_REJ = 2, SEL_SIDE = 4 };  // SEL_SIDE: only the side chain was built
+enum : int { IS_DVALID = 0, IS_DECISION = 1, IS_CYSMV = 2, IS_NMV = 4, IS_NTASK = 5 };
 
-// Shared-memory carve of one CTA for candidates of up to R residues and antigens
-// of up to G staged Calphas.
-struct AnSmem {
-    float4 *pos, *prop, *rej;  // R * SLOT_STRIDE each: state, proposal, rejection rebuild
-    float4* trig;              // 2R: sin/cos of chi1..4
-    float4* chi;               // R (degrees)
-    float4* ldelta;            // R: Langevin translation
-    float4* bb_trig;           // R: cos, sin of the torsion step and of its negation
-    float4* terms;             // min(R, 32) * CG_LANES * CG_SLOTS Langevin pair terms; with the learned
-                               // proposal also the network tile (the two are never live together)
-    float4* stage;             // AN_WARPS * STAGE_CAP: in-cutoff Calpha-energy terms
-    float4 *agq, *agp;         // G staged antigen Calphas: x, y, z, q | r_min_half, eps, hyd, type
-    float4 *cgq, *cgp;         // G staged Calphas in CG-grid order (AgView::ca_pq, ca_prm)
-    float *agx, *agy, *agz;    // anneal_xyz_len(G) each: the staged Calphas' x, y, z (pad +1e30)
-    int* cgcell;               // C staged CG-grid cell starts
-    AgView* ag;
-    double *c_cur, *c_old, *c_new;  // R: Calpha energies (exact f32 values when ACC = float)
-    double* dscal;                  // [0] disulfide energy of the current state
-    double* lhr;                    // R: log Hastings ratio of the move (network path)
-    double* d_turn;                 // R: the disulfide energy current at the move's turn (moves
-                                    // without a Cys, decided after the sequential pass)
-    float *u_acc, *bb_u;            // R
-    int *aa, *kind, *new_aa, *new_rot, *sel, *valid, *bb_att, *bb_phi, *iface;
-    int* tcount;                    // L (>= 2R): Langevin term counts of the lanes; after the Langevin step
-                                    // the Calpha-energy tasks of the step's moves, 2 r + (0 before, 1 after)
-    int *rot, *mvl;                 // R: rotamer index of the state (-1 unknown), residues with a move
-    uint32_t* dz;                   // R: the move's choice draw
-    int* iscal;
-    uint8_t* agaa;                  // learned proposal: G staged antigen amino acids
-    float* lg1p;                    // learned proposal: the log1p count table
-    float* mbias;                   // learned proposal: the network's biases b1 | b2 | b3
-    int* cglist;                    // LR x CG_LIST_MAX: Verlet lists of the Langevin force
-    float4* cgcentre;               // LR: list centre, skin
-    int* cgnl;                      // LR: list length (-1: none yet)
-    // Fv two-chain steps: the partner chain's Calphas, as Calpha atoms (ptq, ptp: the
-    // agq / agp layout) and as residue-level bodies of the CG force (pcq, pcp: the
-    // AgView::ca_pq / ca_prm layout); R each
-    float4 *ptq, *ptp, *pcq, *pcp;
+// What the Calpha energies read of the antigen: its Calphas' positions and amino acids
+// in list order (the CG grid's) and in scan order (list order when staged, else residue
+// order, map giving the residue of a list position).
+struct AnEnv {
+    const float4 *lpos, *pos;
+    const uint8_t* aa;
+    const float4* map;  // AgView::ca_prm (w = residue index bits), or null when list order = scan order
+    int n, np;          // antigen Calphas, Fv: partner residues
 };
-// Entries of each staged x / y / z array: room for the pad, a multiple of 4 (the
-// arrays after them keep their 16-byte alignment).
+
+// Fixed part of a CTA's shared memory: candidates of up to RT residues, W warps, ACC
+// double or float (F32), with the learned proposal (LRN) or one chain of an Fv pair
+// (FV).  Everything the step touches lies at a compile-time offset: with offsets read
+// from the parameter bank each first access of a phase waited for a constant load.  The
+// staged antigen follows it (an_tail_bytes).
+template <int RT_, int W_, bool F32_, bool LRN_, bool FV_>
+struct AnSmem {
+    static constexpr int RT = RT_, W = W_;
+    static constexpr bool F32 = F32_, LRN = LRN_, FV = FV_;
+    float4 pos[RT * SLOT_STRIDE], prop[RT * SLOT_STRIDE], rej[RT * SLOT_STRIDE];  // state, proposals, rejections
+    float4 trig[2 * RT];                      // sin/cos of chi1..4
+    float4 chi[RT];                           // degrees
+    float4 bb_trig[RT];                       // cos, sin of the torsion step and of its negation
+    float4 cgcentre[RT];                      // list centre, skin
+    float4 sct[N_AA * SC_MAX];                // bond, sin, cos of the angle, the reference atoms' bits
+    float4 ca_atom[N_AA], res[N_AA];          // Calpha atom: charge, r_min_half, eps, hyd; residue-level parameters
+    float4 stage[F32 ? W * STAGE_CAP : 1];    // F32: in-cutoff Calpha-energy terms
+    float4 ptq[FV ? RT : 1], ptp[FV && F32 ? RT : 1];  // Fv: the partner's Calpha atoms (x, y, z, q | prm)
+    float4 pcq[FV ? RT : 1], pcp[FV ? RT : 1];  // and residue-level bodies (AgView::ca_pq / ca_prm layout)
+    float2 scf[N_AA * SC_MAX];                // sin, cos of the fixed dihedral
+    float2 rott[N_AA * 20 + 4];               // rotamer sin/cos, then 4 x (0, 1)
+    float2 hits[F32 ? 1 : W * HIT_CAP];       // in-cutoff (r^2, index)
+    double c_cur[RT], c_old[RT], c_new[RT];   // Calpha energies (exact f32 values when F32)
+    double lhr[RT];                           // log Hastings ratio of the move (network path)
+    double d_turn[RT];                        // disulfide energy at the move's turn, then (log) its energy change
+    double dscal;                             // disulfide energy of the current state
+    AgView ag;
+    AnEnv env;
+    float u_acc[RT], bb_u[RT];
+    int aa[RT], kind[RT], new_aa[RT], new_rot[RT], sel[RT], bb_phi[RT], cgnl[RT];
+    int task[2 * RT];                         // 2 r + (0 proposal / energy before, 1 rejection / after) of the moves
+    int rot[RT], mvl[RT];                     // rotamer index of the state (-1 unknown), residues with a move
+    uint32_t dz[RT];                          // the move's choice draw
+    int topo_n[N_AA], sc_n[N_AA], rot_n[N_AA], ca_hb[N_AA];
+    unsigned attw[2 * MASK_WORDS];            // backbone attempts (two: a fast warp may draw the next step's
+                                              // while a slow one still reads)
+    unsigned cysw[MASK_WORDS], mxw[MASK_WORDS];  // Cys residues, moves that involve a Cys
+    int iscal[8];
+    float lg1p[LRN ? MLP_COUNT_CAP + 1 : 1];  // the log1p count table
+    float mbias[LRN ? MLP_BIASES : 1];        // the network's biases b1 | b2 | b3
+    __align__(16) unsigned char tile[LRN ? MT_BYTES : 16];  // the network tile
+    __align__(16) uint16_t cglist[RT * CG_LIST_MAX];  // Verlet lists of the Langevin force
+    uint8_t ptaa[RT];
+};
+// Entries of each staged x / y / z array: room for the pad, a multiple of 4.
 __host__ __device__ inline int anneal_xyz_len(int G) { return G > 0 ? (G + 4) & ~3 : 0; }
-static_assert(32 * CG_LANES >= 2 * ANNEAL_MAX_RES, "the term counts hold two energy tasks per residue");
-// Residues with Verlet lists in shared memory: candidates of up to one Langevin
-// pass (CG_RES_PER_PASS residues); longer ones walk the 27 cells every step.
-__host__ __device__ inline int anneal_list_res(int R) { return R <= CG_RES_PER_PASS ? R : 0; }
-__host__ __device__ inline size_t anneal_terms_bytes(int R, int learned) {
-    const int L = (R < CG_RES_PER_PASS ? R : CG_RES_PER_PASS) * CG_LANES;
-    const size_t t = (size_t)L * CG_SLOTS * 16;
-    return learned && t < (size_t)MT_BYTES ? (size_t)MT_BYTES : t;
+// The staged antigen: Calphas in CG-grid order (x, y, z, residue charge | residue-level
+// epsilon, sigma, hydrophobic), F32 also the Calpha atoms in residue order (x, y, z, q |
+// prm; x, y, z arrays), cell starts, amino acids in grid order.
+__host__ __device__ inline size_t an_tail_bytes(int G, int C, bool f32) {
+    return (size_t)G * (f32 ? 64 : 32) + (f32 ? (size_t)anneal_xyz_len(G) * 12 : 0) + (size_t)C * 4 + (size_t)G;
 }
-__host__ __device__ inline size_t anneal_smem_bytes(int R, int G, int C, int learned, int fv = 0,
-                                                    int warps = AN_WARPS) {
-    const int L = (R < CG_RES_PER_PASS ? R : CG_RES_PER_PASS) * CG_LANES;
-    return (size_t)R * SLOT_STRIDE * 16 * 3 + (size_t)R * 16 * 5 + anneal_terms_bytes(R, learned) +
-           (size_t)warps * STAGE_CAP * 16 + (size_t)G * 64 + (size_t)anneal_xyz_len(G) * 12 +
-           ((size_t)C * 4 + 15) / 16 * 16 +
-           ((sizeof(AgView) + 15) / 16) * 16 +
-           (size_t)R * 8 * 3 + 16 + (size_t)R * 8 * 2 + (size_t)R * 4 * 2 + (size_t)R * 4 * 9 + (size_t)L * 4 +
-           (size_t)R * 4 * 3 + 32 + (learned ? ((size_t)G + 15) / 16 * 16 + (MLP_COUNT_CAP + 1 + MLP_BIASES) * 4 : 0) +
-           15 + (size_t)anneal_list_res(R) * (CG_LIST_MAX * 4 + 16 + 4) +  // 15: alignment of cgcentre
-           (fv ? 15 + (size_t)R * 64 : 0);
-}
-__device__ inline AnSmem carve(unsigned char* b, int R, int G, int C, int learned, int fv = 0, int warps = AN_WARPS) {
-    AnSmem s;
-    const int L = min(R, CG_RES_PER_PASS) * CG_LANES;
-    auto take = [&](size_t bytes) { unsigned char* p = b; b += bytes; return p; };
-    s.pos = (float4*)take((size_t)R * SLOT_STRIDE * 16);
-    s.prop = (float4*)take((size_t)R * SLOT_STRIDE * 16);
-    s.rej = (float4*)take((size_t)R * SLOT_STRIDE * 16);
-    s.trig = (float4*)take((size_t)R * 32);
-    s.chi = (float4*)take((size_t)R * 16);
-    s.ldelta = (float4*)take((size_t)R * 16);
-    s.bb_trig = (float4*)take((size_t)R * 16);
-    s.terms = (float4*)take(anneal_terms_bytes(R, learned));
-    s.stage = (float4*)take((size_t)warps * STAGE_CAP * 16);
-    s.agq = (float4*)take((size_t)G * 16);
-    s.agp = (float4*)take((size_t)G * 16);
-    s.cgq = (float4*)take((size_t)G * 16);
-    s.cgp = (float4*)take((size_t)G * 16);
-    s.agx = (float*)take((size_t)anneal_xyz_len(G) * 4);
-    s.agy = (float*)take((size_t)anneal_xyz_len(G) * 4);
-    s.agz = (float*)take((size_t)anneal_xyz_len(G) * 4);
-    s.cgcell = (int*)take(((size_t)C * 4 + 15) / 16 * 16);
-    s.ag = (AgView*)take(((sizeof(AgView) + 15) / 16) * 16);
-    s.c_cur = (double*)take((size_t)R * 8);
-    s.c_old = (double*)take((size_t)R * 8);
-    s.c_new = (double*)take((size_t)R * 8);
-    s.dscal = (double*)take(16);
-    s.lhr = (double*)take((size_t)R * 8);
-    s.d_turn = (double*)take((size_t)R * 8);
-    s.u_acc = (float*)take((size_t)R * 4);
-    s.bb_u = (float*)take((size_t)R * 4);
-    s.aa = (int*)take((size_t)R * 4);
-    s.kind = (int*)take((size_t)R * 4);
-    s.new_aa = (int*)take((size_t)R * 4);
-    s.new_rot = (int*)take((size_t)R * 4);
-    s.sel = (int*)take((size_t)R * 4);
-    s.valid = (int*)take((size_t)R * 4);
-    s.bb_att = (int*)take((size_t)R * 4);
-    s.bb_phi = (int*)take((size_t)R * 4);
-    s.iface = (int*)take((size_t)R * 4);
-    s.tcount = (int*)take((size_t)L * 4);
-    s.rot = (int*)take((size_t)R * 4);
-    s.mvl = (int*)take((size_t)R * 4);
-    s.dz = (uint32_t*)take((size_t)R * 4);
-    s.iscal = (int*)take(32);
-    s.agaa = learned ? (uint8_t*)take(((size_t)G + 15) / 16 * 16) : nullptr;
-    s.lg1p = learned ? (float*)take((MLP_COUNT_CAP + 1) * 4) : nullptr;
-    s.mbias = learned ? (float*)take(MLP_BIASES * 4) : nullptr;
-    const int LR = anneal_list_res(R);
-    b = (unsigned char*)(((uintptr_t)b + 15) & ~(uintptr_t)15);  // float4 alignment (the arrays before: ints)
-    s.cgcentre = (float4*)take((size_t)LR * 16);
-    s.cglist = (int*)take((size_t)LR * CG_LIST_MAX * 4);
-    s.cgnl = (int*)take((size_t)LR * 4);
-    s.ptq = s.ptp = s.pcq = s.pcp = nullptr;
-    if (fv) {
-        b = (unsigned char*)(((uintptr_t)b + 15) & ~(uintptr_t)15);
-        s.ptq = (float4*)take((size_t)R * 16);
-        s.ptp = (float4*)take((size_t)R * 16);
-        s.pcq = (float4*)take((size_t)R * 16);
-        s.pcp = (float4*)take((size_t)R * 16);
-    }
-    return s;
+template <class L>
+__device__ __forceinline__ L& an_smem() {
+    extern __shared__ __align__(16) unsigned char an_smem_raw[];
+    return *reinterpret_cast<L*>(an_smem_raw);
 }
 
 // hbond_energy (energy.rs:32-39) with the Metropolis-path exponential
-__device__ __forceinline__ float hbond_mc(float r_sq) {
+__device__ __noinline__ float hbond_mc(float r_sq) {
     if (r_sq > HB_CUTOFF_SQ) return 0.0f;
     const float r = xsqrt(r_sq);
     const float z = xdiv(xsub(r, HB_R0), HB_SIGMA);
@@ -327,62 +285,162 @@ __device__ __noinline__ ACC warp_contribution_pairs(const float* __restrict__ ax
     return e;
 }
 
-// Slots of residue j as the sweep currently sees them: its proposal when accepted
-// this sweep, its rejection rebuild when rejected, else the state.
-__device__ __forceinline__ const float4* cur_slots(const AnSmem& S, int j) {
-    const int s = S.sel[j];
-    return (s == SEL_PROP ? S.prop : (s == SEL_REJ ? S.rej : S.pos)) + (size_t)j * SLOT_STRIDE;
-}
-
-// disulfide_energy (allatom.rs:155-180) over the SG atoms (topology atom 5 of Cys)
-// in residue order.  SWEEP: residues take their slots from cur_slots and residue
-// `sub` (>= 0) is taken from `sub_slots` with amino acid `sub_aa` instead; else
-// every residue is read from the state.
-template <class ACC, bool SWEEP>
-__device__ ACC disulfide_of(const AnSmem& S, int n, int sub, const float4* sub_slots, int sub_aa) {
-    ACC e = 0;
-    for (int i = 0; i < n; ++i) {
-        const int ai = (SWEEP && i == sub) ? sub_aa : S.aa[i];
-        if (ai != CYS) continue;
-        const float4 pi = (SWEEP ? (i == sub ? sub_slots : cur_slots(S, i)) : S.pos + (size_t)i * SLOT_STRIDE)[5];
-        for (int j = i + 1; j < n; ++j) {
-            const int aj = (SWEEP && j == sub) ? sub_aa : S.aa[j];
-            if (aj != CYS) continue;
-            const float4 pj = (SWEEP ? (j == sub ? sub_slots : cur_slots(S, j)) : S.pos + (size_t)j * SLOT_STRIDE)[5];
-            const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
-            if (d > 4.0f) continue;
-            const float z = xdiv(xsub(d, 2.05f), 0.4f);
-            e -= (ACC)xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z)));
-        }
-    }
+// residue_contribution_allatom summed in double, order free: the pair of two Calphas
+// within the cutoff, of amino acids with the Calpha atoms a and b (charge, r_min_half,
+// eps, hyd) and H-bond roles -- ca_pair_terms' operations.
+__device__ __noinline__ double ca_pair_sum(const float4 b, int bhb, const float4 a, int ahb, float r_sq) {
+    const float r_ij = xadd(b.y, a.y);
+    const float eps = xsqrt(xmul(b.z, a.z));
+    const float r2 = xdiv(xmul(r_ij, r_ij), r_sq);
+    const float r6 = xmul(xmul(r2, r2), r2);
+    double e = (double)xmul(eps, xsub(xmul(r6, r6), xmul(2.0f, r6)));
+    if (b.x != 0.0f && a.x != 0.0f) e += (double)xdiv(xmul(xmul(COULOMB_K, b.x), a.x), xsqrt(r_sq));
+    if (b.w == 1.0f && a.w == 1.0f && r_sq < HYDRO_CUTOFF_SQ) e -= 0.5;
+    if (((bhb & 1) && (ahb & 2)) || ((bhb & 2) && (ahb & 1))) e += (double)hbond_mc(r_sq);
     return e;
 }
 
-// Metropolis criterion (diffusion.rs:368, 385, 414-415)
-__device__ __forceinline__ bool metropolis(float de, float temp, float u) {
-    return de <= 0.0f || u < mc_exp(xdiv(-de, temp));
+// Calpha energy of a Calpha at `ca` of amino acid `aa` against the scan-order Calphas,
+// in double, by one warp: two tests per lane and step, the in-cutoff ones queued and
+// their terms evaluated 32 at a time, the lanes' sums added by a butterfly (every lane
+// holds the result).
+template <class L>
+__device__ __noinline__ double warp_scan_energy(F3 ca, int aa, float2* hits) {
+    L& S = an_smem<L>();
+    const float4* pos = S.env.pos;
+    const uint8_t* ag_aa = S.env.aa;
+    const int n = S.env.n, lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const float4 b = S.ca_atom[aa];
+    const int bhb = S.ca_hb[aa];
+    double e = 0.0;
+    int cnt = 0;
+#pragma unroll 1
+    for (int base = 0; base < n; base += 64) {
+        const int i0 = base + lane, i1 = i0 + 32;
+        const float4 a0 = pos[min(i0, n - 1)], a1 = pos[min(i1, n - 1)];
+        const float r0 = xdist2(xsub(ca.x, a0.x), xsub(ca.y, a0.y), xsub(ca.z, a0.z));
+        const float r1 = xdist2(xsub(ca.x, a1.x), xsub(ca.y, a1.y), xsub(ca.z, a1.z));
+        const bool in0 = i0 < n && !(r0 > CUTOFF_SQ || r0 < MIN_R_SQ);
+        const bool in1 = i1 < n && !(r1 > CUTOFF_SQ || r1 < MIN_R_SQ);
+        const unsigned m0 = __ballot_sync(0xffffffffu, in0), m1 = __ballot_sync(0xffffffffu, in1);
+        const int c0 = cnt + __popc(m0);
+        if (in0) hits[cnt + __popc(m0 & lt)] = make_float2(r0, __int_as_float(i0));
+        if (in1) hits[c0 + __popc(m1 & lt)] = make_float2(r1, __int_as_float(i1));
+        cnt = c0 + __popc(m1);
+        if (cnt > 32 || base + 64 >= n) {  // room for the next step's 64, or the end
+            __syncwarp();
+#pragma unroll 1
+            do {
+                const int k = max(cnt - 32, 0) + lane;
+                if (k < cnt) {
+                    const float2 h = hits[k];
+                    const int t = ag_aa[__float_as_int(h.y)];
+                    e += ca_pair_sum(b, bhb, S.ca_atom[t], S.ca_hb[t], h.x);
+                }
+                cnt = max(cnt - 32, 0);
+            } while (cnt > 32 || (cnt > 0 && base + 64 >= n));
+            __syncwarp();
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    return e;
 }
-__device__ __forceinline__ bool metropolis(double de, float temp, float u) {
-    return de <= 0.0 || (double)u < exp(-de / (double)temp);
+
+// disulfide_energy (allatom.rs:155-180) over the SG atoms (topology atom 5) of the
+// residues in the bit mask cysw, pairs in residue order, by one warp: lanes test the
+// partners of one Cys at a time and the in-range terms are subtracted in order (the
+// result is on every lane).  sweep: residues take their slots as the sweep sees them
+// (their proposal when accepted, their rejection rebuild when rejected, else the state)
+// and residue `sub` (>= 0) its proposal; else every residue is read from the state.
+template <class L, class ACC>
+__device__ __noinline__ ACC warp_disulfide(bool sweep, int words, int sub) {
+    L& S = an_smem<L>();
+    const unsigned* cys = S.cysw;
+    const int lane = threadIdx.x & 31;
+    int k = 0;
+    for (int w = 0; w < words; ++w) k += __popc(cys[w]);
+    ACC e = 0;
+    if (k < 2) return e;
+    auto sg = [&](int j) -> float4 {
+        const int s = sweep ? (j == sub ? (int)SEL_PROP : S.sel[j] & 3) : (int)SEL_KEEP;
+        return (s == SEL_PROP ? S.prop : s == SEL_REJ ? S.rej : S.pos)[j * SLOT_STRIDE + 5];
+    };
+    for (int wi = 0; wi < words; ++wi)
+        for (unsigned mi = cys[wi]; mi; mi &= mi - 1) {
+            const int i = wi * 32 + __ffs(mi) - 1;
+            const float4 pi = sg(i);
+            for (int wj = wi; wj < words; ++wj) {
+                const unsigned mj = cys[wj];
+                if (!mj) continue;
+                const int j = wj * 32 + lane;
+                float t = 0.0f;
+                bool in = false;
+                if (j > i && (mj >> lane & 1u)) {
+                    const float4 pj = sg(j);
+                    const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
+                    in = !(d > 4.0f);
+                    if (in) {
+                        const float z = xdiv(xsub(d, 2.05f), 0.4f);
+                        t = xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z)));
+                    }
+                }
+                for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1)
+                    e -= (ACC)__shfl_sync(0xffffffffu, t, __ffs(m) - 1);
+            }
+        }
+    return e;
 }
-// Metropolis-Hastings with the log proposal ratio lhr = log q(reverse) - log q(forward):
-// accept when u < exp(-dE/T + lhr).  lhr == 0 (uniform proposal) is exactly the
-// Metropolis criterion above.
+
+// The exponentials and trigonometry of the step, one copy each: inlined at every use
+// their double-precision code was most of the kernel's instruction footprint.
+__device__ __noinline__ bool accept_exact(float de, float temp, float u, double) { return u < mc_exp(xdiv(-de, temp)); }
+__device__ __noinline__ bool accept_exact(double de, float temp, float u, double lhr) {
+    return (double)u < exp(lhr == 0.0 ? -de / (double)temp : -de / (double)temp + lhr);
+}
+__device__ __noinline__ float4 torsion_trig(float delta) {  // cos, sin of delta and of -delta
+    const float ca = mc_cos(delta), sa = mc_sin(delta);
+    return make_float4(ca, sa, ca, -sa);
+}
+__device__ __noinline__ U4 step_draw(uint64_t seed, uint32_t cand, uint32_t step, uint32_t stream, uint32_t r) {
+    return rng_draw(seed, cand, step, stream, r);
+}
+
+// Metropolis-Hastings (diffusion.rs:368, 385, 414-415) with the log proposal ratio lhr
+// = log q(reverse) - log q(forward), 0 for the uniform proposal: accept when de <= 0 or
+// u < exp(-dE/T + lhr) (for lhr = 0 the plain criterion).  The exponential is first
+// taken in fast f32, whose argument x + l is off by less than 1e-6 (|x| + |l|): below
+// -17 with that margin it is smaller than any nonzero u (u is 0 or at least 2^-24 =
+// e^-16.6); with |x| + |l| < 64 the value is off by less than 1e-4 of itself, so a u
+// further away is decided.  The others (about one in 10^4) take the exact test (ACC =
+// float: the reference's f32 one).
 template <class ACC>
-__device__ __forceinline__ bool mh_accept(ACC de, float temp, float u, double lhr) {
-    if (lhr == 0.0) return metropolis(de, temp, u);
-    const double a = -(double)de / (double)temp + lhr;
-    return a >= 0.0 || (double)u < exp(a);
+__device__ __noinline__ bool mh_accept(ACC de, float temp, float u, double lhr) {
+    if (lhr == 0.0 && de <= (ACC)0) return true;
+    const float x = __fdividef(-(float)de, temp), l = (float)lhr, size = fabsf(x) + fabsf(l);
+    if (x + l + 1e-6f * size < -17.0f && u > 0.0f) return false;
+    if (size < 64.0f) {
+        const float pr = __expf(x + l);
+        if (u < pr * 0.9999f) return true;
+        if (u > pr * 1.0001f) return false;
+    }
+    return lhr == 0.0 ? accept_exact(de, temp, u, 0.0) : accept_exact((double)de, temp, u, lhr);
 }
 
 // ---- learned proposal -------------------------------------------------------------
 // Features of the tile rows: row i = residue mvl[base + i]; the one-hot of its amino
 // acid for a rotamer query, none for a mutation query (the network's mutation
 // outputs then depend on the environment alone, the same before and after the
-// move); one warp per row (8 rows, 8 warps).  ag_aa and the log1p table are the
-// shared-memory copies when staged.
-__device__ void an_tile_features(const AnSmem& S, const MlpTile& T, const int* rows_of, int base, int rows,
-                                 const float4* agq, const uint8_t* ag_aa, int nag, const float* lg1p) {
+// move); one warp per row (8 rows, 8 warps).  The environment counts come from the
+// residue's Verlet list when it still covers the Calpha and the antigen is staged,
+// else from all Calphas.
+template <class L>
+__device__ __forceinline__ void an_tile_features(const L& S, const MlpTile& T, const int* rows_of, int base, int rows) {
+    const float4* agq = S.env.pos;
+    const uint8_t* ag_aa = S.env.aa;
+    const bool listed = S.env.map == nullptr;  // list order = scan order
+    const float* lg1p = S.lg1p;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = warp; i < MT_ROWS; i += AN_WARPS) {
         int* cnt = T.cnt + i * MLP_SHELLS * N_AA;
@@ -395,7 +453,20 @@ __device__ void an_tile_features(const AnSmem& S, const MlpTile& T, const int* r
         for (int j = lane; j < MLP_SHELLS * N_AA; j += 32) cnt[j] = 0;
         __syncwarp();
         const float4 ca = S.pos[r * SLOT_STRIDE + 1];
-        mlp_count_env(agq, ag_aa, nag, ca.x, ca.y, ca.z, cnt);
+        const float4 cc = S.cgcentre[r];
+        const int nl = S.cgnl[r];
+        const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
+        if (listed && nl <= CG_LIST_MAX && mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f)) {
+            const uint16_t* list = S.cglist + (size_t)r * CG_LIST_MAX;
+            for (int j = lane; j < nl; j += 32) {
+                const int k = list[j];
+                const float4 q = agq[k];
+                const float r2 = xdist2(xsub(ca.x, q.x), xsub(ca.y, q.y), xsub(ca.z, q.z));
+                if (r2 < 100.0f) atomicAdd(&cnt[mlp_shell(r2) * N_AA + ag_aa[k]], 1);
+            }
+        } else {
+            mlp_count_env(agq, ag_aa, S.env.n, ca.x, ca.y, ca.z, cnt);
+        }
         __syncwarp();
         const int a = S.kind[r] == MV_MUT ? -1 : S.aa[r];
         for (int j = lane; j < MLP_K1; j += 32) {
@@ -433,42 +504,78 @@ __device__ int warp_sample(const float* y, int n, double inv_tp, uint32_t dz) {
 
 // The residue a move leaves: which = SEL_PROP builds the proposal, SEL_REJ the state
 // after a rejection (rebuild_side_chain with the old chi, or mutate_residue back to
-// the old amino acid around the same Calpha; allatom.rs:244-384).  The two kinds
-// differ only in the backbone the side chain is built on (the current one, or the
-// ideal one around the Calpha), so lanes of a warp building different kinds share
-// the side-chain loop.
-__device__ void build_move(const AnSmem& S, int r, int which) {
+// the old amino acid around the same Calpha; allatom.rs:244-384), by four lanes of a
+// warp (all lanes call; live: the four lanes have a build).  The two kinds differ only
+// in the backbone the side chain is built on (the current one, or the ideal one around
+// the Calpha), so the builds of a warp share the side-chain loop.  Lanes 0..2 of four
+// compute x, y, z of each atom -- place_atom (rotamer.rs:198-232) operation for
+// operation, a vector's squares and cross products exchanged by shuffles -- because the
+// chain of dependent atoms is what a build costs: one division instead of three per
+// normalisation is on it.  Atoms go straight into the row of prop / rej, the program
+// comes from the CTA's shared tables one atom ahead.  A side-chain-only build writes
+// the side chain's slots only (SEL_SIDE: the others stay as they are).
+__device__ __forceinline__ float quad_norm(float v) {  // component of norm3 (allatom.rs:486-489)
+    const float q = xmul(v, v);
+    const float d = xadd(xadd(__shfl_sync(0xffffffffu, q, 0, 4), __shfl_sync(0xffffffffu, q, 1, 4)),
+                         __shfl_sync(0xffffffffu, q, 2, 4));
+    return xdiv(v, fmaxf(xsqrt(d), 1e-8f));
+}
+template <class L>
+__device__ __forceinline__ void build_move(L& S, int r, int which, bool live) {
+    const int q = threadIdx.x & 3;
+    const int c = q == 3 ? 0 : q, u = c == 2 ? 0 : c + 1, v = c == 0 ? 2 : c - 1;  // own, next, next but one component
     const int oa = S.aa[r];
     const int kind = S.kind[r];
-    const int na = kind == MV_MUT ? S.new_aa[r] : oa;
+    const int na = S.new_aa[r];
+    const bool side_only = kind == MV_ROT || na == oa;  // side chain rebuilt on the current backbone
     const float4* cur = S.pos + (size_t)r * SLOT_STRIDE;
     float4* out = (which == SEL_PROP ? S.prop : S.rej) + (size_t)r * SLOT_STRIDE;
-    const ChiTrig old_t = unpack_trig(S.trig[2 * r], S.trig[2 * r + 1]);
-    const bool side_only = kind == MV_ROT || na == oa;  // side chain rebuilt on the current backbone
-    F3 atoms[SLOTS];
-    int a, n_bb;
-    ChiTrig t = old_t;
-    if (side_only) {
-        a = oa;
-        if (which == SEL_PROP) {
-            if (kind == MV_ROT) t = rot_trig(oa, S.new_rot[r]);
-            else t = s_rot_n[oa] > 0 ? rot_trig(oa, 0) : zero_trig();
-        }
-        n_bb = 4 + (oa != GLY ? 1 : 0);  // N, CA, C, O[, CB]
-        for (int k = 0; k < n_bb; ++k) atoms[k] = f3(cur[k]);
-    } else {
-        // ideal backbone around the Calpha with the new (or, rejected, the old) residue
-        a = which == SEL_PROP ? na : oa;
-        if (which == SEL_PROP) t = s_rot_n[na] > 0 ? rot_trig(na, 0) : zero_trig();
-        n_bb = ideal_backbone(f3(cur[1]), a, atoms);
+    const int a = which == SEL_PROP ? na : oa;
+    const float2* trig = (const float2*)(S.trig + 2 * r);
+    if (which == SEL_PROP) {
+        const int rot = kind == MV_ROT ? S.new_rot[r] : 0;
+        trig = S.rott + (kind == MV_ROT || S.rot_n[a] > 0 ? (a * 5 + rot) * 4 : N_AA * 20);
     }
-    build_side_chain(a, atoms, n_bb, t);
-    const int n_at = s_topo_n[a];
-    if (side_only) {
-        for (int k = 0; k < SLOT_STRIDE; ++k)
-            out[k] = (k >= n_bb && k < n_at) ? make_float4(atoms[k].x, atoms[k].y, atoms[k].z, 0.f) : cur[k];
-    } else {
-        store_residue(out, atoms, n_at);
+    int n_bb = 4 + (a != GLY ? 1 : 0);  // N, CA, C, O[, CB]
+    const int n_at = S.topo_n[a];
+    const float4* bb = cur;
+    if (live && !side_only) {  // ideal backbone around the Calpha with the new (or, rejected, the old) residue
+        F3 at[5];
+        n_bb = ideal_backbone(f3(cur[1]), a, at);
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            if ((k & 3) == q && k < n_bb) out[k] = make_float4(at[k].x, at[k].y, at[k].z, 0.f);
+        for (int k = n_at + q; k < SLOT_STRIDE; k += 4) out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        bb = out;
+    }
+    const int n = live ? S.sc_n[a] : 0;
+    const int n_max = __reduce_max_sync(0xffffffffu, n);
+    const float4* prog = S.sct + a * SC_MAX;
+    const float2* fix = S.scf + a * SC_MAX;
+    float4 g = prog[0];
+    float2 fx = fix[0];
+    for (int k = 0; k < n_max; ++k) {
+        __syncwarp();                                // the atoms placed so far
+        const unsigned ref = __float_as_uint(g.w);  // reference atoms a, b, c and the chi (255: fixed)
+        const int ia = ref & 255u, ib = ref >> 8 & 255u, ic = ref >> 16 & 255u, chi = ref >> 24;
+        const float2 d = chi == 255 ? fx : trig[chi];
+        const float* pa = (const float*)((ia < n_bb ? bb : out) + ia);
+        const float* pb = (const float*)((ib < n_bb ? bb : out) + ib);
+        const float* pc = (const float*)((ic < n_bb ? bb : out) + ic);
+        const float bu = pb[u], bv = pb[v], cc = pc[c];
+        const float bc = quad_norm(xsub(pb[c], cc));
+        const float ba_u = xsub(bu, pa[u]), ba_v = xsub(bv, pa[v]);
+        const float bond = g.x, sa = g.y, nca = -g.z;
+        if (k + 1 < n) {
+            g = prog[k + 1];
+            fx = fix[k + 1];
+        }
+        const float bc_u = __shfl_sync(0xffffffffu, bc, u, 4), bc_v = __shfl_sync(0xffffffffu, bc, v, 4);
+        const float nn = quad_norm(xsub(xmul(ba_u, bc_v), xmul(ba_v, bc_u)));
+        const float n_u = __shfl_sync(0xffffffffu, nn, u, 4), n_v = __shfl_sync(0xffffffffu, nn, v, 4);
+        const float m = xsub(xmul(bc_u, n_v), xmul(bc_v, n_u));
+        const float p = xadd(cc, xmul(bond, xadd(xadd(xmul(nca, bc), xmul(xmul(sa, d.y), m)), xmul(xmul(sa, d.x), nn))));
+        if (k < n) ((float*)(out + n_bb + k))[q] = q == 3 ? 0.0f : p;
     }
 }
 
@@ -487,15 +594,18 @@ __device__ __forceinline__ float4 rodrigues(float4 p, F3 o, F3 ax, float ca, flo
 // Rotate the atoms a phi (about N-CA through CA: residue r's atoms after CA and all
 // later residues) or psi move (about CA-C through C: residue r's O and all later
 // residues) moves, by the angle whose cosine and sine are ca, sa; allatom.rs:397-455.
-__device__ void rotate_downstream(const AnSmem& S, int n, int r, bool phi, float ca, float sa) {
+template <class L>
+__device__ __noinline__ void rotate_downstream(int n, int r, bool phi, float ca, float sa) {
+    L& S = an_smem<L>();
     const float4* rs = S.pos + (size_t)r * SLOT_STRIDE;
     const F3 a0 = f3(rs[phi ? 0 : 1]), a1 = f3(rs[phi ? 1 : 2]);
     const F3 axis = norm3(sub3(a1, a0));
     const F3 origin = a1;
-    const int n_at_r = s_topo_n[S.aa[r]];
+    const int n_at_r = S.topo_n[S.aa[r]];
+#pragma unroll 1
     for (int idx = threadIdx.x; idx < (n - r) * SLOT_STRIDE; idx += blockDim.x) {
         const int q = r + idx / SLOT_STRIDE, k = idx % SLOT_STRIDE;
-        const bool mv = q == r ? (phi ? (k >= 2 && k < n_at_r) : k == 3) : k < s_topo_n[S.aa[q]];
+        const bool mv = q == r ? (phi ? (k >= 2 && k < n_at_r) : k == 3) : k < S.topo_n[S.aa[q]];
         if (mv) {
             float4* p = S.pos + (size_t)q * SLOT_STRIDE + k;
             *p = rodrigues(*p, origin, axis, ca, sa);
@@ -503,150 +613,77 @@ __device__ void rotate_downstream(const AnSmem& S, int n, int r, bool phi, float
     }
 }
 
-// Coarse-grained force on residue r (compute_forces_with_grid, energy.rs:322-398) by
-// its group of CG_LANES lanes (gl = lane in group, all lanes of the group call).
-// Lane gl evaluates the consecutive probe cells [27 gl / 8, 27 (gl + 1) / 8) of the
-// reference's (dx, dy, dz) order into its term slots; lane 0 then adds the terms
-// lane by lane.  A lane with more in-cutoff terms than slots sends the residue to
-// the one-lane walk (same sum).  Result valid in lane 0 of the group.
-__device__ void group_cg_force(const AgView& A, const CgB& body, int gl, unsigned gmask, float4* my_terms,
-                               int* my_count, const int* group_counts, const float4* group_terms, float& fx,
-                               float& fy, float& fz) {
-    const GridView& g = A.ca_grid;
-    const int cx = cell_coord(body.x, g.inv), cy = cell_coord(body.y, g.inv), cz = cell_coord(body.z, g.inv);
-    const float p[3] = {body.x, body.y, body.z};
-    const int c[3] = {cx, cy, cz};
-    // squared distance to the lower / own / upper slab per dimension (culling only;
-    // the margin covers the f32 rounding of x*inv and of the slab bounds)
-    float sl[3][3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-#pragma unroll
-        for (int o = 0; o < 3; ++o) {
-            const float lo = (float)(c[d] + o - 1) * g.cell, hi = lo + g.cell;
-            const float dd = fmaxf(fmaxf(lo - p[d], p[d] - hi), 0.0f);
-            sl[d][o] = dd * dd;
-        }
-    const float reach = 10.001f + 4e-7f * (fabsf(body.x) + fabsf(body.y) + fabsf(body.z));
-    const float reach2 = reach * reach;
-    const int c_lo = (27 * gl) / CG_LANES, c_hi = (27 * (gl + 1)) / CG_LANES;
-    int nt = 0;
-    for (int ci = c_lo; ci < c_hi; ++ci) {
-        const int dx = ci / 9 - 1, dy = (ci / 3) % 3 - 1, dz = ci % 3 - 1;
-        if (sl[0][dx + 1] + sl[1][dy + 1] + sl[2][dz + 1] > reach2) continue;
-        int a0, a1;
-        if (!probe_cell(g, cx, cy, cz, dx, dy, dz, a0, a1)) continue;
-        for (int i = a0; i < a1; ++i) {
-            float tx, ty, tz;
-            if (!cg_term_parts(body, A.ca_pq[i], A.ca_prm[i], tx, ty, tz)) continue;
-            if (nt < CG_SLOTS) my_terms[nt] = make_float4(tx, ty, tz, 0.f);
-            ++nt;
-        }
-    }
-    *my_count = nt;
-    const bool overflow = (__ballot_sync(gmask, nt > CG_SLOTS) & gmask) != 0u;
-    __syncwarp(gmask);
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    if (gl == 0) {
-        if (!overflow) {
-            for (int L = 0; L < CG_LANES; ++L) {
-                const int cnt = group_counts[L];
-                const float4* t = group_terms + L * CG_SLOTS;
-                for (int k = 0; k < cnt; ++k) {
-                    sx = xadd(sx, t[k].x);
-                    sy = xadd(sy, t[k].y);
-                    sz = xadd(sz, t[k].z);
-                }
-            }
-        } else {
-            cg_force(A, body, sx, sy, sz);
-        }
-    }
-    fx = sx; fy = sy; fz = sz;
-}
-
-// compute_forces_with_grid for the residue of a group of GL lanes from its
-// Verlet list (cg_list.cuh), kept in shared memory across the steps of the launch
-// and rebuilt, with twice the skin up to CG_SKIN_MAX, when the Calpha leaves the
-// skin of the list centre (a backbone move or the steps' drift).  The list entries
-// passing the reference's tests, in list order, are the reference's pairs in its
-// order: the group compacts them (at most CG_IN_MAX a round), its lanes evaluate the
-// terms and lane 0 sums them in that order -- the sum of the 27-cell walk.  A list
-// that overflows, or cells near the i32 limits, fall back to the one-lane walk.
-// in / terms: the group's per-step scratch.  The force is in lane 0.
+// Sum, in order, of the coarse-grained pair terms (compute_forces, energy.rs:353-391)
+// of the lane group's cnt candidates (list entries, or 0 .. cnt-1 without a list) inside
+// the cutoff (with cells, beyond near_sq also in a cell next to the body's, as the
+// reference probes), by the GL lanes of the group; the groups of a warp run in
+// lockstep (every loop is warp-uniform, every ballot full: group masks would split the
+// warp).  The group compacts the passing candidates, its lanes evaluate one pair each
+// into the residue's x / y / z rows, and lanes 0..2 add one component each in order,
+// four terms a load -- the pads are +0, which leaves a sum that starts at +0 unchanged.
+// Scratch: rows xy (x at 0, y at AN_IN) and zi (z, then the compacted entries), 64
+// floats each; entry k of a row lies at (k + 4 group) mod AN_IN, apart in banks from the
+// warp's other groups.  Lanes 0..2 of the group return x, y, z.
 template <int GL>
-__device__ void group_cg_force_list(const AgView& A, const CgB& body, int gl, unsigned gmask, int* list,
-                                    float4* centre, int* nlp, int* in, float4* terms, float& fx, float& fy,
-                                    float& fz) {
-    static_assert(CG_IN_MAX % GL == 0, "a round compacts whole group steps");
-    const GridView& g = A.ca_grid;
-    const F3 ca = {body.x, body.y, body.z};
-    float4 cc = *centre;
-    int nl = *nlp;
-    const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
-    if (nl < 0 || !(mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f))) {
-        const float skin = nl < 0 ? CG_SKIN : fminf(2.0f * cc.w, CG_SKIN_MAX);
-        nl = build_cg_list<GL>(g, A.ca_pq, ca, gl, gmask, list, skin);
-        cc = make_float4(ca.x, ca.y, ca.z, skin);
-        __syncwarp(gmask);
-        if (gl == 0) {
-            *centre = cc;
-            *nlp = nl;
-        }
-    }
-    const int cx = cell_coord(ca.x, g.inv), cy = cell_coord(ca.y, g.inv), cz = cell_coord(ca.z, g.inv);
-    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    if (nl > CG_LIST_MAX || cell_far(cx, cy, cz)) {
-        if (gl == 0) cg_force(A, body, sx, sy, sz);
-    } else {
-        const bool near_adjacent = g.cell >= 10.0f && fabsf(ca.x) < 1e4f && fabsf(ca.y) < 1e4f &&
-                                   fabsf(ca.z) < 1e4f;  // see k_langevin
-        const int gshift = (int)(threadIdx.x & 31) & ~(GL - 1);
-        const unsigned below = (1u << gl) - 1u;
-        int from = 0;
-        while (from < nl) {  // group-uniform
-            int n_in = 0;
-            while (from < nl && n_in + GL <= CG_IN_MAX) {
-                const int j = from + gl;
-                bool ok = false;
-                int i = 0;
-                if (j < nl) {
-                    i = list[j];
-                    const float4 a = A.ca_pq[i];
-                    const float r_sq = xdist2(xsub(ca.x, a.x), xsub(ca.y, a.y), xsub(ca.z, a.z));
-                    ok = !(r_sq > CUTOFF_SQ || r_sq < MIN_R_SQ);
-                    if (ok && !(near_adjacent && r_sq <= CG_NEAR_SQ)) {  // the reference's cell test
-                        const int4 ce = A.ca_cell[i];
-                        ok = abs((long long)ce.x - cx) <= 1 && abs((long long)ce.y - cy) <= 1 &&
-                             abs((long long)ce.z - cz) <= 1;
-                    }
+__device__ __noinline__ float group_force(int cnt, const uint16_t* list, const int4* cells, int cx, int cy, int cz,
+                                          float near_sq, const CgB body, const float4* q, const float4* prm, float* xy, float* zi) {
+    static_assert(AN_IN % GL == 0 && GL >= 4, "a round compacts whole group steps");
+    const int lane = threadIdx.x & 31, gl = lane & (GL - 1), gshift = lane & ~(GL - 1);
+    const int skew = 4 * (lane / GL);
+    uint16_t* in = (uint16_t*)(zi + AN_IN);
+    const float* row = gl == 0 ? xy : gl == 1 ? xy + AN_IN : zi;
+    const unsigned below = (1u << gl) - 1u;
+    const int mx = __reduce_max_sync(0xffffffffu, cnt);
+    float s = 0.0f;
+    int from = 0;
+    while (from < mx) {
+        int n_in = 0;
+#pragma unroll 1
+        for (int st = 0; st < AN_IN / GL && from < mx; ++st, from += GL) {
+            const int j = from + gl;
+            bool ok = false;
+            int i = 0;
+            if (j < cnt) {
+                i = list ? list[j] : j;
+                const float4 a = q[i];
+                const float r_sq = xdist2(xsub(body.x, a.x), xsub(body.y, a.y), xsub(body.z, a.z));
+                ok = !(r_sq > CUTOFF_SQ || r_sq < MIN_R_SQ);
+                if (ok && cells && r_sq > near_sq) {  // the reference's cell test
+                    const int4 ce = cells[i];
+                    ok = abs((long long)ce.x - cx) <= 1 && abs((long long)ce.y - cy) <= 1 &&
+                         abs((long long)ce.z - cz) <= 1;
                 }
-                const unsigned m = (__ballot_sync(gmask, ok) >> gshift) & (GL == 32 ? ~0u : ((1u << GL) - 1u));
-                if (ok) in[n_in + __popc(m & below)] = i;
-                n_in += __popc(m);
-                from += GL;
             }
-            __syncwarp(gmask);
-            for (int k = gl; k < n_in; k += GL) {
+            const unsigned m = __ballot_sync(0xffffffffu, ok) >> gshift & ((1u << GL) - 1u);
+            if (ok) in[n_in + __popc(m & below)] = (uint16_t)i;
+            n_in += __popc(m);
+        }
+        __syncwarp();
+        const int kmax = __reduce_max_sync(0xffffffffu, n_in);
+#pragma unroll 1
+        for (int k = gl; k < kmax + gl; k += GL) {  // kmax / GL rounds, rounded up
+            float tx = 0.0f, ty = 0.0f, tz = 0.0f;
+            if (k < n_in) {
                 const int i = in[k];
-                float tx, ty, tz;
-                cg_term_parts(body, A.ca_pq[i], A.ca_prm[i], tx, ty, tz);
-                terms[k] = make_float4(tx, ty, tz, 0.f);
+                cg_term_parts(body, q[i], prm[i], tx, ty, tz);
             }
-            __syncwarp(gmask);
-            if (gl == 0)
-                for (int k = 0; k < n_in; ++k) {
-                    const float4 t = terms[k];
-                    sx = xadd(sx, t.x);
-                    sy = xadd(sy, t.y);
-                    sz = xadd(sz, t.z);
-                }
-            __syncwarp(gmask);  // the scratch is rewritten next round
+            if (cnt > 0) {
+                const int at = (k + skew) & (AN_IN - 1);
+                xy[at] = tx;
+                xy[AN_IN + at] = ty;
+                zi[at] = tz;
+            }
         }
+        __syncwarp();
+        if (gl < 3 && cnt > 0)
+#pragma unroll 1
+            for (int k = 0; k < kmax; k += 4) {
+                const float4 t = *(const float4*)(row + ((k + skew) & (AN_IN - 1)));
+                s = xadd(xadd(xadd(xadd(s, t.x), t.y), t.z), t.w);
+            }
+        __syncwarp();  // the rows are rewritten next round
     }
-    fx = sx;
-    fy = sy;
-    fz = sz;
+    return s;
 }
 
 // The network's choice of every mutation and (known-rotamer) rotamer move drawn
@@ -654,18 +691,17 @@ __device__ void group_cg_force_list(const AgView& A, const CgB& body, int gl, un
 // network pass per tile of moves.  A move changes neither the residue's environment
 // nor its query (mutation: no amino-acid input; rotamer: the unchanged amino acid),
 // so the reverse move's proposal is the same softmax: log q(reverse) - log q(move)
-// = (y[move] - y[back]) / Tp, the normalisers cancelling.  The shared-memory
-// layout is carved again from its base (smem, R, G, C) and the network comes by
-// value: a reference to the kernel's copies would put them in local memory.  The
-// biases are read from their shared-memory copies (staged by the kernel).
-__device__ __noinline__ void an_learned_choices(unsigned char* smem, int R, int G, int C, int n, const float4* agq,
-                                                const uint8_t* ag_aa, int nag, MlpDev mlp, float temp) {
+// = (y[move] - y[back]) / Tp, the normalisers cancelling.  The network comes by value:
+// a reference to the kernel's copy would put it in local memory.  The biases are read
+// from their shared-memory copies (staged by the kernel).
+template <class L>
+__device__ __noinline__ void an_learned_choices(int n, MlpDev mlp, float temp) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const AnSmem S = carve(smem, R, G, C, 1);
+    L& S = an_smem<L>();
     mlp.b1 = S.mbias;  // the biases' shared-memory copies
     mlp.b2 = S.mbias + MLP_H;
     mlp.b3 = S.mbias + 2 * MLP_H;
-    const MlpTile T = mlp_tile_carve((unsigned char*)S.terms);
+    const MlpTile T = mlp_tile_carve(S.tile);
     const double inv_tp = 1.0 / (double)fmaxf(temp, mlp.t_prop_min);
     uint4 w[MT_WREGS];
     mlp_tile_prefetch(mlp, w);  // the first weights are on their way during the features
@@ -686,7 +722,7 @@ __device__ __noinline__ void an_learned_choices(unsigned char* smem, int R, int 
     for (int base = 0; base < n_mv; base += MT_ROWS) {
         const int rows = min(MT_ROWS, n_mv - base);
         if (base > 0) mlp_tile_prefetch(mlp, w);
-        an_tile_features(S, T, S.mvl, base, rows, agq, ag_aa, nag, S.lg1p);
+        an_tile_features(S, T, S.mvl, base, rows);
         __syncthreads();
         mlp_tile_forward(mlp, T, w, rows);
         for (int i = warp; i < rows; i += AN_WARPS) {  // one warp per row
@@ -694,16 +730,98 @@ __device__ __noinline__ void an_learned_choices(unsigned char* smem, int R, int 
             const bool rot = S.kind[r] == MV_ROT;
             // rotamer query: outputs 20 + j over the residue's rotamers; mutation: outputs 0..19
             const float* y = T.y + i * MT_YS + (rot ? N_AA : 0);
-            const int k = warp_sample(y, rot ? s_rot_n[S.aa[r]] : N_AA, inv_tp, S.dz[r]);
+            const int k = warp_sample(y, rot ? S.rot_n[S.aa[r]] : N_AA, inv_tp, S.dz[r]);
             if (lane == 0) {
                 const int back = rot ? S.rot[r] : S.aa[r];  // the reverse move's option
                 if (rot) S.new_rot[r] = k;
                 else S.new_aa[r] = k;
+                if (back == CYS || (!rot && k == CYS)) S.iscal[IS_CYSMV] = 1;
                 S.lhr[r] = ((double)y[k] - (double)y[back]) * inv_tp;
             }
         }
         __syncthreads();
     }
+}
+
+// Calpha energies (residue_contribution_allatom, diffusion.rs:425-463, and for Fv the
+// partner chain's, :551-553) of four tasks by one warp, EL = 8 lanes each, in double:
+// residue r as amino acid aa (live: the lane's task exists).  A residue still inside
+// its list's skin reads the list's entries (it holds every Calpha within the cutoff);
+// the others are scanned by the whole warp, one after another.  Every lane of a group
+// gets its task's energy.
+template <class L>
+__device__ __noinline__ double task_energies(int r, int aa, bool live) {
+    L& S = an_smem<L>();
+    const int lane = threadIdx.x & 31, gl = lane & (EL - 1);
+    const F3 ca = f3(S.pos[r * SLOT_STRIDE + 1]);
+    const float4 b = S.ca_atom[aa];
+    const int bhb = S.ca_hb[aa];
+    const float4 cc = S.cgcentre[r];
+    const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
+    const int nl = S.cgnl[r];
+    const bool ok = live && nl <= CG_LIST_MAX && mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f);
+    // the group's in-cutoff candidates queued (r^2, amino acid), EL at a time evaluated one
+    // per lane
+    double e = 0.0;
+    const unsigned below = (1u << gl) - 1u;
+    constexpr int CAP = HIT_CAP * EL / 32;
+    float2* hits = S.hits + (threadIdx.x >> 5) * HIT_CAP;
+    float2* q = hits + (lane / EL) * CAP;
+    int n_in = 0;
+    const uint16_t* list = S.cglist + r * CG_LIST_MAX;
+    const float4* lpos = S.env.lpos;
+    const uint8_t* ag_aa = S.env.aa;
+    const float4* map = S.env.map;
+    const int n_list = ok ? nl : 0, n_all = n_list + (L::FV && live ? S.env.np : 0);
+    const int n_max = __reduce_max_sync(0xffffffffu, n_all);
+#pragma unroll 1
+    for (int j0 = 0; j0 < n_max; j0 += EL) {
+        const int j = j0 + gl;
+        bool in = false;
+        int t = 0;
+        float r_sq = 0.0f;
+        if (j < n_all) {
+            int i;
+            float4 a;
+            if (L::FV && j >= n_list) {
+                i = j - n_list;
+                a = S.ptq[i];
+            } else {
+                i = list[j];
+                a = lpos[i];
+            }
+            r_sq = xdist2(xsub(ca.x, a.x), xsub(ca.y, a.y), xsub(ca.z, a.z));
+            in = !(r_sq > CUTOFF_SQ || r_sq < MIN_R_SQ);
+            if (in) t = L::FV && j >= n_list ? S.ptaa[i] : ag_aa[map ? __float_as_int(map[i].w) : i];
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in) >> (lane & ~(EL - 1)) & ((1u << EL) - 1u);
+        if (in) q[n_in + __popc(m & below)] = make_float2(r_sq, __int_as_float(t));
+        n_in += __popc(m);
+        const int k_max = __reduce_max_sync(0xffffffffu, n_in);
+        if (k_max + EL > CAP || j0 + EL >= n_max) {
+            __syncwarp();
+#pragma unroll 1
+            for (int k = gl; k < k_max + gl; k += EL)
+                if (k < n_in) {
+                    const float2 h = q[k];
+                    const int a = __float_as_int(h.y);
+                    e += ca_pair_sum(b, bhb, S.ca_atom[a], S.ca_hb[a], h.x);
+                }
+            __syncwarp();
+            n_in = 0;
+        }
+    }
+#pragma unroll
+    for (int o = EL / 2; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+#pragma unroll 1
+    for (unsigned m = __ballot_sync(0xffffffffu, live && !ok && gl == 0); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const F3 c = {__shfl_sync(0xffffffffu, ca.x, src), __shfl_sync(0xffffffffu, ca.y, src),
+                      __shfl_sync(0xffffffffu, ca.z, src)};
+        const double v = warp_scan_energy<L>(c, __shfl_sync(0xffffffffu, aa, src), hits);
+        if ((lane & ~(EL - 1)) == src) e += v;
+    }
+    return e;
 }
 
 // EXT: the learned proposal and the proposal log are compiled in (a separate
@@ -714,86 +832,117 @@ __device__ __noinline__ void an_learned_choices(unsigned char* smem, int R, int 
 // as it is in the state; Calpha energies gain the partner chain's contribution, the
 // force its compute_forces term, and the mutation / rotamer moves follow the CDR
 // flags fv_cdr (per residue) instead of the interface mask.  Draw streams + 4 * chain.
-template <class ACC, bool EXT, bool FV, int W>
-__global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) k_anneal(StateView st, const AgView* __restrict__ ags, StepParams p,
-                                                       int n_steps, uint32_t step0, int with_noise,
-                                                       const float* __restrict__ temps, int R, int G, int C,
-                                                       uint32_t* __restrict__ err, long long* __restrict__ stats,
-                                                       MlpDev mlp, int learned, MlpTuple* __restrict__ tlog,
-                                                       unsigned long long* __restrict__ log_n, long long log_cap,
-                                                       int fv_chain, const uint8_t* __restrict__ fv_cdr) {
-    static_assert(W == AN_WARPS || (W == 2 * AN_WARPS && !EXT), "8 warps, or 16 without the network");
-    constexpr int NT = W * 32;  // threads of the CTA
-    extern __shared__ __align__(16) unsigned char an_smem[];
-    const AnSmem S = carve(an_smem, R, G, C, learned, FV ? 1 : 0, W);
+// L: the shared memory's fixed part; GL lanes per residue of the Langevin step; G, C
+// staged antigen Calphas and cells (0: none).
+template <class L, bool EXT, int GL>
+__global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LRN ? 3 : 16 / L::W))
+    k_anneal(StateView st, const AgView* __restrict__ ags, StepParams p, int n_steps, uint32_t step0, int with_noise,
+             const float* __restrict__ temps, int G, int C, uint32_t* __restrict__ err, long long* __restrict__ stats,
+             MlpDev mlp, int learned, MlpTuple* __restrict__ tlog, unsigned long long* __restrict__ log_n,
+             long long log_cap, int fv_chain, const uint8_t* __restrict__ fv_cdr) {
+    constexpr int W = L::W;
+    constexpr bool F32 = L::F32, FV = L::FV;
+    using ACC = typename std::conditional<F32, float, double>::type;
+    static_assert(!EXT || W == AN_WARPS, "the network tile takes 8 warps");
+    static_assert(!L::LRN || EXT, "the learned proposal is an EXT instance");
+    constexpr int NT = W * 32;               // threads of the CTA
+    constexpr int RPP = NT / GL;             // residues per Langevin pass
+    constexpr int BW = 2;                    // warps that build moves
+    constexpr int EW = W - BW;               // warps that compute energies beside them
+    L& S = an_smem<L>();
+    // the staged antigen
+    unsigned char* tail = reinterpret_cast<unsigned char*>(&S) + sizeof(L);
+    float4* const s_cgq = (float4*)tail;
+    float4* const s_cgp = s_cgq + G;
+    float4* const s_agq = s_cgp + G;                   // F32 from here ..
+    float4* const s_agp = s_agq + (F32 ? G : 0);
+    float* const s_agx = (float*)(s_agp + (F32 ? G : 0));
+    float* const s_agy = s_agx + (F32 ? anneal_xyz_len(G) : 0);
+    float* const s_agz = s_agy + (F32 ? anneal_xyz_len(G) : 0);
+    int* const s_cell = (int*)(s_agz + (F32 ? anneal_xyz_len(G) : 0));  // .. to here
+    uint8_t* const s_aa = (uint8_t*)(s_cell + C);
     const int c = FV ? 2 * (int)blockIdx.x + fv_chain : (int)blockIdx.x;
     const uint32_t sh = FV ? 4u * (uint32_t)fv_chain : 0u;  // draw stream offset of the chain
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r0 = st.cand_res_off[c];
     const int n = st.cand_res_off[c + 1] - r0;
-    if (n <= 0 || n > R) return;
+    if (n <= 0 || n > L::RT) return;
+    const int words = (n + 31) >> 5;  // of a residue bit mask
     const uint32_t cid = st.cand_id[c];
-    if (tid == 0) *S.ag = ags[st.cand_ag[c]];
+    if (tid == 0) S.ag = ags[st.cand_ag[c]];
     __syncthreads();
-    const AgView& A = *S.ag;
+    const AgView& A = S.ag;
     const int nag = A.n_res;
     const bool staged = nag <= G;
     const int ncell = A.ca_grid.nx * A.ca_grid.ny * A.ca_grid.nz + 1;
     const bool cells_staged = staged && ncell <= C;
+#pragma unroll 2
     for (int i = tid; staged && i < nag; i += NT) {
-        const float4 q = A.ca_atom[i];
-        S.agq[i] = q;
-        S.agp[i] = A.ca_atom_prm[i];
-        S.cgq[i] = A.ca_pq[i];
-        S.cgp[i] = A.ca_prm[i];
-        S.agx[i] = q.x;
-        S.agy[i] = q.y;
-        S.agz[i] = q.z;
+        const float4 prm = A.ca_prm[i];
+        s_cgq[i] = A.ca_pq[i];
+        s_cgp[i] = prm;
+        s_aa[i] = A.res_aa[__float_as_int(prm.w)];  // w: residue of the i-th Calpha in grid order
+        if (F32) {
+            const float4 q = A.ca_atom[i];
+            s_agq[i] = q;
+            s_agp[i] = A.ca_atom_prm[i];
+            s_agx[i] = q.x;
+            s_agy[i] = q.y;
+            s_agz[i] = q.z;
+        }
     }
-    if (tid == 0 && staged && (nag & 1)) S.agx[nag] = S.agy[nag] = S.agz[nag] = 1e30f;
-    for (int i = tid; cells_staged && i < ncell; i += NT) S.cgcell[i] = A.ca_grid.cell_start[i];
-    if (EXT && learned) {  // the network's features and epilogues read these every step
-        for (int i = tid; staged && i < nag; i += NT) S.agaa[i] = A.res_aa[i];
+    if (F32 && tid == 0 && staged && (nag & 1)) s_agx[nag] = s_agy[nag] = s_agz[nag] = 1e30f;
+#pragma unroll 2
+    for (int i = tid; cells_staged && i < ncell; i += NT) s_cell[i] = A.ca_grid.cell_start[i];
+#pragma unroll 1
+    for (int i = tid; i < N_AA * SC_MAX; i += NT) {  // side-chain programs and rotamer trigonometry
+        const uchar4 q = (&s_sc_ref[0][0])[i];
+        const float4 g = (&s_sc_geom[0][0])[i];
+        S.sct[i] = make_float4(g.x, g.y, g.z, __uint_as_float(q.x | q.y << 8 | q.z << 16 | (unsigned)q.w << 24));
+        S.scf[i] = (&s_sc_fix[0][0])[i];
+    }
+#pragma unroll 1
+    for (int i = tid; i < N_AA * 20 + 4; i += NT)
+        S.rott[i] = i < N_AA * 20 ? (&s_rot_trig[0][0][0])[i] : make_float2(0.f, 1.f);
+    for (int i = tid; i < N_AA; i += NT) {
+        S.ca_atom[i] = s_ca_atom[i];
+        S.res[i] = s_res[i];
+        S.ca_hb[i] = s_hb_role[s_ca_type[i]];
+        S.topo_n[i] = s_topo_n[i];
+        S.sc_n[i] = s_sc_n[i];
+        S.rot_n[i] = s_rot_n[i];
+    }
+    if (L::LRN && learned) {  // the network's features and epilogues read these every step
         for (int i = tid; i <= MLP_COUNT_CAP; i += NT) S.lg1p[i] = g_an_log1p[i];
         for (int i = tid; i < MLP_BIASES; i += NT)
             S.mbias[i] = i < MLP_H ? mlp.b1[i] : i < 2 * MLP_H ? mlp.b2[i - MLP_H] : mlp.b3[i - 2 * MLP_H];
     }
-    __syncthreads();
-    if (tid == 0 && cells_staged) {  // the CG probe reads the staged copies through the view
-        S.ag->ca_pq = S.cgq;
-        S.ag->ca_prm = S.cgp;
-        S.ag->ca_grid.cell_start = S.cgcell;
-    }
-    const float4* agq = staged ? S.agq : A.ca_atom;
-    const float4* agp = staged ? S.agp : A.ca_atom_prm;
-    float4* stage = S.stage + warp * STAGE_CAP;
     // Fv: the partner chain's Calphas (it does not move during this launch)
     int np = 0;
     if (FV) {
         const int pc = c ^ 1, p0 = st.cand_res_off[pc];
-        np = min(st.cand_res_off[pc + 1] - p0, R);
+        np = min(st.cand_res_off[pc + 1] - p0, L::RT);
         for (int i = tid; i < np; i += NT) {
             const float4 v = st.res_pos[(size_t)(p0 + i) * SLOT_STRIDE + 1];
             const int a = st.res_aa[p0 + i];
             const float4 q = s_ca_atom[a], rl = s_res[a];
             S.ptq[i] = make_float4(v.x, v.y, v.z, q.x);
-            S.ptp[i] = make_float4(q.y, q.z, q.w, (float)s_ca_type[a]);
+            if (F32) S.ptp[i] = make_float4(q.y, q.z, q.w, (float)s_ca_type[a]);
+            S.ptaa[i] = (uint8_t)a;
             S.pcq[i] = make_float4(v.x, v.y, v.z, rl.x);
             S.pcp[i] = make_float4(rl.y, rl.z, rl.w, 0.f);
         }
-        __syncthreads();
     }
-    // residue_contribution_allatom of a Calpha at q with amino acid a, by the warp (the
-    // scans are noinline: one copy each instead of one per call site, less code to fetch);
-    // Fv: plus the contribution against the partner chain (fv_residue_contribution,
-    // diffusion.rs:551-553)
-    auto ca_energy = [&](F3 q, int a) -> ACC {
-        ACC e = staged ? warp_contribution_pairs<ACC>(S.agx, S.agy, S.agz, agq, agp, nag, q, a, stage)
-                       : warp_contribution<ACC>(agq, agp, nag, q, a, stage);
-        if (FV) e = e + warp_contribution<ACC>(S.ptq, S.ptp, np, q, a, stage);
-        return e;
-    };
-
+    if (tid == 0) {
+        S.env.lpos = staged ? s_cgq : A.ca_pq;
+        S.env.pos = staged ? s_cgq : A.ca_atom;
+        S.env.aa = staged ? s_aa : A.res_aa;
+        S.env.map = staged ? nullptr : A.ca_prm;
+        S.env.n = nag;
+        S.env.np = np;
+        S.iscal[IS_NTASK] = S.iscal[IS_CYSMV] = 0;
+    }
+#pragma unroll 2
     for (int i = tid; i < n * SLOT_STRIDE; i += NT) S.pos[i] = st.res_pos[(size_t)r0 * SLOT_STRIDE + i];
     for (int r = tid; r < n; r += NT) {
         const int a = st.res_aa[r0 + r];
@@ -802,6 +951,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) k_anneal(StateView st,
         S.chi[r] = chi;
         S.trig[2 * r] = st.res_trig[2 * (r0 + r)];
         S.trig[2 * r + 1] = st.res_trig[2 * (r0 + r) + 1];
+        S.cgnl[r] = -1;
+        S.cgcentre[r] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (EXT) {
             // rotamer index of the state: the library entry whose chi it holds, else -1
             int k = -1;
@@ -810,437 +961,569 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) k_anneal(StateView st,
                 if (t.x == chi.x && t.y == chi.y && t.z == chi.z && t.w == chi.w) k = q;
             }
             S.rot[r] = k;
-            S.lhr[r] = 0.0;
         }
     }
-    const bool lists = anneal_list_res(R) > 0;  // Verlet lists of the Langevin force
-    for (int r = tid; lists && r < n; r += NT) S.cgnl[r] = -1;
+    __syncthreads();
+    if (tid == 0 && cells_staged) {  // the list builds read the staged copies through the view
+        S.ag.ca_pq = s_cgq;
+        S.ag.ca_prm = s_cgp;
+        S.ag.ca_grid.cell_start = s_cell;
+    }
+    const float4* agq = staged ? s_agq : A.ca_atom;      // F32: residue order
+    const float4* agp = staged ? s_agp : A.ca_atom_prm;
+    const float4* cgq = staged ? s_cgq : A.ca_pq;        // grid (list) order
+    const float4* cgp = staged ? s_cgp : A.ca_prm;
+    // Calpha energies of the tasks 0 .. count-1, dealt over the warps w0 .. w0+nw-1 of the
+    // CTA (one per warp in turn): get(k, r, aa) names task k's residue and amino acid
+    // (false: none), put(k, e) takes its energy (one lane)
+    auto run_tasks = [&](int w0, int nw, int count, auto get, auto put) {
+        if constexpr (F32) {
+            float4* stage = S.stage + warp * STAGE_CAP;
+#pragma unroll 1
+            for (int k = warp - w0; k < count; k += nw) {
+                int r, a;
+                if (!get(k, r, a)) continue;
+                const F3 q = f3(S.pos[r * SLOT_STRIDE + 1]);
+                ACC e = staged ? warp_contribution_pairs<ACC>(s_agx, s_agy, s_agz, agq, agp, nag, q, a, stage)
+                               : warp_contribution<ACC>(agq, agp, nag, q, a, stage);
+                if (FV) e = e + warp_contribution<ACC>(S.ptq, S.ptp, np, q, a, stage);
+                if (lane == 0) put(k, (double)e);
+            }
+        } else {
+#pragma unroll 1
+            for (int k0 = warp - w0; k0 < count; k0 += nw * (32 / EL)) {
+                const int k = k0 + nw * (lane / EL);
+                int r = 0, a = 0;
+                const bool live = k < count && get(k, r, a);
+                const double e = task_energies<L>(live ? r : 0, live ? a : 0, live);
+                if (live && (lane & (EL - 1)) == 0) put(k, e);
+            }
+        }
+    };
     long long n_mc = 0, n_mc_acc = 0, n_bb = 0, n_bb_acc = 0;
     __syncthreads();
 
+    float next_temp = temps ? temps[0] : p.t_hot;
+#pragma unroll 1
     for (int s = 0; s < n_steps; ++s) {
         const uint32_t step = step0 + (uint32_t)s;
-        const float temp = temps ? temps[s] : p.t_hot;
-        // ---- 1. Langevin (diffusion.rs:306-339): CG_LANES lanes per residue, LW with
-        // Verlet lists (16 in the 16-warp instance: the list scans and terms take half
-        // the rounds; the sum in list order by the group's lane 0 is the same) ----
-        {
-            constexpr int LW = W == 2 * AN_WARPS ? 2 * CG_LANES : CG_LANES;
-            const int glanes = lists ? LW : CG_LANES;
-            const int gl = tid % glanes;
-            const unsigned gmask = ((1u << glanes) - 1u) << (lane & ~(glanes - 1));
-            const int g0 = tid - gl;  // first thread of the group
-            // the first CG_RES_PER_PASS groups (whole warps; with 16 warps and 8-lane
-            // groups the others wait at the barrier below)
-            for (int base = 0; tid < CG_RES_PER_PASS * glanes && base < n; base += CG_RES_PER_PASS) {
-                const int r = base + tid / glanes;
-                if (lists) {
-                    // lists the residues' Calphas outran: rebuilt by the whole warp, one
-                    // residue after another (a one-pass build with 32 lanes instead of a
-                    // two-pass build with the group's 8 lanes)
-                    bool need = false;
-                    F3 ca = {0.f, 0.f, 0.f};
-                    float skin = CG_SKIN;
-                    if (gl == 0 && r < n) {
-                        ca = f3(S.pos[r * SLOT_STRIDE + 1]);
-                        const float4 cc = S.cgcentre[r];
-                        const int nl = S.cgnl[r];
-                        const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
-                        need = nl < 0 || !(mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f));
-                        skin = nl < 0 ? CG_SKIN : fminf(2.0f * cc.w, CG_SKIN_MAX);
-                    }
-                    for (unsigned m = __ballot_sync(0xffffffffu, need); m; m &= m - 1) {
+        const float temp = next_temp;
+        if (temps && s + 1 < n_steps) next_temp = temps[s + 1];
+        unsigned* const attw = S.attw + (s & 1) * MASK_WORDS;
+        // ---- backbone move draws (diffusion.rs:403-405): 32 residues per warp, the last
+        // warps first (with up to NT / GL - 32 / GL residues the Langevin step leaves them idle)
+#pragma unroll 1
+        for (int w = W - 1 - warp; w < words; w += W) {
+            const int r = w * 32 + lane;
+            bool att = false;
+            if (r < n) {
+                const U4 d = step_draw(p.seed, cid, step, STREAM_BACKBONE + sh, (uint32_t)r);
+                att = u01(d.x) < p.backbone_move_p;
+                if (att) {
+                    const float delta = xmul(frange(d.y, -p.max_torsion_deg, p.max_torsion_deg), RADS_PER_DEG);
+                    S.bb_trig[r] = torsion_trig(delta);
+                }
+                S.bb_phi[r] = (int)((d.z >> 31) & 1u);
+                S.bb_u[r] = u01(d.w);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, att);
+            if (lane == 0) attw[w] = m;
+        }
+        // ---- 1. Langevin (diffusion.rs:306-339), interface test, move draws ----
+#pragma unroll 1
+        for (int base = warp * (32 / GL); base < n; base += RPP) {  // whole warps
+            const int gl = lane & (GL - 1);
+            const int r = base + lane / GL;
+            const bool live = r < n;
+            const int rr = live ? r : 0;
+            float4* row = S.pos + (size_t)rr * SLOT_STRIDE;
+            const F3 ca = f3(row[1]);
+            const int aa = S.aa[rr];
+            float4 cc = S.cgcentre[rr];
+            int nl = S.cgnl[rr];
+            {   // lists the residues' Calphas outran (a backbone move, the drift): rebuilt by the
+                // whole warp, one residue after another, with twice the skin
+                const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
+                const bool need = live && gl == 0 &&
+                                  (nl < 0 || !(mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f)));
+                const unsigned todo = __ballot_sync(0xffffffffu, need);
+                if (todo) {
+#pragma unroll 1
+                    for (unsigned m = todo; m; m &= m - 1) {
                         const int q = __ffs(m) - 1;
-                        const int rq = __shfl_sync(0xffffffffu, r, q);
-                        const F3 cq = {__shfl_sync(0xffffffffu, ca.x, q), __shfl_sync(0xffffffffu, ca.y, q),
-                                       __shfl_sync(0xffffffffu, ca.z, q)};
-                        const float sq = __shfl_sync(0xffffffffu, skin, q);
-                        const int nl = build_cg_list_warp<int>(A.ca_grid, A.ca_pq, cq, lane,
-                                                               S.cglist + (size_t)rq * CG_LIST_MAX, sq);
+                        const int rq = __shfl_sync(0xffffffffu, rr, q);
+                        const F3 cq = f3(S.pos[(size_t)rq * SLOT_STRIDE + 1]);
+                        const int nq = S.cgnl[rq];
+                        const float sq = nq < 0 ? CG_SKIN : fminf(2.0f * S.cgcentre[rq].w, CG_SKIN_MAX);
+                        __syncwarp();
+                        const int len = nag <= 65536 ? build_cg_list_warp<uint16_t>(A.ca_grid, A.ca_pq, cq, lane,
+                                                                                     S.cglist + (size_t)rq * CG_LIST_MAX, sq)
+                                                     : CG_LIST_MAX + 1;
                         if (lane == q) {
                             S.cgcentre[rq] = make_float4(cq.x, cq.y, cq.z, sq);
-                            S.cgnl[rq] = nl;
+                            S.cgnl[rq] = len;
                         }
                     }
                     __syncwarp();
+                    cc = S.cgcentre[rr];
+                    nl = S.cgnl[rr];
                 }
-                if (r >= n) continue;  // whole groups leave together
-                const F3 ca = f3(S.pos[r * SLOT_STRIDE + 1]);
-                if (gl == 0 && err && (!isfinite(ca.x) || !isfinite(ca.y) || !isfinite(ca.z))) atomicOr(err, ERRF_NAN);
-                const CgB body = cg_body(ca.x, ca.y, ca.z, S.aa[r]);
-                float fx, fy, fz;
-                if (lists) {
-                    // the group's scratch: the term slots of CG_LANES lanes
-                    unsigned char* scratch =
-                        (unsigned char*)(S.terms + (size_t)(tid / glanes) * CG_LANES * CG_SLOTS);
-                    group_cg_force_list<LW>(A, body, gl, gmask, S.cglist + (size_t)r * CG_LIST_MAX,
-                                            S.cgcentre + r, S.cgnl + r, (int*)(scratch + CG_IN_MAX * 16),
-                                            (float4*)scratch, fx, fy, fz);
-                } else {
-                    group_cg_force(A, body, gl, gmask, S.terms + (size_t)tid * CG_SLOTS, S.tcount + tid,
-                                   S.tcount + g0, S.terms + (size_t)g0 * CG_SLOTS, fx, fy, fz);
-                }
-                if (gl == 0) {
-                    if (FV) {  // VH-VL packing force: compute_forces over the partner's Calphas
-                        float px = 0.0f, py = 0.0f, pz = 0.0f;
-                        for (int i = 0; i < np; ++i) cg_term(body, S.pcq[i], S.pcp[i], px, py, pz);
-                        fx = xadd(fx, px);
-                        fy = xadd(fy, py);
-                        fz = xadd(fz, pz);
-                    }
-                    const float dx_c = xsub(ca.x, A.cx), dy_c = xsub(ca.y, A.cy), dz_c = xsub(ca.z, A.cz);
-                    const float d = fmaxf(xsqrt(xdist2(dx_c, dy_c, dz_c)), 0.001f);
-                    const float f_r = xdiv(xmul(-p.restraint_k, xsub(d, p.shell_radius)), d);
-                    fx = xadd(fx, xmul(f_r, dx_c));
-                    fy = xadd(fy, xmul(f_r, dy_c));
-                    fz = xadd(fz, xmul(f_r, dz_c));
-                    float nx = 0.f, ny = 0.f, nz = 0.f;
-                    if (with_noise) {
-                        const float sigma = xmul(p.noise_base, xsqrt(temp));
-                        const U4 u = rng_draw(p.seed, cid, step, STREAM_NOISE + sh, (uint32_t)r);
-                        nx = frange(u.x, -sigma, sigma);
-                        ny = frange(u.y, -sigma, sigma);
-                        nz = frange(u.z, -sigma, sigma);
-                    }
-                    const float md = p.max_disp;
-                    const F3 nca = {xadd(xadd(ca.x, fminf(fmaxf(xmul(p.step, fx), -md), md)), nx),
-                                    xadd(xadd(ca.y, fminf(fmaxf(xmul(p.step, fy), -md), md)), ny),
-                                    xadd(xadd(ca.z, fminf(fmaxf(xmul(p.step, fz), -md), md)), nz)};
-                    const F3 dl = sub3(nca, ca);
-                    S.ldelta[r] = make_float4(dl.x, dl.y, dl.z, 0.f);
-                    S.valid[r] = 0;
-                }
-                __syncwarp(gmask);  // the group's term slots are reused by the next pass
             }
-        }
-        if (tid == 0) {
-            S.iscal[IS_DVALID] = 0;  // disulfide energy stale
-            S.iscal[IS_NCYS] = 0;
-            S.iscal[IS_LASTCYS] = -1;
-            S.iscal[IS_NTASK] = 0;
-        }
-        __syncthreads();
-        for (int i = tid; i < n * SLOT_STRIDE; i += NT) {
-            const int r = i / SLOT_STRIDE, k = i % SLOT_STRIDE;
-            if (k < s_topo_n[S.aa[r]]) {
-                const float4 d = S.ldelta[r];
-                float4 v = S.pos[i];
-                v.x = xadd(v.x, d.x); v.y = xadd(v.y, d.y); v.z = xadd(v.z, d.z);
-                S.pos[i] = v;
+            if (live && gl == 0 && err && (!isfinite(ca.x) || !isfinite(ca.y) || !isfinite(ca.z)))
+                atomicOr(err, ERRF_NAN);
+            const float4 rl = S.res[aa];
+            const CgB body{ca.x, ca.y, ca.z, rl.x, rl.y, rl.z, rl.w};
+            float* xy = (float*)(S.prop + (size_t)rr * SLOT_STRIDE);  // the residue's proposal rows are free here
+            float* zi = (float*)(S.rej + (size_t)rr * SLOT_STRIDE);
+            float fx, fy, fz;
+            {
+                const GridView& g = A.ca_grid;
+                const int cx = cell_coord(ca.x, g.inv), cy = cell_coord(ca.y, g.inv), cz = cell_coord(ca.z, g.inv);
+                const bool walk = nl > CG_LIST_MAX || cell_far(cx, cy, cz);  // no usable list: the one-lane walk
+                // cells at least as wide as the cutoff: closer pairs are in adjacent cells (see k_langevin)
+                const float near_sq = g.cell >= 10.0f && fabsf(ca.x) < 1e4f && fabsf(ca.y) < 1e4f && fabsf(ca.z) < 1e4f
+                                          ? CG_NEAR_SQ : -1.0f;
+                const uint16_t* list = S.cglist + (size_t)rr * CG_LIST_MAX;
+                const float f = group_force<GL>(live && !walk ? nl : 0, list, A.ca_cell, cx, cy, cz, near_sq, body, cgq, cgp,
+                                                xy, zi);
+                fx = __shfl_sync(0xffffffffu, f, 0, GL);
+                fy = __shfl_sync(0xffffffffu, f, 1, GL);
+                fz = __shfl_sync(0xffffffffu, f, 2, GL);
+                if (__any_sync(0xffffffffu, live && walk)) {
+                    float wx = 0.0f, wy = 0.0f, wz = 0.0f;
+                    if (live && walk && gl == 0) cg_force(A, body, wx, wy, wz);
+                    __syncwarp();
+                    wx = __shfl_sync(0xffffffffu, wx, 0, GL);
+                    wy = __shfl_sync(0xffffffffu, wy, 0, GL);
+                    wz = __shfl_sync(0xffffffffu, wz, 0, GL);
+                    if (walk) {
+                        fx = wx;
+                        fy = wy;
+                        fz = wz;
+                    }
+                }
             }
-        }
-        __syncthreads();
-
-        // ---- 2. interface mask (diffusion.rs:343-351; Fv: CDR flags instead) + move draws ----
-        for (int r = warp; !FV && r < n; r += W) {
-            const F3 ca = f3(S.pos[r * SLOT_STRIDE + 1]);
-            bool hit = false;
-            for (int base = 0; base < nag && !hit; base += 64) {
-                bool h = false;
+            if (FV) {  // VH-VL packing force: compute_forces over the partner's Calphas
+                const float f = group_force<GL>(live ? np : 0, nullptr, nullptr, 0, 0, 0, 0.0f, body, S.pcq,
+                                                S.pcp, xy, zi);
+                fx = xadd(fx, __shfl_sync(0xffffffffu, f, 0, GL));
+                fy = xadd(fy, __shfl_sync(0xffffffffu, f, 1, GL));
+                fz = xadd(fz, __shfl_sync(0xffffffffu, f, 2, GL));
+            }
+            const float dx_c = xsub(ca.x, A.cx), dy_c = xsub(ca.y, A.cy), dz_c = xsub(ca.z, A.cz);
+            const float d = fmaxf(xsqrt(xdist2(dx_c, dy_c, dz_c)), 0.001f);
+            const float f_r = xdiv(xmul(-p.restraint_k, xsub(d, p.shell_radius)), d);
+            fx = xadd(fx, xmul(f_r, dx_c));
+            fy = xadd(fy, xmul(f_r, dy_c));
+            fz = xadd(fz, xmul(f_r, dz_c));
+            // one generator call per lane: lane 1 of the group draws the residue's move, the
+            // others its noise
+            const U4 u = step_draw(p.seed, cid, step, (gl == 1 ? STREAM_MC : STREAM_NOISE) + sh, (uint32_t)r);
+            const U4 dm = {__shfl_sync(0xffffffffu, u.x, 1, GL), __shfl_sync(0xffffffffu, u.y, 1, GL),
+                           __shfl_sync(0xffffffffu, u.z, 1, GL), __shfl_sync(0xffffffffu, u.w, 1, GL)};
+            float nx = 0.f, ny = 0.f, nz = 0.f;
+            if (with_noise) {
+                const float sigma = xmul(p.noise_base, xsqrt(temp));
+                nx = frange(__shfl_sync(0xffffffffu, u.x, 0, GL), -sigma, sigma);
+                ny = frange(__shfl_sync(0xffffffffu, u.y, 0, GL), -sigma, sigma);
+                nz = frange(__shfl_sync(0xffffffffu, u.z, 0, GL), -sigma, sigma);
+            }
+            const float md = p.max_disp;
+            const F3 nca = {xadd(xadd(ca.x, fminf(fmaxf(xmul(p.step, fx), -md), md)), nx),
+                            xadd(xadd(ca.y, fminf(fmaxf(xmul(p.step, fy), -md), md)), ny),
+                            xadd(xadd(ca.z, fminf(fmaxf(xmul(p.step, fz), -md), md)), nz)};
+            // set_ca_pos: delta = new - old; every atom (the Calpha included) += delta
+            const F3 dl = sub3(nca, ca);
+            const F3 cn = {xadd(ca.x, dl.x), xadd(ca.y, dl.y), xadd(ca.z, dl.z)};
+            if (live) {
+                const int n_at = S.topo_n[aa];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int i = base + u * 32 + lane;
-                    if (i < nag) {
-                        const float4 a = agq[i];
-                        h |= xdist2(xsub(ca.x, a.x), xsub(ca.y, a.y), xsub(ca.z, a.z)) < p.iface_cutoff_sq;
+                for (int k = gl; k < SLOT_STRIDE; k += GL)
+                    if (k < n_at) {
+                        float4 v = row[k];
+                        v.x = xadd(v.x, dl.x);
+                        v.y = xadd(v.y, dl.y);
+                        v.z = xadd(v.z, dl.z);
+                        row[k] = v;
                     }
-                }
-                hit = __any_sync(0xffffffffu, h);
             }
-            if (lane == 0) S.iface[r] = hit;
-        }
-        for (int r = tid; r < n; r += NT) {
-            const U4 d = rng_draw(p.seed, cid, step, STREAM_BACKBONE + sh, (uint32_t)r);
-            const bool att = u01(d.x) < p.backbone_move_p;
-            S.bb_att[r] = att;
-            if (att) {
-                const float delta = xmul(frange(d.y, -p.max_torsion_deg, p.max_torsion_deg), RADS_PER_DEG);
-                S.bb_trig[r] = make_float4(mc_cos(delta), mc_sin(delta), mc_cos(-delta), mc_sin(-delta));
-            }
-            S.bb_phi[r] = (int)((d.z >> 31) & 1u);
-            S.bb_u[r] = u01(d.w);
-            S.sel[r] = SEL_KEEP;
-        }
-        __syncthreads();
-
-        // ---- 3. mutation / rotamer proposals (diffusion.rs:354-399) ----
-        for (int r = tid; r < n; r += NT) {
-            const U4 d = rng_draw(p.seed, cid, step, STREAM_MC + sh, (uint32_t)r);
-            const int aa = S.aa[r];
-            int kind = MV_NONE;
-            if (FV) {
-                // CDR positions: mutation / rotamer moves (MUTATION_P * 3, ROTAMER_MOVE_P * 2);
-                // every residue without one: rotamer relaxation (ROTAMER_MOVE_P * 0.3)
-                if (fv_cdr[r0 + r] && u01(d.x) < xmul(p.mutation_p, 3.0f)) {
-                    if (u01(d.y) < xmul(p.rotamer_move_p, 2.0f)) {
-                        if (s_rot_n[aa] > 0) kind = MV_ROT;
-                    } else {
-                        kind = MV_MUT;
-                    }
-                } else if (u01(d.y) < xmul(p.rotamer_move_p, 0.3f) && s_rot_n[aa] > 0) {
-                    kind = MV_ROT;
+            // interface residue (diffusion.rs:343-351), where the move's draw depends on it: from
+            // the list while it reaches far enough around the moved Calpha, else from all
+            // antigen Calphas
+            bool itf = false;
+            if (!FV) {
+                const float mx = cn.x - cc.x, my = cn.y - cc.y, mz = cn.z - cc.z;
+                const float reach = 10.0f + cc.w - 0.01f - sqrtf(mx * mx + my * my + mz * mz);
+                const bool listed = nl <= CG_LIST_MAX && reach > 0.0f && p.iface_cutoff_sq <= reach * reach;
+                const uint16_t* list = S.cglist + (size_t)rr * CG_LIST_MAX;
+                const bool asked = live && u01(dm.x) < fmaxf(xmul(p.mutation_p, 3.0f), xmul(p.mutation_p, 0.4f));
+                const int cnt = asked ? (listed ? nl : nag) : 0;
+                const int mxc = __reduce_max_sync(0xffffffffu, cnt);
+#pragma unroll 1
+                for (int j = gl; j < mxc; j += GL) {
+                    if (j >= cnt) continue;
+                    const float4 a = cgq[listed ? (int)list[j] : j];
+                    itf |= xdist2(xsub(cn.x, a.x), xsub(cn.y, a.y), xsub(cn.z, a.z)) < p.iface_cutoff_sq;
                 }
-                if (kind == MV_ROT) {
-                    S.new_rot[r] = (int)urange(d.z, (uint32_t)s_rot_n[aa]);
-                    S.new_aa[r] = aa;
-                } else if (kind == MV_MUT) {
-                    S.new_aa[r] = (int)urange(d.z, (uint32_t)N_AA);
-                    S.new_rot[r] = 0;
-                }
+                __syncwarp();
+                const unsigned m = __ballot_sync(0xffffffffu, itf) >> (lane & ~(GL - 1));
+                itf = (m & ((1u << GL) - 1u)) != 0u;
             }
-            const bool itf = !FV && S.iface[r] != 0;
-            const float eff_mut_p = itf ? xmul(p.mutation_p, 3.0f) : xmul(p.mutation_p, 0.4f);
-            const float eff_rot_p = itf ? xmul(p.rotamer_move_p, 2.0f) : p.rotamer_move_p;
-            if (!FV && u01(d.x) < eff_mut_p) {
-                if (u01(d.y) < eff_rot_p) {
-                    if (s_rot_n[aa] > 0) {
+            // mutation / rotamer proposal (diffusion.rs:354-399)
+            if (live && gl == 0) {
+                int kind = MV_NONE, new_aa = aa, new_rot = 0;
+                if (FV) {
+                    // CDR positions: mutation / rotamer moves (MUTATION_P * 3, ROTAMER_MOVE_P * 2);
+                    // every residue without one: rotamer relaxation (ROTAMER_MOVE_P * 0.3)
+                    if (fv_cdr[r0 + r] && u01(dm.x) < xmul(p.mutation_p, 3.0f)) {
+                        if (u01(dm.y) < xmul(p.rotamer_move_p, 2.0f)) {
+                            if (S.rot_n[aa] > 0) kind = MV_ROT;
+                        } else {
+                            kind = MV_MUT;
+                        }
+                    } else if (u01(dm.y) < xmul(p.rotamer_move_p, 0.3f) && S.rot_n[aa] > 0) {
                         kind = MV_ROT;
-                        S.new_rot[r] = (int)urange(d.z, (uint32_t)s_rot_n[aa]);
-                        S.new_aa[r] = aa;
                     }
                 } else {
-                    kind = MV_MUT;
-                    S.new_aa[r] = (int)urange(d.z, (uint32_t)N_AA);
-                    S.new_rot[r] = 0;
+                    const float eff_mut_p = itf ? xmul(p.mutation_p, 3.0f) : xmul(p.mutation_p, 0.4f);
+                    const float eff_rot_p = itf ? xmul(p.rotamer_move_p, 2.0f) : p.rotamer_move_p;
+                    if (u01(dm.x) < eff_mut_p) {
+                        if (u01(dm.y) < eff_rot_p) {
+                            if (S.rot_n[aa] > 0) kind = MV_ROT;
+                        } else {
+                            kind = MV_MUT;
+                        }
+                    }
                 }
-            }
-            S.kind[r] = kind;
-            S.u_acc[r] = u01(d.w);
-            if (EXT) {
-                S.dz[r] = d.z;
-                S.lhr[r] = 0.0;
-            }
-            if (aa == CYS) atomicAdd(&S.iscal[IS_NCYS], 1);
-            if (kind != MV_NONE) {  // its two energy tasks (in any order: each writes its own results)
-                const int k = atomicAdd(&S.iscal[IS_NTASK], 2);
-                S.tcount[k] = 2 * r;  // the Langevin step's term counts are free until the next step
-                S.tcount[k + 1] = 2 * r + 1;
+                if (kind == MV_ROT) new_rot = (int)urange(dm.z, (uint32_t)S.rot_n[aa]);
+                else if (kind == MV_MUT) new_aa = (int)urange(dm.z, (uint32_t)N_AA);
+                S.kind[r] = kind;
+                S.new_aa[r] = new_aa;
+                S.new_rot[r] = new_rot;
+                S.sel[r] = SEL_KEEP;
+                S.u_acc[r] = u01(dm.w);
+                if (EXT) {
+                    S.dz[r] = dm.z;
+                    S.lhr[r] = 0.0;
+                }
+                if (kind != MV_NONE) {  // its two tasks (in any order: each writes its own results)
+                    if (aa == CYS || new_aa == CYS) S.iscal[IS_CYSMV] = 1;
+                    const int k = atomicAdd(&S.iscal[IS_NTASK], 2);
+                    S.task[k] = 2 * r;
+                    S.task[k + 1] = 2 * r + 1;
+                }
             }
         }
         __syncthreads();
         // learned proposal: the choice of each drawn move comes from the network
         // (same draw d.z, inverse CDF) and the move carries its Hastings ratio
-        if (EXT && learned && temp <= mlp.t_max)
-            an_learned_choices(an_smem, R, G, C, n, agq, staged ? S.agaa : A.res_aa, nag, mlp, temp);
-        // proposals and rejection rebuilds on the upper half of the warps (two threads per
-        // residue), the Calpha energies before / after each move on the lower half, the
-        // listed tasks dealt one per warp in turn
-        if (warp >= W / 2) {
-            for (int t = tid - NT / 2; t < 2 * n; t += NT / 2) {
-                const int r = t >> 1;
-                if (S.kind[r] != MV_NONE) build_move(S, r, (t & 1) ? SEL_REJ : SEL_PROP);
-            }
-        } else {
+        if constexpr (L::LRN) {
+            if (learned && temp <= mlp.t_max) an_learned_choices<L>(n, mlp, temp);
+        }
+        // ---- 2. proposals and rejection rebuilds on the last two warps (four lanes each), on
+        // the others the Calpha energies before / after each move and those of the residues
+        // the first backbone move starts from; without a Cys among the moves the decisions
+        // need no built atom and follow the energies while the builds still run ----
+        const bool cysmv = S.iscal[IS_CYSMV] != 0;
+        int first_att = n;
+#pragma unroll 1
+        for (int w = words - 1; w >= 0; --w)
+            if (const unsigned m = attw[w]) first_att = w * 32 + __ffs(m) - 1;
+        {
             const int ntask = S.iscal[IS_NTASK];
-            for (int k = warp; k < ntask; k += W / 2) {
-                const int t = S.tcount[k];
-                const int r = t >> 1, which = t & 1;
-                const int kind = S.kind[r];
-                const bool same = kind == MV_ROT || S.new_aa[r] == S.aa[r];
-                if (which == 1 && same) continue;  // same Calpha, same amino acid: same energy
-                const int a = which ? S.new_aa[r] : S.aa[r];
-                const ACC e = ca_energy(f3(S.pos[r * SLOT_STRIDE + 1]), a);
+            if (warp >= EW) {  // proposals on one, rejections on the other
+#pragma unroll 1
+                for (int k0 = warp - EW; k0 < ntask; k0 += 8 * BW) {
+                    const int k = k0 + BW * (lane >> 2);
+                    const int t = S.task[k < ntask ? k : 0];
+                    build_move(S, t >> 1, (t & 1) ? SEL_REJ : SEL_PROP, k < ntask);
+                }
+            } else {
+                run_tasks(
+                    0, EW, ntask + (n - first_att),
+                    [&](int k, int& r, int& a) {
+                        if (k >= ntask) {
+                            r = first_att + (k - ntask);
+                            a = S.aa[r];
+                            return S.kind[r] == MV_NONE;
+                        }
+                        const int t = S.task[k];
+                        r = t >> 1;
+                        const int oa = S.aa[r];
+                        a = t & 1 ? S.new_aa[r] : oa;
+                        return !((t & 1) && a == oa);  // same Calpha, same amino acid: same energy
+                    },
+                    [&](int k, double e) {
+                        if (k >= ntask) {
+                            S.c_cur[first_att + (k - ntask)] = e;
+                            return;
+                        }
+                        const int t = S.task[k], r = t >> 1;
+                        if (t & 1) {
+                            S.c_new[r] = e;
+                        } else {
+                            S.c_old[r] = e;
+                            if (S.new_aa[r] == S.aa[r]) S.c_new[r] = e;
+                        }
+                    });
+            }
+        }
+        if (cysmv) __syncthreads();
+        else if (warp < EW) asm volatile("bar.sync 1, %0;" ::"n"(EW * 32) : "memory");
+        // the sweep's decisions, by warp 0 (applied after the barrier: the builds still read
+        // the state)
+        if (warp == 0) {
+            int ncys = 0;
+            bool any = first_att < n;  // a backbone move needs the disulfide energy too
+#pragma unroll 1
+            for (int w = 0; w < words; ++w) {
+                const int r = w * 32 + lane;
+                const int kd = r < n ? S.kind[r] : MV_NONE;
+                const bool cys = r < n && S.aa[r] == CYS;
+                const bool mc = kd != MV_NONE && (cys || S.new_aa[r] == CYS);
+                const unsigned bc = __ballot_sync(0xffffffffu, cys), bx = __ballot_sync(0xffffffffu, mc);
+                any |= __any_sync(0xffffffffu, kd != MV_NONE);
                 if (lane == 0) {
-                    if (which == 0) {
-                        S.c_old[r] = (double)e;
-                        if (same) S.c_new[r] = (double)e;
-                    } else {
-                        S.c_new[r] = (double)e;
-                    }
+                    S.cysw[w] = bc;
+                    S.mxw[w] = bx;
                 }
+                ncys += __popc(bc);
             }
-        }
-        __syncthreads();
-        // the sweep's decisions, in residue order; moves without a Cys are deferred to
-        // the parallel pass below, except while the proposal log is written (its
-        // records keep residue order within a candidate)
-        const bool defer = !EXT || !tlog;
-        if (tid == 0) {
-            int ncys = S.iscal[IS_NCYS];
-            bool have_d = false;
+            __syncwarp();
             ACC D = 0;
-            for (int r = 0; r < n; ++r) {
-                const int kind = S.kind[r];
-                if (kind == MV_NONE) continue;
-                if (!have_d) {
-                    D = ncys >= 2 ? disulfide_of<ACC, true>(S, n, -1, nullptr, 0) : (ACC)0;
-                    have_d = true;
-                }
-                const int oa = S.aa[r];
-                const int na = kind == MV_MUT ? S.new_aa[r] : oa;
-                const bool cys = oa == CYS || na == CYS;
-                if (defer && !cys) {  // decided in parallel below, with the disulfide energy of its turn
-                    S.d_turn[r] = (double)D;
-                    continue;
-                }
-                const int ncys_new = ncys + (na == CYS) - (oa == CYS);
-                ACC Dn = D;
-                if (cys)
-                    Dn = ncys_new >= 2 ? disulfide_of<ACC, true>(S, n, r, S.prop + (size_t)r * SLOT_STRIDE, na)
-                                       : (ACC)0;
-                const ACC old_e = (ACC)S.c_old[r] + D;
-                const ACC new_e = (ACC)S.c_new[r] + Dn;
-                const double lhr = EXT ? S.lhr[r] : 0.0;
-                const bool acc = EXT ? mh_accept(new_e - old_e, temp, S.u_acc[r], lhr)
-                                     : metropolis(new_e - old_e, temp, S.u_acc[r]);
+            if (any && ncys >= 2)
+                D = warp_disulfide<L, ACC>(true, words, -1);
+            auto settle = [&](int r, bool side, bool acc, ACC de) {  // one lane
                 ++n_mc;
                 n_mc_acc += acc;
-                if (EXT && tlog) {
-                    const unsigned long long slot = atomicAdd(log_n, 1ull);
-                    if ((long long)slot < log_cap) {
-                        const float4 ca = S.pos[r * SLOT_STRIDE + 1];
-                        MlpTuple t;
-                        t.x = ca.x; t.y = ca.y; t.z = ca.z;
-                        t.delta_e = (float)(new_e - old_e);
-                        t.cand = c;
-                        t.log_ratio = (float)lhr;
-                        t.residue = (int16_t)r;
-                        t.aa = (uint8_t)oa;
-                        t.action = (uint8_t)(kind == MV_MUT ? na : N_AA + S.new_rot[r]);
-                        t.antigen = (uint8_t)st.cand_ag[c];
-                        t.accepted = acc ? 1 : 0;
-                        t.pad[0] = t.pad[1] = 0;
-                        tlog[slot] = t;
+                if (EXT && tlog) S.d_turn[r] = (double)de;
+                S.sel[r] = (acc ? SEL_PROP : SEL_REJ) | (side ? SEL_SIDE : 0);
+                S.c_cur[r] = acc ? S.c_new[r] : S.c_old[r];
+            };
+#pragma unroll 1
+            for (int w = 0; w < words; ++w) {  // moves without a Cys: the disulfide energy of their turn
+                const int r = w * 32 + lane;
+                if (r < n) S.d_turn[r] = (double)D;
+            }
+#pragma unroll 1
+            for (int wx = 0; wx < words; ++wx)
+#pragma unroll 1
+                for (unsigned x = S.mxw[wx]; x; x &= x - 1) {  // the moves that involve a Cys, in residue order
+                    const int r = wx * 32 + __ffs(x) - 1;
+                    const unsigned bit = 1u << (r & 31);
+                    const int kind = S.kind[r], oa = S.aa[r], na = S.new_aa[r];
+                    const int ncys_new = ncys + (na == CYS) - (oa == CYS);
+                    ACC Dn = 0;
+                    __syncwarp();
+                    if (lane == 0) S.cysw[wx] = na == CYS ? S.cysw[wx] | bit : S.cysw[wx] & ~bit;
+                    __syncwarp();
+                    if (ncys_new >= 2)
+                        Dn = warp_disulfide<L, ACC>(true, words, r);
+                    const ACC old_e = (ACC)S.c_old[r] + D;
+                    const ACC new_e = (ACC)S.c_new[r] + Dn;
+                    const double lhr = EXT ? S.lhr[r] : 0.0;
+                    const bool acc = mh_accept(new_e - old_e, temp, S.u_acc[r], lhr);
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (!acc) S.cysw[wx] = oa == CYS ? S.cysw[wx] | bit : S.cysw[wx] & ~bit;
+                        settle(r, kind == MV_ROT || na == oa, acc, new_e - old_e);
+                    }
+                    __syncwarp();
+                    if (acc) {
+                        D = Dn;
+                        ncys = ncys_new;
+                    } else if (oa == CYS && ncys >= 2) {  // SG rebuilt
+                        D = warp_disulfide<L, ACC>(true, words, -1);
+                    }
+#pragma unroll 1
+                    for (int w = wx; w < words; ++w) {
+                        const int q = w * 32 + lane;
+                        if (q > r && q < n) S.d_turn[q] = (double)D;
                     }
                 }
-                if (acc) {
-                    if (EXT) S.rot[r] = kind == MV_ROT ? S.new_rot[r] : (s_rot_n[na] > 0 ? 0 : -1);
-                    S.sel[r] = SEL_PROP;
-                    S.aa[r] = na;
-                    const int rot = S.new_rot[r];
-                    const bool has = s_rot_n[na] > 0;
-                    S.chi[r] = has ? s_rot_chi[na][rot] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const ChiTrig t = has ? rot_trig(na, rot) : zero_trig();
-                    S.trig[2 * r] = make_float4(t.t[0].x, t.t[0].y, t.t[1].x, t.t[1].y);
-                    S.trig[2 * r + 1] = make_float4(t.t[2].x, t.t[2].y, t.t[3].x, t.t[3].y);
-                    S.c_cur[r] = S.c_new[r];
-                    D = Dn;
-                    ncys = ncys_new;
-                } else {
-                    S.sel[r] = SEL_REJ;
-                    S.c_cur[r] = S.c_old[r];
-                    if (oa == CYS && ncys >= 2) D = disulfide_of<ACC, true>(S, n, -1, nullptr, 0);  // SG rebuilt
-                }
-                S.valid[r] = 1;
+#pragma unroll 1
+            for (int w = 0; w < words; ++w) {  // the others, each by its lane
+                const int r = w * 32 + lane;
+                const int kind = r < n ? S.kind[r] : MV_NONE;
+                if (kind == MV_NONE || (S.mxw[w] >> lane & 1u)) continue;
+                const int na = S.new_aa[r];
+                const ACC Dr = (ACC)S.d_turn[r];
+                const ACC old_e = (ACC)S.c_old[r] + Dr;
+                const ACC new_e = (ACC)S.c_new[r] + Dr;
+                const double lhr = EXT ? S.lhr[r] : 0.0;
+                const bool acc = mh_accept(new_e - old_e, temp, S.u_acc[r], lhr);
+                settle(r, kind == MV_ROT || na == S.aa[r], acc, new_e - old_e);
             }
-            if (have_d) {
-                S.dscal[0] = (double)D;
-                S.iscal[IS_DVALID] = 1;
+            __syncwarp();
+            if (EXT && tlog) {  // the log: this step's decisions in residue order
+                int total = 0;
+#pragma unroll 1
+                for (int w = 0; w < words; ++w) {
+                    const int r = w * 32 + lane;
+                    total += __popc(__ballot_sync(0xffffffffu, r < n && S.kind[r] != MV_NONE));
+                }
+                unsigned long long slot = 0;
+                if (lane == 0 && total) slot = atomicAdd(log_n, (unsigned long long)total);
+                slot = __shfl_sync(0xffffffffu, slot, 0);
+#pragma unroll 1
+                for (int w = 0; w < words; ++w) {
+                    const int r = w * 32 + lane;
+                    const int kind = r < n ? S.kind[r] : MV_NONE;
+                    const unsigned m = __ballot_sync(0xffffffffu, kind != MV_NONE);
+                    const long long at = (long long)slot + __popc(m & ((1u << lane) - 1u));
+                    slot += __popc(m);
+                    if (kind == MV_NONE || at >= log_cap) continue;
+                    const float4 ca = S.pos[r * SLOT_STRIDE + 1];
+                    MlpTuple t;
+                    t.x = ca.x; t.y = ca.y; t.z = ca.z;
+                    t.delta_e = (float)(ACC)S.d_turn[r];
+                    t.cand = c;
+                    t.log_ratio = (float)S.lhr[r];
+                    t.residue = (int16_t)r;
+                    t.aa = (uint8_t)S.aa[r];
+                    t.action = (uint8_t)(kind == MV_MUT ? S.new_aa[r] : N_AA + S.new_rot[r]);
+                    t.antigen = (uint8_t)st.cand_ag[c];
+                    t.accepted = (S.sel[r] & 3) == SEL_PROP ? 1 : 0;
+                    t.pad[0] = t.pad[1] = 0;
+                    tlog[at] = t;
+                }
+            }
+            if (lane == 0) {
+                S.dscal = (double)D;
+                S.iscal[IS_DVALID] = any;
             }
         }
         __syncthreads();
-        if (defer) {
-            // the moves that involve no Cys leave the disulfide energy as it is, so each
-            // is decided on its own with the disulfide energy current at its turn (the
-            // loop above recorded it): the same decisions as the sequential sweep
-            for (int r = tid; r < n; r += NT) {
-                const int kind = S.kind[r];
-                if (kind == MV_NONE || S.valid[r]) continue;  // valid: decided above (Cys)
-                const int oa = S.aa[r];
-                const int na = kind == MV_MUT ? S.new_aa[r] : oa;
-                const ACC D = (ACC)S.d_turn[r];
-                const ACC old_e = (ACC)S.c_old[r] + D;
-                const ACC new_e = (ACC)S.c_new[r] + D;
-                const bool acc = EXT ? mh_accept(new_e - old_e, temp, S.u_acc[r], S.lhr[r])
-                                     : metropolis(new_e - old_e, temp, S.u_acc[r]);
-                ++n_mc;
-                n_mc_acc += acc;
-                if (acc) {
-                    if (EXT) S.rot[r] = kind == MV_ROT ? S.new_rot[r] : (s_rot_n[na] > 0 ? 0 : -1);
-                    S.sel[r] = SEL_PROP;
-                    S.aa[r] = na;
-                    const int rot = S.new_rot[r];
-                    const bool has = s_rot_n[na] > 0;
-                    S.chi[r] = has ? s_rot_chi[na][rot] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    const ChiTrig t = has ? rot_trig(na, rot) : zero_trig();
-                    S.trig[2 * r] = make_float4(t.t[0].x, t.t[0].y, t.t[1].x, t.t[1].y);
-                    S.trig[2 * r + 1] = make_float4(t.t[2].x, t.t[2].y, t.t[3].x, t.t[3].y);
-                    S.c_cur[r] = S.c_new[r];
-                } else {
-                    S.sel[r] = SEL_REJ;
-                    S.c_cur[r] = S.c_old[r];
-                }
-                S.valid[r] = 1;
-            }
-            __syncthreads();
-        }
+#pragma unroll 1
         for (int i = tid; i < n * SLOT_STRIDE; i += NT) {
-            const int r = i / SLOT_STRIDE;
+            const int r = i / SLOT_STRIDE, k = i % SLOT_STRIDE;
             const int sl = S.sel[r];
-            if (sl == SEL_PROP) S.pos[i] = S.prop[i];
-            else if (sl == SEL_REJ) S.pos[i] = S.rej[i];
-            if ((i % SLOT_STRIDE) == 0 && S.aa[r] == CYS) atomicMax(&S.iscal[IS_LASTCYS], r);
+            if (sl == SEL_KEEP) continue;
+            if (sl & SEL_SIDE) {
+                const int a = S.aa[r];
+                if (k < 4 + (a != GLY ? 1 : 0) || k >= S.topo_n[a]) continue;
+            }
+            S.pos[i] = (sl & SEL_PROP ? S.prop : S.rej)[i];
         }
+#pragma unroll 1
+        for (int r = tid; r < n; r += NT) {  // accepted moves (side-chain-only ones keep the amino acid)
+            if ((S.sel[r] & 3) != SEL_PROP) continue;
+            const int na = S.new_aa[r], rot = S.new_rot[r];
+            const bool has = S.rot_n[na] > 0;
+            if (EXT) S.rot[r] = S.kind[r] == MV_ROT ? rot : (has ? 0 : -1);
+            S.aa[r] = na;
+            S.chi[r] = has ? s_rot_chi[na][rot] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float2* t = S.rott + (has ? (na * 5 + rot) * 4 : N_AA * 20);
+            S.trig[2 * r] = make_float4(t[0].x, t[0].y, t[1].x, t[1].y);
+            S.trig[2 * r + 1] = make_float4(t[2].x, t[2].y, t[3].x, t[3].y);
+        }
+        if (tid == 0) S.iscal[IS_NTASK] = S.iscal[IS_CYSMV] = 0;
         __syncthreads();
 
-        // ---- 4. backbone phi/psi moves (diffusion.rs:403-418) ----
-        const int last_cys = S.iscal[IS_LASTCYS];
-        for (int r = 0; r < n; ++r) {
-            if (!S.bb_att[r]) continue;
-            const bool phi = S.bb_phi[r] != 0;
-            const bool cys_down = r <= last_cys;  // a Cys at or after r: the disulfide term can change
-            // Calpha energies of residues r..n at the current positions, and the
-            // disulfide energy
-            if (tid == 0 && !S.iscal[IS_DVALID]) {
-                S.dscal[0] = (double)disulfide_of<ACC, false>(S, n, -1, nullptr, 0);
-                S.iscal[IS_DVALID] = 1;
-            }
-            for (int i = r + warp; i < n; i += W) {
-                if (S.valid[i]) continue;
-                const ACC e = ca_energy(f3(S.pos[i * SLOT_STRIDE + 1]), S.aa[i]);
-                if (lane == 0) {
-                    S.c_cur[i] = (double)e;
-                    S.valid[i] = 1;
+        // ---- 3. backbone phi/psi moves (diffusion.rs:403-418) ----
+        int last_cys = -1, stale = n;  // stale: residues from here on have no current Calpha energy
+        if (first_att < n)
+#pragma unroll 1
+            for (int w = 0; w < words; ++w)
+                if (const unsigned m = S.cysw[w]) last_cys = w * 32 + 31 - __clz(m);
+#pragma unroll 1
+        for (int wa = first_att < n ? first_att >> 5 : words; wa < words; ++wa)
+#pragma unroll 1
+            for (unsigned at = attw[wa]; at; at &= at - 1) {
+                const int r = wa * 32 + __ffs(at) - 1;
+                const bool phi = S.bb_phi[r] != 0;
+                const bool cys_down = r <= last_cys;  // a Cys at or after r: the disulfide term can change
+                if (stale < n) {  // after a rejected move: energies of residues r..n, and the disulfide energy
+                    if (warp == W - 1 && !S.iscal[IS_DVALID]) {
+                        const ACC D = warp_disulfide<L, ACC>(false, words, -1);
+                        if (lane == 0) {
+                            S.dscal = (double)D;
+                            S.iscal[IS_DVALID] = 1;
+                        }
+                    }
+                    run_tasks(
+                        0, W, n - r,
+                        [&](int k, int& i, int& a) {
+                            i = r + k;
+                            a = S.aa[i];
+                            return true;
+                        },
+                        [&](int k, double e) { S.c_cur[r + k] = e; });
+                    stale = n;
+                    __syncthreads();
                 }
-            }
-            __syncthreads();
-            ACC old_e = 0;
-            if (tid == 0) {
-                for (int i = r; i < n; ++i) old_e += (ACC)S.c_cur[i];
-                old_e += (ACC)S.dscal[0];
-            }
-            const float4 bt = S.bb_trig[r];
-            rotate_downstream(S, n, r, phi, bt.x, bt.y);
-            __syncthreads();
-            for (int i = r + 1 + warp; i < n; i += W) {
-                const ACC e = ca_energy(f3(S.pos[i * SLOT_STRIDE + 1]), S.aa[i]);
-                if (lane == 0) S.c_new[i] = (double)e;
-            }
-            __syncthreads();
-            if (tid == 0) {
-                const ACC Dn = cys_down ? disulfide_of<ACC, false>(S, n, -1, nullptr, 0) : (ACC)S.dscal[0];
-                ACC new_e = 0;
-                new_e += (ACC)S.c_cur[r];
-                for (int i = r + 1; i < n; ++i) new_e += (ACC)S.c_new[i];
-                new_e += Dn;
-                const bool acc = metropolis(new_e - old_e, temp, S.bb_u[r]);
-                ++n_bb;
-                n_bb_acc += acc;
-                if (acc) {
-                    for (int i = r + 1; i < n; ++i) S.c_cur[i] = S.c_new[i];
-                    S.dscal[0] = (double)Dn;
+                const float4 bt = S.bb_trig[r];
+                rotate_downstream<L>(n, r, phi, bt.x, bt.y);
+                __syncthreads();
+                run_tasks(
+                    0, W, n - r - 1,
+                    [&](int k, int& i, int& a) {
+                        i = r + 1 + k;
+                        a = S.aa[i];
+                        return true;
+                    },
+                    [&](int k, double e) { S.c_new[r + 1 + k] = e; });
+                __syncthreads();
+                if (warp == 0) {
+                    ACC Dn = (ACC)S.dscal;
+                    if (cys_down)
+                        Dn = warp_disulfide<L, ACC>(false, words, -1);
+                    bool acc;
+                    if constexpr (F32) {  // the reference's sequential f32 sums, on every lane
+                        ACC old_e = 0, new_e = 0;
+#pragma unroll 1
+                        for (int i = r; i < n; ++i) old_e += (ACC)S.c_cur[i];
+                        old_e += (ACC)S.dscal;
+                        new_e += (ACC)S.c_cur[r];
+#pragma unroll 1
+                        for (int i = r + 1; i < n; ++i) new_e += (ACC)S.c_new[i];
+                        new_e += Dn;
+                        acc = mh_accept(new_e - old_e, temp, S.bb_u[r], 0.0);
+                    } else {
+                        double old_e = 0.0, new_e = 0.0;
+#pragma unroll 1
+                        for (int i = r + lane; i < n; i += 32) {
+                            old_e += S.c_cur[i];
+                            new_e += i == r ? S.c_cur[i] : S.c_new[i];
+                        }
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) {
+                            old_e += __shfl_xor_sync(0xffffffffu, old_e, o);
+                            new_e += __shfl_xor_sync(0xffffffffu, new_e, o);
+                        }
+                        acc = mh_accept((new_e + (double)Dn) - (old_e + S.dscal), temp, S.bb_u[r], 0.0);
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        ++n_bb;
+                        n_bb_acc += acc;
+                        if (acc) S.dscal = (double)Dn;
+                        else if (cys_down) S.iscal[IS_DVALID] = 0;
+                        S.iscal[IS_DECISION] = acc;
+                    }
+                }
+                __syncthreads();
+                if (S.iscal[IS_DECISION]) {
+#pragma unroll 1
+                    for (int i = r + 1 + tid; i < n; i += NT) S.c_cur[i] = S.c_new[i];
                 } else {
-                    for (int i = r + 1; i < n; ++i) S.valid[i] = 0;
-                    if (cys_down) S.iscal[IS_DVALID] = 0;
+                    rotate_downstream<L>(n, r, phi, bt.z, bt.w);
+                    stale = r + 1;
                 }
-                S.iscal[IS_DECISION] = acc;
-            }
-            __syncthreads();
-            if (!S.iscal[IS_DECISION]) {
-                rotate_downstream(S, n, r, phi, bt.z, bt.w);
                 __syncthreads();
             }
-        }
     }
 
+#pragma unroll 1
     for (int i = tid; i < n * SLOT_STRIDE; i += NT) st.res_pos[(size_t)r0 * SLOT_STRIDE + i] = S.pos[i];
+#pragma unroll 1
     for (int r = tid; r < n; r += NT) {
         st.res_aa[r0 + r] = (uint8_t)S.aa[r];
         st.res_chi[r0 + r] = S.chi[r];
         st.res_trig[2 * (r0 + r)] = S.trig[2 * r];
         st.res_trig[2 * (r0 + r) + 1] = S.trig[2 * r + 1];
     }
-    if (stats && (n_mc || n_bb)) {  // the decisions are spread over the threads
+    if (stats && (n_mc || n_bb)) {  // the decisions are spread over the lanes of warp 0
         atomicAdd((unsigned long long*)&stats[4 * c], (unsigned long long)n_mc);
         atomicAdd((unsigned long long*)&stats[4 * c + 1], (unsigned long long)n_mc_acc);
         atomicAdd((unsigned long long*)&stats[4 * c + 2], (unsigned long long)n_bb);
@@ -1298,55 +1581,57 @@ void launch_mc_energy(cudaStream_t s, const StateView& st, const AgView* ags, do
     if (st.n_cand > 0) k_mc_energy<<<st.n_cand, AN_THREADS, 0, s>>>(st, ags, out);
 }
 
-size_t anneal_smem(int max_res, int max_ag_res, int max_cells, int learned) {
-    const int G = max_ag_res <= AG_STAGE_MAX ? max_ag_res : 0;
-    return anneal_smem_bytes(max_res, G, G && max_cells <= CELL_STAGE_MAX ? max_cells : 0, learned);
-}
-
 cudaError_t launch_anneal(cudaStream_t s, const StateView& st, const AgView* ags, const StepParams& p, int n_steps,
                           uint32_t step0, int with_noise, const float* temps, int accumulate, int max_res,
                           int max_ag_res, int max_cells, uint32_t* err, long long* stats, const AnnealExtras& x,
                           int fv_chain, const uint8_t* fv_cdr) {
     if (st.n_cand <= 0 || n_steps <= 0 || max_res <= 0) return cudaSuccess;
-    const int G = max_ag_res <= AG_STAGE_MAX ? max_ag_res : 0;
-    const int C = G && max_cells <= CELL_STAGE_MAX ? max_cells : 0;
-    const bool fv = fv_chain >= 0;
-    const int learned = x.learned && !fv ? 1 : 0;
-    const size_t smem = anneal_smem_bytes(max_res, G, C, learned, fv ? 1 : 0);
+    if (max_res > ANNEAL_MAX_RES) return cudaErrorInvalidValue;
+    const bool fv = fv_chain >= 0, f32 = accumulate == 1;
+    const bool learned = x.learned && !fv;
     const bool ext = !fv && (x.learned || x.log);
     const int grid = fv ? st.n_cand / 2 : st.n_cand;
     if (grid <= 0) return cudaSuccess;
-    // a grid that leaves SMs idle (the 64 survivors of phase 2) takes 16 warps per
-    // candidate: the per-residue passes (Calpha energies, builds, backbone moves) need
-    // fewer rounds; the network path keeps 8
-    int sms = 148;
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
-    const bool wide = !ext && grid <= sms;
-    const size_t smem16 = anneal_smem_bytes(max_res, G, C, learned, fv ? 1 : 0, 2 * AN_WARPS);
-    auto run = [&](auto kern, int warps) -> cudaError_t {
-        const size_t sm = warps == AN_WARPS ? smem : smem16;
+    int dev = 0, sms = 148, smem_max = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    // 16 warps per candidate while every candidate has an SM of its own (64 candidates: 600
+    // steps in 9.5 ms, with 8 warps 11.1), else 8 and several candidates per SM (1024
+    // candidates, 60 steps: 4.2 ms, with 16 warps 6.7; three CTAs of 80 registers per SM
+    // for up to 32 residues 4.2, two of 128 registers 4.35): a step is a chain of latencies
+    // that more warps shorten only a little.  The network path takes 8 warps.
+    const int warps = ext || grid > sms ? 8 : 16;
+    auto run = [&](auto kern, size_t fixed) -> cudaError_t {
+        // the antigen and its cells are staged when they fit
+        int G = max_ag_res <= AG_STAGE_MAX ? max_ag_res : 0;
+        if (fixed + an_tail_bytes(G, 0, f32) > (size_t)smem_max) G = 0;
+        int C = G && max_cells <= CELL_STAGE_MAX ? max_cells : 0;
+        if (fixed + an_tail_bytes(G, C, f32) > (size_t)smem_max) C = 0;
+        const size_t sm = fixed + an_tail_bytes(G, C, f32);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e) return e;
-        kern<<<grid, warps * 32, sm, s>>>(st, ags, p, n_steps, step0, with_noise, temps, max_res, G, C, err, stats,
-                                          x.mlp, learned, x.log, x.log_n, x.log_cap, fv ? fv_chain : 0, fv_cdr);
+        kern<<<grid, warps * 32, sm, s>>>(st, ags, p, n_steps, step0, with_noise, temps, G, C, err, stats, x.mlp,
+                                 learned ? 1 : 0, x.log, x.log_n, x.log_cap, fv ? fv_chain : 0, fv_cdr);
         return cudaSuccess;
     };
-    constexpr int W8 = AN_WARPS, W16 = 2 * AN_WARPS;
     cudaError_t e;
-    if (fv) {
-        if (accumulate == 1) e = wide ? run(k_anneal<float, false, true, W16>, W16) : run(k_anneal<float, false, true, W8>, W8);
-        else e = wide ? run(k_anneal<double, false, true, W16>, W16) : run(k_anneal<double, false, true, W8>, W8);
-    } else if (ext) {
-        e = accumulate == 1 ? run(k_anneal<float, true, false, W8>, W8) : run(k_anneal<double, true, false, W8>, W8);
-    } else if (accumulate == 1) {
-        e = wide ? run(k_anneal<float, false, false, W16>, W16) : run(k_anneal<float, false, false, W8>, W8);
-    } else {
-        e = wide ? run(k_anneal<double, false, false, W16>, W16) : run(k_anneal<double, false, false, W8>, W8);
-    }
+#define BINDER_AN1(RT, W, F, LRN, FV, EXT, GL) run(k_anneal<AnSmem<RT, W, F, LRN, FV>, EXT, GL>, sizeof(AnSmem<RT, W, F, LRN, FV>))
+#define BINDER_AN(F)                                                                       \
+    (fv ? (warps == 16 ? BINDER_AN1(128, 16, F, false, true, false, 4)                     \
+                       : BINDER_AN1(128, 8, F, false, true, false, 4))                     \
+     : ext ? (max_res <= 32   ? BINDER_AN1(32, 8, F, true, false, true, 8)                 \
+              : max_res <= 64 ? BINDER_AN1(64, 8, F, true, false, true, 4)                 \
+                              : BINDER_AN1(128, 8, F, true, false, true, 4))               \
+     : warps == 16 ? (max_res <= 32   ? BINDER_AN1(32, 16, F, false, false, false, 16)     \
+                      : max_res <= 64 ? BINDER_AN1(64, 16, F, false, false, false, 8)      \
+                                      : BINDER_AN1(128, 16, F, false, false, false, 4))    \
+                   : (max_res <= 32   ? BINDER_AN1(32, 8, F, false, false, false, 8)       \
+                      : max_res <= 64 ? BINDER_AN1(64, 8, F, false, false, false, 4)       \
+                                      : BINDER_AN1(128, 8, F, false, false, false, 4)))
+    e = f32 ? BINDER_AN(true) : BINDER_AN(false);
+#undef BINDER_AN
+#undef BINDER_AN1
     if (e) return e;
     return cudaGetLastError();
 }
