@@ -271,6 +271,10 @@ struct binder_ctx {
     DBuf<uint8_t> fv_cdr, fv_baa;
     DBuf<double> fv_best, fv_pair_e;
     DBuf<float4> fv_bpos, fv_bchi, fv_btrig;
+    // post-search refinement: trial positions, best energies, counts (kept between calls)
+    DBuf<float4> post_pos;
+    DBuf<double> post_e;
+    DBuf<int> post_i;
     // binder_block_io: the state download runs on a second stream beside the score
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1485,11 +1489,12 @@ int enqueue_score_state(binder_ctx* ctx, int full) {
 
 // Score the resident state and select each segment's stable top-k into ctx->topk:
 // one fused launch for the candidate sums and the selection when it fits (k <= 64,
-// segments of at most 4096 candidates), else the sums and launch_topk_segments.
+// segments of at most 4096 candidates; not the full energy, whose disulfide terms take a
+// warp per candidate), else the sums and launch_topk_segments.
 int enqueue_score_topk(binder_ctx* ctx, int full, int k, cudaEvent_t mid = nullptr, bool defer = false) {
     State& S = ctx->st;
     if (k <= 0 && !mid) return enqueue_score_state(ctx, full);
-    if (k > 0 && full != 2 && S.n_segments > 0 && sum_topk_fits(k, S.max_segment)) {
+    if (k > 0 && full == 0 && S.n_segments > 0 && sum_topk_fits(k, S.max_segment)) {
         CK(ctx->energy.ensure(S.n_cand), "alloc");
         if (!S.order_valid && ctx->cfg.score_order == 0) {
             int s = enqueue_order(ctx);
@@ -1520,7 +1525,7 @@ int flush_select(binder_ctx* ctx) {
     ctx->sel_pending = false;
     if (S.n_cand == 0 || ctx->sel_k <= 0) return BINDER_OK;
     const SumTopk tk{S.ag_cand_idx.p, S.ag_cand_off.p, S.n_segments, ctx->sel_k, ctx->topk.p, nullptr, false};
-    launch_sum_select(ctx->stream, S.view(), S.res_e.p, 0, ctx->energy.p, tk);
+    launch_sum_select(ctx->stream, S.view(), S.res_e.p, ctx->energy.p, tk);
     LAUNCHED("sum_select");
     return BINDER_OK;
 }
@@ -1614,7 +1619,7 @@ int enqueue_block_pipe(binder_ctx* ctx, int n_steps, int k) {
     CK(cudaEventRecord(ctx->ev_fork, ctx->stream), "event");
     CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0), "event");
     const SumTopk tk{S.ag_cand_idx.p, S.ag_cand_off.p, S.n_segments, k, ctx->topk.p, nullptr, false};
-    launch_sum_select(ctx->side, S.view(), S.res_e.p, 0, ctx->energy.p, tk);
+    launch_sum_select(ctx->side, S.view(), S.res_e.p, ctx->energy.p, tk);
     LAUNCHED("sum_select");
     CK(cudaEventRecord(ctx->ev_join, ctx->side), "event");
     if (n_steps > 0 && (s = enqueue_diffuse(ctx, n_steps, 0, 0, 0, nullptr))) return s;
@@ -2137,11 +2142,10 @@ int binder_minimize(binder_ctx* ctx, int steps, double* out_energy) {
     if (steps < 0) return fail(ctx, BINDER_ERR_ARG, "negative step count");
     if ((s = ensure_trig(ctx))) return s;
     if ((s = clear_err(ctx))) return s;
-    DBuf<float4> trial;
-    DBuf<double> best, e_trial;
+    DBuf<float4>& trial = ctx->post_pos;
+    DBuf<double>& best = ctx->post_e;
     CK(trial.ensure((size_t)S.total_res * SLOT_STRIDE), "alloc");
     CK(best.ensure(S.n_cand), "alloc");
-    CK(e_trial.ensure(S.n_cand), "alloc");
     // the energy minimize starts from (partners_energy, diffusion.rs:859)
     if ((s = enqueue_score_state(ctx, 1))) return s;
     CK(cudaMemcpyAsync(best.p, ctx->energy.p, S.n_cand * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream),
@@ -2149,17 +2153,16 @@ int binder_minimize(binder_ctx* ctx, int steps, double* out_energy) {
     StateView tv = S.view();
     tv.res_pos = trial.p;
     const StateScoreScratch scr{nullptr, S.queue.p, S.res_e.p, S.res_abs.p};
-    const ScoreOut o{e_trial.p, nullptr, nullptr, nullptr, ctx->errf.p};
     for (int step = 0; step < steps; ++step) {
         // step size decaying linearly to zero (diffusion.rs:880-881), f32 as the reference
         const float frac = 1.0f - (float)step / (float)steps;
         const float step_size = 0.04f * frac;
         launch_min_move(ctx->stream, S.view(), ctx->d_views.p, S.res_pos.p, trial.p, step_size);
         LAUNCHED("min_move");
-        ctx->launches += launch_score_state(ctx->stream, tv, ctx->d_views.p, ctx->params.accumulate, 1, o, scr,
-                                            persistent_ctas(ctx), ctx->cfg.score_warps) - 1;
+        launch_score_full_residues(ctx->stream, tv, ctx->d_views.p, ctx->params.accumulate, ctx->errf.p, scr,
+                                   persistent_ctas(ctx), ctx->cfg.score_warps);
         LAUNCHED("score_state");
-        launch_min_accept(ctx->stream, S.view(), trial.p, e_trial.p, best.p, nullptr);
+        launch_min_accept(ctx->stream, S.view(), trial.p, S.res_e.p, best.p);
         LAUNCHED("min_accept");
     }
     S.order_valid = false;  // residues moved
@@ -2179,8 +2182,8 @@ int binder_affinity_maturation(binder_ctx* ctx, double* out_energy, int32_t* out
         return fail(ctx, BINDER_ERR_ARG, "affinity maturation holds at most %d residues per candidate", ANNEAL_MAX_RES);
     if ((s = ensure_trig(ctx))) return s;
     if ((s = clear_err(ctx))) return s;
-    DBuf<double> best;
-    DBuf<int> kept;
+    DBuf<double>& best = ctx->post_e;
+    DBuf<int>& kept = ctx->post_i;
     CK(best.ensure(S.n_cand), "alloc");
     CK(kept.ensure(S.n_cand), "alloc");
     // per-residue full energies of the state (the scan changes one residue at a time)
@@ -2203,7 +2206,7 @@ int binder_validate(binder_ctx* ctx, int32_t* out_clashes, int32_t* out_rama) {
     State& S = ctx->st;
     if (S.n_cand == 0) return fail(ctx, BINDER_ERR_STATE, "no candidates uploaded");
     if ((s = clear_err(ctx))) return s;
-    DBuf<int> counts;
+    DBuf<int>& counts = ctx->post_i;
     CK(counts.ensure(2 * (size_t)S.n_cand), "alloc");
     if (S.max_res > 640) return fail(ctx, BINDER_ERR_ARG, "validation holds at most 640 residues per candidate");
     CK(launch_validate(ctx->stream, S.view(), counts.p, counts.p + S.n_cand), "validate");
@@ -2275,7 +2278,7 @@ int binder_fv_run(binder_ctx* ctx, int iterations, double* out_energy) {
     if ((s = upload(ctx, ctx->temps, t.data(), t.size(), "temps"))) return s;
     CK(ctx->energy.ensure(S.n_cand), "alloc");
     CK(ctx->fv_best.ensure(np), "alloc");
-    CK(ctx->fv_pair_e.ensure(np), "alloc");
+    CK(ctx->fv_pair_e.ensure((size_t)np * FV_PAIR_PARTS), "alloc");
     CK(ctx->fv_bpos.ensure((size_t)S.total_res * SLOT_STRIDE), "alloc");
     CK(ctx->fv_baa.ensure(S.total_res), "alloc");
     CK(ctx->fv_bchi.ensure(S.total_res), "alloc");

@@ -169,6 +169,61 @@ __device__ __noinline__ int build_cg_list_warp(const GridView& g, const float4* 
     return n;
 }
 
+// compute_forces_with_grid (energy.rs:322-398) for one body by a warp (every lane gets
+// the force): lanes 0..8 look up the atom ranges of the 9 (dx, dy) columns of the 27
+// probe cells (for fixed (dx, dy) the cells along z are one range of the sorted array, so
+// the ranges in column order are the reference's probe order), the warp tests 32
+// consecutive atoms of their concatenation per round, each lane evaluates its in-cutoff
+// pair and the terms are added in order.
+__device__ __forceinline__ F3 warp_cg_force(const AgView& A, const CgB& body, int lane) {
+    const GridView& g = A.ca_grid;
+    const int cx = cell_coord(body.x, g.inv), cy = cell_coord(body.y, g.inv), cz = cell_coord(body.z, g.inv);
+    float sx = 0.0f, sy = 0.0f, sz = 0.0f;
+    if (cell_far(cx, cy, cz)) {  // i32 wrap of the probe: the one-lane walk
+        if (lane == 0) cg_force(A, body, sx, sy, sz);
+        __syncwarp();
+        return {__shfl_sync(0xffffffffu, sx, 0), __shfl_sync(0xffffffffu, sy, 0), __shfl_sync(0xffffffffu, sz, 0)};
+    }
+    int a0 = 0, len = 0;
+    if (lane < 9) {
+        const int X = cx + lane / 3 - 1 - g.ox, Y = cy + lane % 3 - 1 - g.oy;
+        const int Z0 = max(cz - 1 - g.oz, 0), Z1 = min(cz + 1 - g.oz, g.nz - 1);
+        if (X >= 0 && Y >= 0 && X < g.nx && Y < g.ny && Z0 <= Z1) {
+            const int base = (X * g.ny + Y) * g.nz;
+            a0 = g.cell_start[base + Z0];
+            len = g.cell_start[base + Z1 + 1] - a0;
+        }
+    }
+    int incl = len;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    const int tot = __shfl_sync(0xffffffffu, incl, 8);
+#pragma unroll 1
+    for (int f0 = 0; f0 < tot; f0 += 32) {
+        const int f = f0 + lane, fq = min(f, tot - 1);
+        int lo = 0;  // the first column whose inclusive prefix exceeds fq
+#pragma unroll
+        for (int step = 8; step > 0; step >>= 1) {
+            const int v = __shfl_sync(0xffffffffu, incl, lo + step - 1);
+            if (lo + step <= 9 && v <= fq) lo += step;
+        }
+        const int v_lo = __shfl_sync(0xffffffffu, incl, lo), len_lo = __shfl_sync(0xffffffffu, len, lo);
+        const int i = __shfl_sync(0xffffffffu, a0, lo) + (fq - (v_lo - len_lo));
+        float tx = 0.0f, ty = 0.0f, tz = 0.0f;
+        const bool in = f < tot && cg_term_parts(body, A.ca_pq[i], A.ca_prm[i], tx, ty, tz);
+        for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) {
+            const int b = __ffs(m) - 1;
+            sx = xadd(sx, __shfl_sync(0xffffffffu, tx, b));
+            sy = xadd(sy, __shfl_sync(0xffffffffu, ty, b));
+            sz = xadd(sz, __shfl_sync(0xffffffffu, tz, b));
+        }
+    }
+    return {sx, sy, sz};
+}
+
 constexpr int CG_IN_MAX = 48;      // in-cutoff list entries a residue holds per step
 constexpr float CG_NEAR_SQ = 99.0f;  // r^2 below which a pair is in adjacent 10 A cells
 

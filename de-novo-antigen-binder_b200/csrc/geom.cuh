@@ -15,6 +15,7 @@
 #pragma once
 
 #include <cmath>
+#include <cstring>
 
 #include "common.cuh"
 
@@ -25,6 +26,8 @@ static __constant__ int s_sc_n[N_AA];
 static __constant__ uchar4 s_sc_ref[N_AA][9];     // ref a, b, c, chi index (255 = fixed)
 static __constant__ float4 s_sc_geom[N_AA][9];    // bond, sin(angle), cos(angle), unused
 static __constant__ float2 s_sc_fix[N_AA][9];     // sin, cos of the fixed dihedral
+static __device__ float4 g_sc_prog[N_AA * 9];     // the programs as stage_side_chains lays them out
+static __device__ float2 g_sc_fix[N_AA * 9];
 static __constant__ int s_rot_n[N_AA];
 static __constant__ float4 s_rot_chi[N_AA][5];    // chi1..chi4 in degrees
 static __constant__ float2 s_rot_trig[N_AA][5][4];// sin, cos of each rotamer chi
@@ -68,7 +71,18 @@ static cudaError_t geom_init_tables() {
         ca_type[a] = t;
     }
     for (int t = 0; t < 16; ++t) hb[t] = BT_HB[t];
+    float4 prog[N_AA * 9];
+    for (int a = 0; a < N_AA; ++a)
+        for (int k = 0; k < 9; ++k) {
+            const uchar4 q = ref[a][k];
+            const uint32_t bits = q.x | (uint32_t)q.y << 8 | (uint32_t)q.z << 16 | (uint32_t)q.w << 24;
+            float w;
+            std::memcpy(&w, &bits, 4);
+            prog[a * 9 + k] = make_float4(geom[a][k].x, geom[a][k].y, geom[a][k].z, w);
+        }
     cudaError_t e;
+    if ((e = cudaMemcpyToSymbol(g_sc_prog, prog, sizeof(prog))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(g_sc_fix, fix, sizeof(fix))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(s_topo_n, BT_TOPO_N, sizeof(BT_TOPO_N))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(s_sc_n, BT_SC_N, sizeof(BT_SC_N))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(s_sc_ref, ref, sizeof(ref))) != cudaSuccess) return e;
@@ -144,6 +158,65 @@ __device__ __forceinline__ void build_side_chain(int aa, F3* atoms, int n_bb, co
         else d = chi.t[r.w];
         atoms[n_bb + k] = place_atom(atoms[r.x], atoms[r.y], atoms[r.z], g.x, g.y, g.z, d.x, d.y);
     }
+}
+
+// ---- side chains by four lanes ---------------------------------------------------------
+// A CTA's shared copy of the side-chain programs: bond, sin, cos of the angle and the
+// reference atoms' bits (a, b, c, chi; 255 = fixed dihedral), sin / cos of the fixed ones.
+// Copied from global memory: the constant tables' rows would be fetched one lane at a time.
+constexpr int SC_MAX = 9;  // side-chain atoms of a residue program
+__device__ __forceinline__ void stage_side_chains(float4* sct, float2* scf, int tid, int threads) {
+#pragma unroll 1
+    for (int i = tid; i < N_AA * SC_MAX; i += threads) {
+        sct[i] = g_sc_prog[i];
+        scf[i] = g_sc_fix[i];
+    }
+}
+__device__ __forceinline__ float quad_norm(float v) {  // component of norm3 (allatom.rs:486-489)
+    const float q = xmul(v, v);
+    const float d = xadd(xadd(__shfl_sync(0xffffffffu, q, 0, 4), __shfl_sync(0xffffffffu, q, 1, 4)),
+                         __shfl_sync(0xffffffffu, q, 2, 4));
+    return xdiv(v, fmaxf(xsqrt(d), 1e-8f));
+}
+// build_side_chain (rotamer.rs:439-462) of n atoms by four lanes of a warp: all 32 lanes
+// call, each four with their own residue (n = 0: none).  Lanes 0..2 compute x, y, z of
+// each atom -- place_atom operation for operation, a vector's squares and cross products
+// exchanged by shuffles -- because the chain of dependent atoms is what a build costs: one
+// division instead of three per normalisation is on it.  prog, fix: the residue's rows of
+// the staged programs; trig: sin / cos of chi1..4; atoms below n_bb are read from bb, the
+// others placed in and read from out (shared memory).
+__device__ __forceinline__ void quad_side_chain(const float4* prog, const float2* fix, const float2* trig,
+                                                const float4* bb, float4* out, int n_bb, int n) {
+    const int q = threadIdx.x & 3;
+    const int c = q == 3 ? 0 : q, u = c == 2 ? 0 : c + 1, v = c == 0 ? 2 : c - 1;  // own, next, next but one component
+    const int n_max = __reduce_max_sync(0xffffffffu, n);
+    float4 g = prog[0];
+    float2 fx = fix[0];
+#pragma unroll 1
+    for (int k = 0; k < n_max; ++k) {
+        __syncwarp();                                // the atoms placed so far
+        const unsigned ref = __float_as_uint(g.w);
+        const int ia = ref & 255u, ib = ref >> 8 & 255u, ic = ref >> 16 & 255u, chi = ref >> 24;
+        const float2 d = chi == 255 ? fx : trig[chi];
+        const float* pa = (const float*)((ia < n_bb ? bb : out) + ia);
+        const float* pb = (const float*)((ib < n_bb ? bb : out) + ib);
+        const float* pc = (const float*)((ic < n_bb ? bb : out) + ic);
+        const float bu = pb[u], bv = pb[v], cc = pc[c];
+        const float bc = quad_norm(xsub(pb[c], cc));
+        const float ba_u = xsub(bu, pa[u]), ba_v = xsub(bv, pa[v]);
+        const float bond = g.x, sa = g.y, nca = -g.z;
+        if (k + 1 < n) {
+            g = prog[k + 1];
+            fx = fix[k + 1];
+        }
+        const float bc_u = __shfl_sync(0xffffffffu, bc, u, 4), bc_v = __shfl_sync(0xffffffffu, bc, v, 4);
+        const float nn = quad_norm(xsub(xmul(ba_u, bc_v), xmul(ba_v, bc_u)));
+        const float n_u = __shfl_sync(0xffffffffu, nn, u, 4), n_v = __shfl_sync(0xffffffffu, nn, v, 4);
+        const float m = xsub(xmul(bc_u, n_v), xmul(bc_v, n_u));
+        const float p = xadd(cc, xmul(bond, xadd(xadd(xmul(nca, bc), xmul(xmul(sa, d.y), m)), xmul(xmul(sa, d.x), nn))));
+        if (k < n) ((float*)(out + n_bb + k))[q] = q == 3 ? 0.0f : p;
+    }
+    __syncwarp();
 }
 
 // build_ideal_backbone_around_ca (allatom.rs:502-517); returns the backbone length

@@ -69,7 +69,6 @@ constexpr int HIT_CAP = 96;                          // in-cutoff entries a warp
 constexpr int EL = 8;                                // lanes per Calpha energy (ACC = double)
 constexpr int MASK_WORDS = ANNEAL_MAX_RES / 32;      // residue bit masks of a candidate
 constexpr int AN_IN = 32;                            // in-cutoff entries of the force a residue holds per round
-constexpr int SC_MAX = 9;                            // side-chain atoms of a residue program
 constexpr int AG_STAGE_MAX = 1024;                   // antigen Calphas staged in shared memory
 constexpr int CELL_STAGE_MAX = 4096;                 // Calpha-grid cells staged in shared memory
 enum : int { MV_NONE = 0, MV_ROT = 1, MV_MUT = 2 };
@@ -507,23 +506,13 @@ __device__ int warp_sample(const float* y, int n, double inv_tp, uint32_t dz) {
 // the old amino acid around the same Calpha; allatom.rs:244-384), by four lanes of a
 // warp (all lanes call; live: the four lanes have a build).  The two kinds differ only
 // in the backbone the side chain is built on (the current one, or the ideal one around
-// the Calpha), so the builds of a warp share the side-chain loop.  Lanes 0..2 of four
-// compute x, y, z of each atom -- place_atom (rotamer.rs:198-232) operation for
-// operation, a vector's squares and cross products exchanged by shuffles -- because the
-// chain of dependent atoms is what a build costs: one division instead of three per
-// normalisation is on it.  Atoms go straight into the row of prop / rej, the program
-// comes from the CTA's shared tables one atom ahead.  A side-chain-only build writes
-// the side chain's slots only (SEL_SIDE: the others stay as they are).
-__device__ __forceinline__ float quad_norm(float v) {  // component of norm3 (allatom.rs:486-489)
-    const float q = xmul(v, v);
-    const float d = xadd(xadd(__shfl_sync(0xffffffffu, q, 0, 4), __shfl_sync(0xffffffffu, q, 1, 4)),
-                         __shfl_sync(0xffffffffu, q, 2, 4));
-    return xdiv(v, fmaxf(xsqrt(d), 1e-8f));
-}
+// the Calpha), so the builds of a warp share the side-chain loop (quad_side_chain).
+// Atoms go straight into the row of prop / rej, the programs are the CTA's shared copy.
+// A side-chain-only build writes the side chain's slots only (SEL_SIDE: the others stay
+// as they are).
 template <class L>
 __device__ __forceinline__ void build_move(L& S, int r, int which, bool live) {
     const int q = threadIdx.x & 3;
-    const int c = q == 3 ? 0 : q, u = c == 2 ? 0 : c + 1, v = c == 0 ? 2 : c - 1;  // own, next, next but one component
     const int oa = S.aa[r];
     const int kind = S.kind[r];
     const int na = S.new_aa[r];
@@ -548,35 +537,7 @@ __device__ __forceinline__ void build_move(L& S, int r, int which, bool live) {
         for (int k = n_at + q; k < SLOT_STRIDE; k += 4) out[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         bb = out;
     }
-    const int n = live ? S.sc_n[a] : 0;
-    const int n_max = __reduce_max_sync(0xffffffffu, n);
-    const float4* prog = S.sct + a * SC_MAX;
-    const float2* fix = S.scf + a * SC_MAX;
-    float4 g = prog[0];
-    float2 fx = fix[0];
-    for (int k = 0; k < n_max; ++k) {
-        __syncwarp();                                // the atoms placed so far
-        const unsigned ref = __float_as_uint(g.w);  // reference atoms a, b, c and the chi (255: fixed)
-        const int ia = ref & 255u, ib = ref >> 8 & 255u, ic = ref >> 16 & 255u, chi = ref >> 24;
-        const float2 d = chi == 255 ? fx : trig[chi];
-        const float* pa = (const float*)((ia < n_bb ? bb : out) + ia);
-        const float* pb = (const float*)((ib < n_bb ? bb : out) + ib);
-        const float* pc = (const float*)((ic < n_bb ? bb : out) + ic);
-        const float bu = pb[u], bv = pb[v], cc = pc[c];
-        const float bc = quad_norm(xsub(pb[c], cc));
-        const float ba_u = xsub(bu, pa[u]), ba_v = xsub(bv, pa[v]);
-        const float bond = g.x, sa = g.y, nca = -g.z;
-        if (k + 1 < n) {
-            g = prog[k + 1];
-            fx = fix[k + 1];
-        }
-        const float bc_u = __shfl_sync(0xffffffffu, bc, u, 4), bc_v = __shfl_sync(0xffffffffu, bc, v, 4);
-        const float nn = quad_norm(xsub(xmul(ba_u, bc_v), xmul(ba_v, bc_u)));
-        const float n_u = __shfl_sync(0xffffffffu, nn, u, 4), n_v = __shfl_sync(0xffffffffu, nn, v, 4);
-        const float m = xsub(xmul(bc_u, n_v), xmul(bc_v, n_u));
-        const float p = xadd(cc, xmul(bond, xadd(xadd(xmul(nca, bc), xmul(xmul(sa, d.y), m)), xmul(xmul(sa, d.x), nn))));
-        if (k < n) ((float*)(out + n_bb + k))[q] = q == 3 ? 0.0f : p;
-    }
+    quad_side_chain(S.sct + a * SC_MAX, S.scf + a * SC_MAX, trig, bb, out, n_bb, live ? S.sc_n[a] : 0);
 }
 
 // rodrigues (allatom.rs:467-479)
@@ -894,13 +855,7 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
     if (F32 && tid == 0 && staged && (nag & 1)) s_agx[nag] = s_agy[nag] = s_agz[nag] = 1e30f;
 #pragma unroll 2
     for (int i = tid; cells_staged && i < ncell; i += NT) s_cell[i] = A.ca_grid.cell_start[i];
-#pragma unroll 1
-    for (int i = tid; i < N_AA * SC_MAX; i += NT) {  // side-chain programs and rotamer trigonometry
-        const uchar4 q = (&s_sc_ref[0][0])[i];
-        const float4 g = (&s_sc_geom[0][0])[i];
-        S.sct[i] = make_float4(g.x, g.y, g.z, __uint_as_float(q.x | q.y << 8 | q.z << 16 | (unsigned)q.w << 24));
-        S.scf[i] = (&s_sc_fix[0][0])[i];
-    }
+    stage_side_chains(S.sct, S.scf, tid, NT);
 #pragma unroll 1
     for (int i = tid; i < N_AA * 20 + 4; i += NT)
         S.rott[i] = i < N_AA * 20 ? (&s_rot_trig[0][0][0])[i] : make_float2(0.f, 1.f);

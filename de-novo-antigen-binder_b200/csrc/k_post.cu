@@ -9,7 +9,7 @@
 //    only when the all-atom energy (allatom_energy: interaction_energy_atoms +
 //    disulfide_energy, diffusion.rs:281-283, 835-840) drops.  Three launches per
 //    step: the move of every residue into a trial copy of the positions, the full
-//    score of the trial copy, the per-candidate keep-or-restore.
+//    score of the trial copy's residues, the per-candidate sum with keep-or-restore.
 //  * affinity_maturation_allatom (diffusion.rs:924-961) over the interface
 //    residues (filters.rs:96-105, main.rs:342-344): one CTA per candidate walks its
 //    mutable positions in order; at a position the 19 other amino acids (ALL_AA
@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "cg_list.cuh"
 #include "geom.cuh"
 #include "score.cuh"
 
@@ -37,55 +38,74 @@ cudaError_t post_init_tables() {
 }
 
 // ---- minimize -----------------------------------------------------------------------
-// One thread per residue: the grid force on the pre-step Calpha (pos_in), the
-// clamped move, the translated residue and its rebuilt side chain (pos_out).
-__global__ void k_min_move(StateView st, const AgView* __restrict__ ags, const float4* __restrict__ pos_in,
-                           float4* __restrict__ pos_out, float step_size) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= st.total_res) return;
-    const int aa = st.res_aa[r];
-    const AgView& A = ags[st.cand_ag[st.res_cand[r]]];
-    const float4* in = pos_in + (size_t)r * SLOT_STRIDE;
-    const int n_at = s_topo_n[aa];
-    const float4 c4 = in[1];  // Calpha = topology atom 1
-    const F3 ca = {c4.x, c4.y, c4.z};
-    float fx, fy, fz;
-    cg_force(A, cg_body(ca.x, ca.y, ca.z, aa), fx, fy, fz);
-    // fx_buf (zeroed) += the one partner's force, then the clamped step (f32 clamp)
-    constexpr float MAXD = 0.5f;
-    auto clampf = [](float v) { return v < -MAXD ? -MAXD : (v > MAXD ? MAXD : v); };
-    const float dx = clampf(xmul(step_size, xadd(0.0f, fx)));
-    const float dy = clampf(xmul(step_size, xadd(0.0f, fy)));
-    const float dz = clampf(xmul(step_size, xadd(0.0f, fz)));
-    const F3 new_ca = {xadd(ca.x, dx), xadd(ca.y, dy), xadd(ca.z, dz)};
-    const F3 dl = sub3(new_ca, ca);  // set_ca_pos: every atom += new - old
-    F3 atoms[SLOTS];
-#pragma unroll
-    for (int k = 0; k < SLOTS; ++k) {
-        const float4 v = in[k];
-        atoms[k] = k < n_at ? F3{xadd(v.x, dl.x), xadd(v.y, dl.y), xadd(v.z, dl.z)} : F3{v.x, v.y, v.z};
+// One warp per residue: the grid force on the pre-step Calpha (pos_in) and the clamped
+// move; then the CTA's first warp rebuilds the side chains of its eight residues, four
+// lanes each (pos_out).  Latency-bound (one residue's chain of dependent pair terms and
+// atoms): 64 candidates x 20 residues took 69 us a launch with one thread per residue, 15 us now.
+constexpr int MIN_WARPS = 8;
+__global__ void __launch_bounds__(MIN_WARPS * 32) k_min_move(StateView st, const AgView* __restrict__ ags,
+                                                             const float4* __restrict__ pos_in,
+                                                             float4* __restrict__ pos_out, float step_size) {
+    __shared__ float4 s_row[MIN_WARPS][SLOT_STRIDE];
+    __shared__ float4 s_prog[N_AA * SC_MAX];
+    __shared__ float2 s_fix[N_AA * SC_MAX];
+    __shared__ float2 s_trig[MIN_WARPS][4];
+    __shared__ int s_aa[MIN_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = blockIdx.x * MIN_WARPS + warp;
+    const bool valid = r < st.total_res;
+    stage_side_chains(s_prog, s_fix, tid, MIN_WARPS * 32);
+    if (valid) {
+        const int aa = st.res_aa[r];
+        const AgView& A = ags[st.cand_ag[st.res_cand[r]]];
+        const float4* in = pos_in + (size_t)r * SLOT_STRIDE;
+        float4 v = lane < SLOT_STRIDE ? in[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        // Calpha = topology atom 1
+        const F3 ca = {__shfl_sync(0xffffffffu, v.x, 1), __shfl_sync(0xffffffffu, v.y, 1),
+                       __shfl_sync(0xffffffffu, v.z, 1)};
+        const F3 f = warp_cg_force(A, cg_body(ca.x, ca.y, ca.z, aa), lane);
+        // fx_buf (zeroed) += the one partner's force, then the clamped step (f32 clamp)
+        constexpr float MAXD = 0.5f;
+        auto clampf = [](float x) { return x < -MAXD ? -MAXD : (x > MAXD ? MAXD : x); };
+        const float dx = clampf(xmul(step_size, xadd(0.0f, f.x)));
+        const float dy = clampf(xmul(step_size, xadd(0.0f, f.y)));
+        const float dz = clampf(xmul(step_size, xadd(0.0f, f.z)));
+        const F3 new_ca = {xadd(ca.x, dx), xadd(ca.y, dy), xadd(ca.z, dz)};
+        const F3 dl = sub3(new_ca, ca);  // set_ca_pos: every atom += new - old
+        if (lane < SLOT_STRIDE) {
+            if (lane < s_topo_n[aa]) v = make_float4(xadd(v.x, dl.x), xadd(v.y, dl.y), xadd(v.z, dl.z), 0.f);
+            s_row[warp][lane] = v;
+        }
+        if (lane < 4) s_trig[warp][lane] = ((const float2*)(st.res_trig + 2 * (size_t)r))[lane];
+        if (lane == 0) s_aa[warp] = aa;
+    } else if (lane == 0) {
+        s_aa[warp] = 0;
     }
-    // rebuild_side_chain: the side chain from the moved backbone at the residue's chi
-    const int n_bb = aa == GLY ? 4 : 5;
-    const ChiTrig ct = unpack_trig(st.res_trig[2 * r], st.res_trig[2 * r + 1]);
-    build_side_chain(aa, atoms, n_bb, ct);
-    float4* out = pos_out + (size_t)r * SLOT_STRIDE;
-#pragma unroll
-    for (int k = 0; k < SLOT_STRIDE; ++k)
-        out[k] = k < n_at ? make_float4(atoms[k].x, atoms[k].y, atoms[k].z, 0.f) : in[k];
+    __syncthreads();
+    if (warp == 0) {  // rebuild_side_chain: the side chain from the moved backbone at the residue's chi
+        const int w = lane >> 2, aa = s_aa[w];
+        const bool live = blockIdx.x * MIN_WARPS + w < st.total_res;
+        quad_side_chain(s_prog + aa * SC_MAX, s_fix + aa * SC_MAX, s_trig[w], s_row[w], s_row[w], aa == GLY ? 4 : 5,
+                        live ? s_sc_n[aa] : 0);
+    }
+    __syncthreads();
+    if (valid && lane < SLOT_STRIDE) pos_out[(size_t)r * SLOT_STRIDE + lane] = s_row[warp][lane];
 }
 
-// Keep the trial positions of candidate c when its energy is strictly lower.
-__global__ void k_min_accept(StateView st, const float4* __restrict__ trial, const double* __restrict__ e_trial,
-                             double* __restrict__ best, int* __restrict__ kept) {
+// The trial's energy of candidate c (its residues' energies and its disulfide term), and
+// the trial positions kept when it is strictly lower.
+__global__ void __launch_bounds__(128) k_min_accept(StateView st, float4* __restrict__ trial,
+                                                    const double* __restrict__ res_e,
+                                                    double* __restrict__ best) {
     const int c = blockIdx.x;
     __shared__ int s_take;
-    if (threadIdx.x == 0) {
-        const double e = e_trial[c];
-        s_take = e < best[c];
-        if (s_take) {
-            best[c] = e;
-            if (kept) kept[c] += 1;
+    if (threadIdx.x < 32) {
+        StateView tv = st;
+        tv.res_pos = trial;
+        const double e = warp_candidate_sum(tv, c, res_e, 1);
+        if (threadIdx.x == 0) {
+            s_take = e < best[c];
+            if (s_take) best[c] = e;
         }
     }
     __syncthreads();
@@ -96,43 +116,24 @@ __global__ void k_min_accept(StateView st, const float4* __restrict__ trial, con
 
 void launch_min_move(cudaStream_t s, const StateView& st, const AgView* ags, const float4* pos_in, float4* pos_out,
                      float step_size) {
-    if (st.total_res > 0) k_min_move<<<(st.total_res + 127) / 128, 128, 0, s>>>(st, ags, pos_in, pos_out, step_size);
+    if (st.total_res > 0)
+        k_min_move<<<(st.total_res + MIN_WARPS - 1) / MIN_WARPS, MIN_WARPS * 32, 0, s>>>(st, ags, pos_in, pos_out,
+                                                                                         step_size);
 }
-void launch_min_accept(cudaStream_t s, const StateView& st, const float4* trial, const double* e_trial, double* best,
-                       int* kept) {
-    if (st.n_cand > 0) k_min_accept<<<st.n_cand, 128, 0, s>>>(st, trial, e_trial, best, kept);
+void launch_min_accept(cudaStream_t s, const StateView& st, float4* trial, const double* res_e, double* best) {
+    if (st.n_cand > 0) k_min_accept<<<st.n_cand, 128, 0, s>>>(st, trial, res_e, best);
 }
 
 // ---- affinity maturation ------------------------------------------------------------
 constexpr int MAT_TRIALS = 20;  // 19 other amino acids + the mutation back
-constexpr int MAT_WARPS = 10;
-
-// disulfide_energy (allatom.rs:155-180) of candidate c with residue `rr` replaced by
-// (aa_r, sg_r): Gaussian well between every pair of Cys SG atoms (topology atom 5),
-// pairs in the reference's order, f32.
-__device__ float disulfide_with(const StateView& st, int c, int rr, int aa_r, float4 sg_r) {
-    const int r0 = st.cand_res_off[c], r1 = st.cand_res_off[c + 1];
-    float ds = 0.0f;
-    for (int ri = r0; ri < r1; ++ri) {
-        const int ai = ri == rr ? aa_r : st.res_aa[ri];
-        if (ai != CYS) continue;
-        const float4 pi = ri == rr ? sg_r : st.res_pos[(size_t)ri * SLOT_STRIDE + 5];
-        for (int rj = ri + 1; rj < r1; ++rj) {
-            const int aj = rj == rr ? aa_r : st.res_aa[rj];
-            if (aj != CYS) continue;
-            const float4 pj = rj == rr ? sg_r : st.res_pos[(size_t)rj * SLOT_STRIDE + 5];
-            const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
-            if (d > 4.0f) continue;
-            const float z = xdiv(xsub(d, 2.05f), 0.4f);
-            ds = xsub(ds, xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z))));
-        }
-    }
-    return ds;
-}
+constexpr int MAT_WARPS = MAT_TRIALS;  // one warp per trial
 
 // One CTA per candidate.  res_e: the per-residue full energies of the state (kept
 // current); out_best: the final score (the reference's `best`); out_kept:
-// mutations kept.
+// mutations kept.  Positions are sequential, so a position's latency counts: its 20
+// trials are built by four lanes each and scored by one warp each at once (64 candidates
+// x 20 residues 1.18 ms with ten warps, one-thread builds and per-thread disulfide
+// scans, 0.58 ms now).
 __global__ void __launch_bounds__(MAT_WARPS * 32) k_mature(StateView st, const AgView* __restrict__ ags,
                                                             double* __restrict__ res_e, double* __restrict__ out_best,
                                                             int* __restrict__ out_kept, uint32_t* __restrict__ err) {
@@ -142,7 +143,10 @@ __global__ void __launch_bounds__(MAT_WARPS * 32) k_mature(StateView st, const A
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     __shared__ GroupSmem gs[MAT_WARPS];
-    __shared__ float4 s_pos[MAT_TRIALS][SLOTS];
+    __shared__ GroupFull gfs[MAT_WARPS];
+    __shared__ float4 s_pos[MAT_TRIALS][SLOT_STRIDE];
+    __shared__ float4 s_prog[N_AA * SC_MAX];
+    __shared__ float2 s_fix[N_AA * SC_MAX];
     __shared__ int s_aa[MAT_TRIALS];
     __shared__ float4 s_chi[MAT_TRIALS], s_trig[MAT_TRIALS][2];
     __shared__ double s_e[MAT_TRIALS];
@@ -154,71 +158,73 @@ __global__ void __launch_bounds__(MAT_WARPS * 32) k_mature(StateView st, const A
         if (threadIdx.x == 0) atomicOr(err, ERRF_RANGE);
         return;
     }
+    stage_side_chains(s_prog, s_fix, threadIdx.x, MAT_WARPS * 32);
     // mutable = interface residues (filters.rs:96-105): an antigen Calpha closer than 8 A
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = warp; i < n; i += MAT_WARPS) {
         const float4 p = st.res_pos[(size_t)(r0 + i) * SLOT_STRIDE + 1];
         bool any = false;
-        for (int j = 0; j < A.n_res && !any; ++j) {
+        for (int j = lane; j < A.n_res; j += 32) {
             const float4 q = A.ca_atom[j];
-            any = xdist2(xsub(p.x, q.x), xsub(p.y, q.y), xsub(p.z, q.z)) < 64.0f;
+            any |= xdist2(xsub(p.x, q.x), xsub(p.y, q.y), xsub(p.z, q.z)) < 64.0f;
         }
-        s_mut[i] = any;
+        any = __any_sync(0xffffffffu, any);
+        if (lane == 0) s_mut[i] = any;
     }
-    if (threadIdx.x == 0) {
-        double e = 0.0;
-        for (int r = r0; r < r1; ++r) e += res_e[r];
-        s_best = e + (double)disulfide_with(st, c, -1, 0, make_float4(0.f, 0.f, 0.f, 0.f));
-        s_kept = 0;
+    if (warp == 0) {
+        const double e = warp_candidate_sum(st, c, res_e, 1);
+        if (lane == 0) {
+            s_best = e;
+            s_kept = 0;
+        }
     }
     __syncthreads();
     for (int i = 0; i < n; ++i) {
         if (!s_mut[i]) continue;  // CTA-uniform
         const int r = r0 + i;
         const int old_aa = st.res_aa[r];
-        // build the trials: t < 19 the t-th other amino acid at its top rotamer, 19 the old one at its chi
-        if (threadIdx.x < MAT_TRIALS) {
-            const int t = threadIdx.x;
+        // build the trials, eight per warp: t < 19 the t-th other amino acid at its top rotamer,
+        // 19 the old one at its chi
+        if (warp < (MAT_TRIALS + 7) / 8) {
+            const int t0 = warp * 8 + (lane >> 2), q = lane & 3;
+            const bool live = t0 < MAT_TRIALS;
+            const int t = live ? t0 : 0;
             const float4 c4 = st.res_pos[(size_t)r * SLOT_STRIDE + 1];
-            int aa;
-            ChiTrig ct;
-            float4 chi, tr0, tr1;
-            if (t < MAT_TRIALS - 1) {
-                aa = t < old_aa ? t : t + 1;
-                if (s_rot_n[aa] > 0) {
-                    ct = rot_trig(aa, 0);
-                    chi = s_rot_chi[aa][0];
+            const int aa = t < MAT_TRIALS - 1 ? (t < old_aa ? t : t + 1) : old_aa;
+            if (live && q == 0) {
+                float4 chi, tr0, tr1;
+                if (t < MAT_TRIALS - 1) {
+                    const bool has = s_rot_n[aa] > 0;
+                    const ChiTrig ct = has ? rot_trig(aa, 0) : zero_trig();
+                    chi = has ? s_rot_chi[aa][0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    tr0 = make_float4(ct.t[0].x, ct.t[0].y, ct.t[1].x, ct.t[1].y);
+                    tr1 = make_float4(ct.t[2].x, ct.t[2].y, ct.t[3].x, ct.t[3].y);
                 } else {
-                    ct = zero_trig();
-                    chi = make_float4(0.f, 0.f, 0.f, 0.f);
+                    tr0 = st.res_trig[2 * r];
+                    tr1 = st.res_trig[2 * r + 1];
+                    chi = st.res_chi[r];
                 }
-                tr0 = make_float4(ct.t[0].x, ct.t[0].y, ct.t[1].x, ct.t[1].y);
-                tr1 = make_float4(ct.t[2].x, ct.t[2].y, ct.t[3].x, ct.t[3].y);
-            } else {
-                aa = old_aa;
-                tr0 = st.res_trig[2 * r];
-                tr1 = st.res_trig[2 * r + 1];
-                ct = unpack_trig(tr0, tr1);
-                chi = st.res_chi[r];
+                s_aa[t] = aa;
+                s_chi[t] = chi;
+                s_trig[t][0] = tr0;
+                s_trig[t][1] = tr1;
             }
-            F3 atoms[SLOTS];
-            const int n_bb = ideal_backbone(F3{c4.x, c4.y, c4.z}, aa, atoms);
-            build_side_chain(aa, atoms, n_bb, ct);
+            F3 bb[5];
+            const int n_bb = ideal_backbone(F3{c4.x, c4.y, c4.z}, aa, bb);
             const int n_at = s_topo_n[aa];
-            for (int k = 0; k < SLOTS; ++k)
-                s_pos[t][k] = k < n_at ? make_float4(atoms[k].x, atoms[k].y, atoms[k].z, 0.f)
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
-            s_aa[t] = aa;
-            s_chi[t] = chi;
-            s_trig[t][0] = tr0;
-            s_trig[t][1] = tr1;
-            s_ds[t] = disulfide_with(st, c, r, aa, s_pos[t][5]);
+            if (live) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k)
+                    if ((k & 3) == q && k < n_bb) s_pos[t][k] = make_float4(bb[k].x, bb[k].y, bb[k].z, 0.f);
+                for (int k = n_at + q; k < SLOT_STRIDE; k += 4) s_pos[t][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            __syncwarp();
+            quad_side_chain(s_prog + aa * SC_MAX, s_fix + aa * SC_MAX, (const float2*)s_trig[t], s_pos[t], s_pos[t],
+                            n_bb, live ? s_sc_n[aa] : 0);
         }
         __syncthreads();
-        // residue energy of every trial: one warp per trial
-        GroupSmem& g = gs[warp];
-        for (int t = warp; t < MAT_TRIALS; t += MAT_WARPS) {
-            const int aa = s_aa[t];
-            const int na = c_topo_n[aa];
+        {  // residue energy of every trial and the disulfide term with it, one warp per trial
+            GroupSmem& g = gs[warp];
+            const int t = warp, aa = s_aa[t], na = c_topo_n[aa];
             if (lane < na) {
                 const float4 p = s_pos[t][lane];
                 const float4 m = c_slot_prm[aa][lane];
@@ -232,37 +238,36 @@ __global__ void __launch_bounds__(MAT_WARPS * 32) k_mature(StateView st, const A
             }
             __syncwarp();
             Acc acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
-            score_group<true, true, false, false>(&A, g, na, lane, lt, acc);
+            score_group<true, true, false, false>(&A, g, &gfs[warp], na, lane, lt, acc);
             const double e = warp_sum_d((double)acc.s - (double)acc.c);
-            if (lane == 0) s_e[t] = e;
-            __syncwarp();
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double others = 0.0;
-            for (int q = r0; q < r1; ++q)
-                if (q != r) others += res_e[q];
-            int pick = MAT_TRIALS - 1;
-            for (int t = 0; t < MAT_TRIALS - 1; ++t) {
-                const double tot = (others + s_e[t]) + (double)s_ds[t];
-                if (tot < s_best) {
-                    s_best = tot;
-                    pick = t;
-                    ++s_kept;
-                    break;
-                }
+            const float ds = warp_disulfide(st, r0, r1, r, aa, s_pos[t][5]);
+            if (lane == 0) {
+                s_e[t] = e;
+                s_ds[t] = ds;
             }
-            s_pick = pick;
-            res_e[r] = s_e[pick];
-            st.res_aa[r] = (uint8_t)s_aa[pick];
-            st.res_chi[r] = s_chi[pick];
-            st.res_trig[2 * r] = s_trig[pick][0];
-            st.res_trig[2 * r + 1] = s_trig[pick][1];
         }
         __syncthreads();
-        if (threadIdx.x < SLOT_STRIDE)
-            st.res_pos[(size_t)r * SLOT_STRIDE + threadIdx.x] =
-                threadIdx.x < SLOTS ? s_pos[s_pick][threadIdx.x] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (warp == 0) {  // the first trial below the best
+            const double others = warp_ordered_sum(res_e, r0, r1, r);
+            const double tot = lane < MAT_TRIALS - 1 ? (others + s_e[lane]) + (double)s_ds[lane] : 0.0;
+            const unsigned m = __ballot_sync(0xffffffffu, lane < MAT_TRIALS - 1 && tot < s_best);
+            const int pick = m ? __ffs(m) - 1 : MAT_TRIALS - 1;
+            __syncwarp();
+            if (lane == pick && m) {
+                s_best = tot;
+                ++s_kept;
+            }
+            if (lane == 0) {
+                s_pick = pick;
+                res_e[r] = s_e[pick];
+                st.res_aa[r] = (uint8_t)s_aa[pick];
+                st.res_chi[r] = s_chi[pick];
+                st.res_trig[2 * r] = s_trig[pick][0];
+                st.res_trig[2 * r + 1] = s_trig[pick][1];
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < SLOT_STRIDE) st.res_pos[(size_t)r * SLOT_STRIDE + threadIdx.x] = s_pos[s_pick][threadIdx.x];
         __syncthreads();
     }
     if (threadIdx.x == 0) {
@@ -279,27 +284,48 @@ void launch_mature(cudaStream_t s, const StateView& st, const AgView* ags, doubl
 // ---- Fv two-chain engine (diffusion.rs:477-827) -----------------------------------------
 // The resident state interleaves the heavy (2i) and light (2i + 1) chain of each Fv
 // candidate i.
-constexpr int FVP_THREADS = 256;
+constexpr int FVP_OWNERS = 256;   // compensated sums per pair, taking the residue pairs in turn
+constexpr int FVP_LANES = 16;     // lanes per sum
+constexpr int FVP_WARPS = FVP_OWNERS / FV_PAIR_PARTS * FVP_LANES / 32;
 constexpr int FVP_MAX_RES = 160;  // residues of a chain the pair kernel stages
 
 // interaction_energy_atoms (energy.rs:256-314, solvation.rs:52-84) between the two chains
 // of candidate i (heavy as energy.rs's "antigen", light as its "antibody"), all five
 // terms, FP64 total; residue pairs whose bounding spheres are further apart than the
-// cutoff are skipped (they hold no pair within 10 A).
-__global__ void __launch_bounds__(FVP_THREADS) k_fv_pair(StateView st, double* __restrict__ out) {
-    const int i = blockIdx.x;
+// cutoff are skipped (they hold no pair within 10 A).  FVP_OWNERS compensated sums take
+// the residue pairs in turn; 16 lanes work on each -- they evaluate 16 atom pairs of a
+// close residue pair at a time and add the in-cutoff ones in order -- and FV_PAIR_PARTS
+// CTAs share a pair's sums.  (With one thread per sum and 32 different residue pairs per
+// warp most lanes idled: 160 us for 32 pairs of 115 + 106 residues, 35 us now.)
+__global__ void __launch_bounds__(FVP_WARPS * 32) k_fv_pair(StateView st, double* __restrict__ out) {
+    const int i = blockIdx.x / FV_PAIR_PARTS, part = blockIdx.x % FV_PAIR_PARTS;
     const int h0 = st.cand_res_off[2 * i], nh = st.cand_res_off[2 * i + 1] - h0;
     const int l0 = st.cand_res_off[2 * i + 1], nl = st.cand_res_off[2 * i + 2] - l0;
     __shared__ float4 s_c[2][FVP_MAX_RES];  // residue centroid, radius
-    __shared__ double s_sum[FVP_THREADS / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ unsigned char s_aa[2][FVP_MAX_RES];
+    __shared__ float4 s_prm[N_AA * SLOT_STRIDE];  // c_slot_prm, type, EEF1 parameters
+    __shared__ unsigned char s_type[N_AA * SLOT_STRIDE];
+    __shared__ float4 s_eef[16];
+    __shared__ float s_rl[16];
+    __shared__ int s_hb[16];
+    __shared__ double s_sum[FVP_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (nh > FVP_MAX_RES || nl > FVP_MAX_RES) {
-        if (threadIdx.x == 0) out[i] = nan("");
+        if (tid == 0) out[blockIdx.x] = nan("");
         return;
     }
-    for (int t = threadIdx.x; t < nh + nl; t += blockDim.x) {
+    for (int t = tid; t < N_AA * SLOT_STRIDE; t += blockDim.x) {
+        s_prm[t] = (&c_slot_prm[0][0])[t];
+        s_type[t] = (unsigned char)(&c_slot_type[0][0])[t];
+    }
+    if (tid < 16) {
+        s_eef[tid] = c_eef1[tid];
+        s_rl[tid] = __frcp_rn(c_eef1[tid].z);
+        s_hb[tid] = c_hb[tid];
+    }
+    for (int t = tid; t < nh + nl; t += blockDim.x) {
         const int r = t < nh ? h0 + t : l0 + (t - nh);
-        const int na = c_topo_n[st.res_aa[r]];
+        const int aa = st.res_aa[r], na = c_topo_n[aa];
         const float4* p = st.res_pos + (size_t)r * SLOT_STRIDE;
         float cx = 0.f, cy = 0.f, cz = 0.f;
         for (int k = 0; k < na; ++k) {
@@ -312,44 +338,88 @@ __global__ void __launch_bounds__(FVP_THREADS) k_fv_pair(StateView st, double* _
             rad = fmaxf(rad, sqrtf(dx * dx + dy * dy + dz * dz));
         }
         s_c[t < nh ? 0 : 1][t < nh ? t : t - nh] = make_float4(cx, cy, cz, rad * 1.0001f + 1e-3f);
+        s_aa[t < nh ? 0 : 1][t < nh ? t : t - nh] = (unsigned char)aa;
     }
     __syncthreads();
-    float s = 0.f, comp = 0.f;  // compensated sum of this thread's pair terms
-    for (int t = threadIdx.x; t < nh * nl; t += blockDim.x) {
-        const int a = t / nl, b = t - a * nl;
-        const float4 ca = s_c[0][a], cb = s_c[1][b];
-        const float dx = ca.x - cb.x, dy = ca.y - cb.y, dz = ca.z - cb.z;
-        const float reach = 10.01f + ca.w + cb.w;
-        if (dx * dx + dy * dy + dz * dz > reach * reach) continue;
-        const int aa_a = st.res_aa[h0 + a], aa_b = st.res_aa[l0 + b];
-        const int na = c_topo_n[aa_a], nb = c_topo_n[aa_b];
-        const float4* pa = st.res_pos + (size_t)(h0 + a) * SLOT_STRIDE;
-        const float4* pb = st.res_pos + (size_t)(l0 + b) * SLOT_STRIDE;
-        for (int kb = 0; kb < nb; ++kb) {
-            const float4 m = c_slot_prm[aa_b][kb];
-            const float4 B = make_float4(pb[kb].x, pb[kb].y, pb[kb].z, m.x);
-            const float4 Bp = make_float4(m.y, m.z, m.w, (float)c_slot_type[aa_b][kb]);
-            for (int ka = 0; ka < na; ++ka) {
-                const float4 n = c_slot_prm[aa_a][ka];
-                const float4 A = make_float4(pa[ka].x, pa[ka].y, pa[ka].z, n.x);
-                const float r2 = xdist2(B.x - A.x, B.y - A.y, B.z - A.z);
-                if (r2 > CUTOFF_SQ || r2 < MIN_R_SQ) continue;
-                const float4 Ap = make_float4(n.y, n.z, n.w, (float)c_slot_type[aa_a][ka]);
-                float lj, coul, hyd;
-                const float e = pair_energy<true>(B, Bp, A, Ap, r2, lj, coul, hyd);
-                const float y = e - comp, tt = s + y;
+    float s = 0.f, comp = 0.f;  // the owner's compensated sum (the same on its 16 lanes)
+    const int hl = lane & (FVP_LANES - 1), hs = lane & ~(FVP_LANES - 1);  // lane in the half-warp, its first lane
+    const int owner = part * (FVP_OWNERS / FV_PAIR_PARTS) + tid / FVP_LANES;
+    // the next close residue pair of the owner from t on: 16 candidates tested at a time
+    int t = owner;
+    const int total = nh * nl;
+    int na = 0, nb = 0, p0 = 0;  // atom pairs of the current residue pair, the next ones
+    const float4 *pa = nullptr, *pb = nullptr;
+    int aa_a = 0, aa_b = 0;
+    for (;;) {
+        if (p0 >= na * nb) {  // (half-warp uniform)
+            na = nb = p0 = 0;
+            while (t < total) {
+                const int mine = t + hl * FVP_OWNERS;
+                bool close = false;
+                if (mine < total) {
+                    const int a = mine / nl, b = mine - a * nl;
+                    const float4 ca = s_c[0][a], cb = s_c[1][b];
+                    const float dx = ca.x - cb.x, dy = ca.y - cb.y, dz = ca.z - cb.z;
+                    const float reach = 10.01f + ca.w + cb.w;
+                    close = !(dx * dx + dy * dy + dz * dz > reach * reach);
+                }
+                const unsigned m = __ballot_sync(0xffffu << hs, close) >> hs;
+                if (!m) {
+                    t += FVP_LANES * FVP_OWNERS;
+                    continue;
+                }
+                t += (__ffs(m) - 1) * FVP_OWNERS;
+                const int a = t / nl, b = t - a * nl;
+                t += FVP_OWNERS;
+                aa_a = s_aa[0][a];
+                aa_b = s_aa[1][b];
+                na = c_topo_n[aa_a];
+                nb = c_topo_n[aa_b];
+                pa = st.res_pos + (size_t)(h0 + a) * SLOT_STRIDE;
+                pb = st.res_pos + (size_t)(l0 + b) * SLOT_STRIDE;
+                break;
+            }
+        }
+        __syncwarp();
+        if (__all_sync(0xffffffffu, na == 0)) break;
+        const int p = p0 + hl;
+        bool in = false;
+        float e = 0.0f;
+        if (p < na * nb) {
+            const int kb = p / na, ka = p - kb * na;
+            const float4 xa = pa[ka], xb = pb[kb];
+            const float r2 = xdist2(xb.x - xa.x, xb.y - xa.y, xb.z - xa.z);
+            in = !(r2 > CUTOFF_SQ || r2 < MIN_R_SQ);
+            if (in) {
+                const float4 mb = s_prm[aa_b * SLOT_STRIDE + kb], ma = s_prm[aa_a * SLOT_STRIDE + ka];
+                const int tb = s_type[aa_b * SLOT_STRIDE + kb], ta = s_type[aa_a * SLOT_STRIDE + ka];
+                const float4 B = make_float4(xb.x, xb.y, xb.z, mb.x), Bp = make_float4(mb.y, mb.z, mb.w, 0.f);
+                const float4 A = make_float4(xa.x, xa.y, xa.z, ma.x), Ap = make_float4(ma.y, ma.z, ma.w, 0.f);
+                float ir;
+                e = pair_base(B, Bp, A, Ap, r2, ir);
+                e = full_terms(e, hb_pair(s_hb[tb], s_hb[ta]), s_eef[ta], s_rl[ta], s_eef[tb], s_rl[tb], r2, ir);
+            }
+        }
+        p0 += FVP_LANES;
+        unsigned m = __ballot_sync(0xffffffffu, in) >> hs & 0xffffu;
+        while (__any_sync(0xffffffffu, m != 0)) {
+            const float x = __shfl_sync(0xffffffffu, e, hs + (m ? __ffs(m) - 1 : 0));
+            if (m) {
+                const float y = x - comp, tt = s + y;
                 comp = (tt - s) - y;
                 s = tt;
             }
+            m &= m - 1;
         }
     }
+    if (hl) s = comp = 0.f;
     const double v = warp_sum_d((double)s - (double)comp);
     if (lane == 0) s_sum[warp] = v;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         double e = 0.0;
-        for (int w = 0; w < FVP_THREADS / 32; ++w) e += s_sum[w];
-        out[i] = e;
+        for (int w = 0; w < FVP_WARPS; ++w) e += s_sum[w];
+        out[blockIdx.x] = e;
     }
 }
 
@@ -364,7 +434,9 @@ __global__ void k_fv_keep(StateView st, const double* __restrict__ e_chain, cons
     const int i = blockIdx.x;
     __shared__ int s_dec;
     if (threadIdx.x == 0) {
-        const double e = e_chain[2 * i] + e_chain[2 * i + 1] + e_pair[i];
+        double ep = 0.0;
+        for (int p = 0; p < FV_PAIR_PARTS; ++p) ep += e_pair[i * FV_PAIR_PARTS + p];
+        const double e = e_chain[2 * i] + e_chain[2 * i + 1] + ep;
         int dec = 0;
         if (restore == 1) dec = -1;
         else if (restore == 2 || e < best[i]) dec = 1;
@@ -396,7 +468,7 @@ __global__ void k_fv_keep(StateView st, const double* __restrict__ e_chain, cons
 }
 
 void launch_fv_pair(cudaStream_t s, const StateView& st, double* out) {
-    if (st.n_cand >= 2) k_fv_pair<<<st.n_cand / 2, FVP_THREADS, 0, s>>>(st, out);
+    if (st.n_cand >= 2) k_fv_pair<<<st.n_cand / 2 * FV_PAIR_PARTS, FVP_WARPS * 32, 0, s>>>(st, out);
 }
 void launch_fv_keep(cudaStream_t s, const StateView& st, const double* e_chain, const double* e_pair, double* best,
                     float4* b_pos, uint8_t* b_aa, float4* b_chi, float4* b_trig, int restore) {

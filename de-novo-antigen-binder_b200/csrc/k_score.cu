@@ -151,27 +151,41 @@ struct SrcFlatG {
     }
 };
 
-// Resident state: persistent warps take residues from a work queue (an atomic
-// counter; residues in index order, or in Calpha-cell order so that neighbouring
+// Resident state: persistent teams of TEAM warps take residues from a work queue (an
+// atomic counter; residues in index order, or in Calpha-cell order so that neighbouring
 // warps share antigen atoms in L1 -- whichever the autotuner timed faster) and
 // write one FP64 energy per residue; k_sum_residues adds a candidate's residues in
-// index order.  No CTA barrier: warps never wait for each other.
-template <int NW, bool KAHAN, bool FULL, bool ABS, bool COUNT>
+// index order.  No CTA barrier: teams never wait for each other.
+template <int NW, bool KAHAN, bool FULL, bool ABS, bool COUNT, int TEAM>
 __global__ void __launch_bounds__(NW * 32) k_score_residues(StateView st, const AgView* __restrict__ ags,
                                                              const int* __restrict__ order, int* __restrict__ queue,
                                                              double* __restrict__ res_e, double* __restrict__ res_abs,
                                                              long long* __restrict__ pair_count,
                                                              uint32_t* __restrict__ err) {
+    static_assert(NW % TEAM == 0 && NW / TEAM < 16 + (TEAM == 1), "one named barrier per team");
     __shared__ GroupSmem gs[NW];
+    __shared__ GroupFull gfs[FULL ? NW : 1];
+    extern __shared__ __align__(16) unsigned char team_raw[];  // TEAM > 1: a TeamSmem per team
+    TeamSmem* teams = reinterpret_cast<TeamSmem*>(team_raw);
+    __shared__ int s_task[TEAM > 1 ? NW / TEAM : 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int team = warp / TEAM, rank = warp % TEAM;
     const unsigned lt = (1u << lane) - 1u;
     GroupSmem& s = gs[warp];
     SrcStateG src{st};
+    auto sync = [team] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(TEAM * 32) : "memory"); };
     int my_pairs = 0;
     for (;;) {
         int gi = 0;
-        if (lane == 0) gi = atomicAdd(queue, 1);
-        gi = __shfl_sync(0xffffffffu, gi, 0);
+        if (lane == 0 && rank == 0) gi = atomicAdd(queue, 1);
+        if (TEAM > 1) {
+            if (lane == 0 && rank == 0) s_task[team] = gi;
+            sync();
+            gi = s_task[team];
+            sync();
+        } else {
+            gi = __shfl_sync(0xffffffffu, gi, 0);
+        }
         if (gi >= st.total_res) break;
         const int r = order ? order[gi] : gi;
         const int c = st.res_cand[r];
@@ -182,14 +196,21 @@ __global__ void __launch_bounds__(NW * 32) k_score_residues(StateView st, const 
             if (lane == 0) atomicOr(err, ERRF_NAN);
         } else if (n > 0) {
             __syncwarp();
-            score_group<KAHAN, FULL, ABS, COUNT>(&ags[st.cand_ag[c]], s, n, lane, lt, acc);
+            if constexpr (TEAM > 1)
+                score_group_team<KAHAN, TEAM>(&ags[st.cand_ag[c]], s, &gfs[warp], n, lane, lt, acc, rank, teams[team],
+                                              sync);
+            else
+                score_group<KAHAN, FULL, ABS, COUNT>(&ags[st.cand_ag[c]], s, FULL ? &gfs[warp] : nullptr, n, lane, lt,
+                                                     acc);
         }
         __syncwarp();
-        const double e = warp_sum_d(KAHAN ? ((double)acc.s - (double)acc.c) : (double)acc.s);
-        const double ea = ABS ? warp_sum_d((double)acc.abs_s) : 0.0;
-        if (lane == 0) {
-            if (res_e) res_e[r] = e;
-            if (ABS) res_abs[r] = ea;
+        if (rank == 0) {
+            const double e = warp_sum_d(KAHAN ? ((double)acc.s - (double)acc.c) : (double)acc.s);
+            const double ea = ABS ? warp_sum_d((double)acc.abs_s) : 0.0;
+            if (lane == 0) {
+                if (res_e) res_e[r] = e;
+                if (ABS) res_abs[r] = ea;
+            }
         }
         if (COUNT) my_pairs += acc.pairs;
     }
@@ -208,6 +229,7 @@ __global__ void __launch_bounds__(NW * 32) k_score_grouped(Src src, int n_cand, 
                                                             long long* __restrict__ pair_count,
                                                             uint32_t* __restrict__ err) {
     __shared__ GroupSmem gs[NW];
+    __shared__ GroupFull gfs[FULL ? NW : 1];
     __shared__ double sm[NW];
     __shared__ double sm2[NW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -228,7 +250,7 @@ __global__ void __launch_bounds__(NW * 32) k_score_grouped(Src src, int n_cand, 
             }
             if (n == 0) continue;
             __syncwarp();
-            score_group<KAHAN, FULL, ABS, COUNT>(Ap, s, n, lane, lt, acc);
+            score_group<KAHAN, FULL, ABS, COUNT>(Ap, s, FULL ? &gfs[warp] : nullptr, n, lane, lt, acc);
         }
         const double lane_e = KAHAN ? ((double)acc.s - (double)acc.c) : (double)acc.s;
         const double e = cta_sum<NW>(lane_e, sm, lane, warp);
@@ -307,31 +329,6 @@ __global__ void __launch_bounds__(NW * 32) k_score_flat(const float4* __restrict
 // ---- launchers ----------------------------------------------------------------------
 constexpr int NW_SCORE = 8;
 
-// disulfide_energy (allatom.rs:155-180) of candidate c of the resident state: Gaussian
-// well between every pair of Cys SG atoms (topology atom 5), reference f32 order.
-__device__ float disulfide_energy(const StateView& st, int c) {
-    const int r0 = st.cand_res_off[c], r1 = st.cand_res_off[c + 1];
-    float ds = 0.0f;
-    for (int ri = r0; ri < r1; ++ri) {
-        if (st.res_aa[ri] != CYS) continue;
-        const float4 pi = st.res_pos[(size_t)ri * SLOT_STRIDE + 5];
-        for (int rj = ri + 1; rj < r1; ++rj) {
-            if (st.res_aa[rj] != CYS) continue;
-            const float4 pj = st.res_pos[(size_t)rj * SLOT_STRIDE + 5];
-            const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
-            if (d > 4.0f) continue;
-            const float z = xdiv(xsub(d, 2.05f), 0.4f);
-            ds = xsub(ds, xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z))));
-        }
-    }
-    return ds;
-}
-
-__global__ void k_add_disulfide(StateView st, double* __restrict__ out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < st.n_cand) out[c] += (double)disulfide_energy(st, c);
-}
-
 template <class Src>
 static void grouped(cudaStream_t s, const Src& src, int n_cand, const AgView* ags, bool kahan, bool full, bool abs_,
                     bool count, const ScoreOut& o, int g) {
@@ -366,19 +363,25 @@ int launch_score_flat(cudaStream_t s, const float* atoms, const long long* offse
     return 1;
 }
 
-// candidate energy = its residues' energies added in index order (+ disulfide when full)
-__global__ void k_sum_residues(StateView st, const double* __restrict__ res_e, const double* __restrict__ res_abs,
-                               int full, double* __restrict__ out, double* __restrict__ out_abs) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// Candidate energy = its residues' energies added in index order (+ disulfide when full),
+// one warp per candidate: the loads of 32 residues at a time run in parallel, the
+// additions keep their order.  One thread per candidate had waited for every load and
+// scanned all residues for every Cys: 64 x 20 residues 29 us, 6 us now; 64 chains of about
+// 115 residues 129 us, 13 us now.
+constexpr int SUM_WARPS = 4;
+__global__ void __launch_bounds__(SUM_WARPS * 32) k_sum_residues(StateView st, const double* __restrict__ res_e,
+                                                                 const double* __restrict__ res_abs, int full,
+                                                                 double* __restrict__ out,
+                                                                 double* __restrict__ out_abs) {
+    const int c = blockIdx.x * SUM_WARPS + (threadIdx.x >> 5);
     if (c >= st.n_cand) return;
-    double e = 0.0, ea = 0.0;
-    for (int r = st.cand_res_off[c]; r < st.cand_res_off[c + 1]; ++r) {
-        e += res_e[r];
-        if (res_abs) ea += res_abs[r];
+    double ea = 0.0;
+    const double e = warp_candidate_sum(st, c, res_e, full);
+    if (res_abs) ea = warp_ordered_sum(res_abs, st.cand_res_off[c], st.cand_res_off[c + 1]);
+    if ((threadIdx.x & 31) == 0) {
+        out[c] = e;
+        if (out_abs) out_abs[c] = ea;
     }
-    if (full) e += (double)disulfide_energy(st, c);
-    out[c] = e;
-    if (out_abs) out_abs[c] = ea;
 }
 
 // Candidate sums and survivor selection in one launch (k <= 64, segments of at most
@@ -396,7 +399,7 @@ constexpr int SS_THREADS = 1024;
 constexpr int SS_PER = 4;
 constexpr int SS_MAX = SS_THREADS * SS_PER;
 
-__global__ void __launch_bounds__(SS_THREADS) k_sum_select(StateView st, const double* __restrict__ res_e, int full,
+__global__ void __launch_bounds__(SS_THREADS) k_sum_select(StateView st, const double* __restrict__ res_e,
                                                            double* __restrict__ out, const int* __restrict__ idx_list,
                                                            const long long* __restrict__ seg_off, int k,
                                                            int* __restrict__ out_idx) {
@@ -432,7 +435,6 @@ __global__ void __launch_bounds__(SS_THREADS) k_sum_select(StateView st, const d
                 e += v3;
             }
             for (; r < r1; ++r) e += res_e[r];
-            if (full) e += (double)disulfide_energy(st, c);
             out[c] = e;
             key[q] = order_key(e);
             cid[q] = c;
@@ -578,24 +580,53 @@ __global__ void __launch_bounds__(SS_THREADS) k_sum_select(StateView st, const d
 
 bool sum_topk_fits(int k, long long max_segment) { return k > 0 && k <= 64 && max_segment <= SS_MAX; }
 
-void launch_sum_select(cudaStream_t s, const StateView& st, const double* res_e, int full, double* energy,
-                       const SumTopk& tk) {
+void launch_sum_select(cudaStream_t s, const StateView& st, const double* res_e, double* energy, const SumTopk& tk) {
     if (st.n_cand <= 0 || tk.n_seg <= 0) return;
-    k_sum_select<<<tk.n_seg, SS_THREADS, 0, s>>>(st, res_e, full, energy, tk.idx_list, tk.seg_off, tk.k, tk.out_idx);
+    k_sum_select<<<tk.n_seg, SS_THREADS, 0, s>>>(st, res_e, energy, tk.idx_list, tk.seg_off, tk.k, tk.out_idx);
 }
+
+// Four warps share a residue of the full energy while the grid's warps outnumber the
+// residues twice: a warp evaluates a residue's batches one after another, and the residues
+// deep in contact set the launch's length (1280 residues: 63 us with one warp each and
+// per-pair table lookups, 28 us now).
+static bool full_team(const StateView& st, int g, int warps) { return st.total_res * 2ll <= (long long)g * warps; }
 
 template <int NW>
 static void score_residues_nw(cudaStream_t s, int g, const StateView& st, const AgView* ags, bool kahan, bool full,
                               bool abs_, bool count, const ScoreOut& o, const StateScoreScratch& scr) {
-#define BINDER_R(K, FU, A, C)                                                                                    \
-    k_score_residues<NW, K, FU, A, C><<<g, NW * 32, 0, s>>>(st, ags, scr.order, scr.queue,                      \
-                                                            count ? nullptr : scr.res_e, scr.res_abs, o.pairs,  \
-                                                            o.err)
-    if (count) BINDER_R(true, false, false, true);
-    else if (full) BINDER_R(true, true, false, false);
-    else if (abs_) { if (kahan) BINDER_R(true, false, true, false); else BINDER_R(false, false, true, false); }
-    else { if (kahan) BINDER_R(true, false, false, false); else BINDER_R(false, false, false, false); }
+    constexpr size_t team_bytes = NW / 4 * sizeof(TeamSmem);
+#define BINDER_R(K, FU, A, C, T)                                                                                 \
+    k_score_residues<NW, K, FU, A, C, T><<<g, NW * 32, T > 1 ? team_bytes : 0, s>>>(                            \
+        st, ags, scr.order, scr.queue, count ? nullptr : scr.res_e, scr.res_abs, o.pairs, o.err)
+    if (count) BINDER_R(true, false, false, true, 1);
+    else if (full) {
+        if (full_team(st, g, NW)) {
+            if (team_bytes > 32 * 1024)
+                cudaFuncSetAttribute(k_score_residues<NW, true, true, false, false, 4>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)team_bytes);
+            BINDER_R(true, true, false, false, 4);
+        } else {
+            BINDER_R(true, true, false, false, 1);
+        }
+    }
+    else if (abs_) { if (kahan) BINDER_R(true, false, true, false, 1); else BINDER_R(false, false, true, false, 1); }
+    else { if (kahan) BINDER_R(true, false, false, false, 1); else BINDER_R(false, false, false, false, 1); }
 #undef BINDER_R
+}
+
+static void score_residues(cudaStream_t s, const StateView& st, const AgView* ags, bool kahan, bool full, bool abs_,
+                           bool count, const ScoreOut& o, const StateScoreScratch& scr, int g, int warps) {
+    switch (warps) {
+        case 4: score_residues_nw<4>(s, g, st, ags, kahan, full, abs_, count, o, scr); break;
+        case 16: score_residues_nw<16>(s, g, st, ags, kahan, full, abs_, count, o, scr); break;
+        default: score_residues_nw<8>(s, g, st, ags, kahan, full, abs_, count, o, scr); break;
+    }
+}
+
+void launch_score_full_residues(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, uint32_t* err,
+                                const StateScoreScratch& scr, int grid_ctas, int warps_per_cta) {
+    const ScoreOut o{nullptr, nullptr, nullptr, nullptr, err};
+    score_residues(s, st, ags, accumulate == 0, true, false, false, o, scr, grid_ctas, warps_per_cta);
 }
 
 int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, int full,
@@ -604,18 +635,14 @@ int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, i
     if (st.n_cand <= 0) return 0;
     const bool kahan = accumulate == 0, abs_ = o.abs_sum != nullptr, count = o.pairs != nullptr;
     const int g = grid_ctas > 0 ? grid_ctas : 148 * 4;
-    switch (warps_per_cta) {
-        case 4: score_residues_nw<4>(s, g, st, ags, kahan, full, abs_, count, o, scr); break;
-        case 16: score_residues_nw<16>(s, g, st, ags, kahan, full, abs_, count, o, scr); break;
-        default: score_residues_nw<8>(s, g, st, ags, kahan, full, abs_, count, o, scr); break;
-    }
+    score_residues(s, st, ags, kahan, full, abs_, count, o, scr, g, warps_per_cta);
     if (!count && tk && !abs_) {
         if (tk->defer) return 1;  // the sums and the selection come later (launch_sum_select)
         if (tk->mid) cudaEventRecord(tk->mid, s);
-        launch_sum_select(s, st, scr.res_e, full, o.energy, *tk);
+        launch_sum_select(s, st, scr.res_e, o.energy, *tk);
     } else if (!count) {
-        k_sum_residues<<<(st.n_cand + 127) / 128, 128, 0, s>>>(st, scr.res_e, abs_ ? scr.res_abs : nullptr, full,
-                                                               o.energy, o.abs_sum);
+        k_sum_residues<<<(st.n_cand + SUM_WARPS - 1) / SUM_WARPS, SUM_WARPS * 32, 0, s>>>(
+            st, scr.res_e, abs_ ? scr.res_abs : nullptr, full, o.energy, o.abs_sum);
     }
     return count ? 1 : 2;  // launches issued
 }

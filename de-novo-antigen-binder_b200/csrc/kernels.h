@@ -75,11 +75,13 @@ struct SumTopk {
 bool sum_topk_fits(int k, long long max_segment);
 // the candidate sums of res_e (residue energies of launch_score_state) and the
 // selection, as launch_score_state runs them after the residues
-void launch_sum_select(cudaStream_t s, const StateView& st, const double* res_e, int full, double* energy,
-                       const SumTopk& tk);
+void launch_sum_select(cudaStream_t s, const StateView& st, const double* res_e, double* energy, const SumTopk& tk);
 int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, int full,
                        const ScoreOut& out, const StateScoreScratch& scr, int grid_ctas, int warps_per_cta,
                        const SumTopk* tk = nullptr);
+// the full residue energies only (res_e)
+void launch_score_full_residues(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, uint32_t* err,
+                                const StateScoreScratch& scr, int grid_ctas, int warps_per_cta);
 
 void launch_uniform_offsets(cudaStream_t s, long long* off, int n_cand, long long n_ab);
 
@@ -163,16 +165,18 @@ cudaError_t post_init_tables();
 // every residue: the clamped grid-force step from pos_in, side chain rebuilt, into pos_out
 void launch_min_move(cudaStream_t s, const StateView& st, const AgView* ags, const float4* pos_in, float4* pos_out,
                      float step_size);
-// per candidate: keep the trial positions when e_trial < best (best updated, kept[c]++)
-void launch_min_accept(cudaStream_t s, const StateView& st, const float4* trial, const double* e_trial, double* best,
-                       int* kept);
+// per candidate: the trial's energy from its residues' (launch_score_full_residues), and
+// the trial positions kept when it is below best (best updated)
+void launch_min_accept(cudaStream_t s, const StateView& st, float4* trial, const double* res_e, double* best);
 // affinity_maturation_allatom of every candidate over its interface residues; res_e
 // (per-residue full energies of the state) kept current
 void launch_mature(cudaStream_t s, const StateView& st, const AgView* ags, double* res_e, double* out_best,
                    int* out_kept, uint32_t* err);
 
 // Fv pairs (chains 2i, 2i + 1 of the state): the all-atom energy between the chains (at
-// most 160 residues per chain, else NaN), and the elitist keep / restore of each pair
+// most 160 residues per chain, else NaN) in FV_PAIR_PARTS parts per pair, and the elitist
+// keep / restore of each pair
+constexpr int FV_PAIR_PARTS = 4;
 void launch_fv_pair(cudaStream_t s, const StateView& st, double* out);
 void launch_fv_keep(cudaStream_t s, const StateView& st, const double* e_chain, const double* e_pair, double* best,
                     float4* b_pos, uint8_t* b_aa, float4* b_chi, float4* b_trig, int restore);

@@ -138,6 +138,24 @@ struct GroupSmem {
     __align__(8) float shy[GMAX];
     int q[64];         // queued antigen atom indices
 };
+// FULL scoring: the group atoms' EEF1 parameters (c_eef1), reciprocal lambdas and H-bond
+// roles, looked up once per group.
+struct GroupFull {
+    float4 eef[GMAX];
+    float rl[GMAX];
+    int hb[GMAX];
+};
+
+// r / d, correctly rounded, from y = RN(1 / d): q = RN(r y), then one correction by the
+// exact remainder (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  For the five divisors this is used with (the EEF1
+// lambdas 3.15, 3.5, 3.7, 3.9 and the H-bond sigma 0.35) it equals the IEEE quotient for
+// every float |r| in [2^-60, 16) and 0 (checked exhaustively); three operations instead
+// of a division's dozen.
+__device__ __forceinline__ float div_by(float r, float d, float y) {
+    const float q = __fmul_rn(r, y);
+    return __fmaf_rn(__fmaf_rn(-d, q, r), y, q);
+}
 
 __device__ __forceinline__ void group_xyz(GroupSmem& s, int lane, int n, float x, float y, float z) {
     if (lane < n) {
@@ -160,57 +178,71 @@ __device__ __forceinline__ void group_prm(GroupSmem& s, int lane, int n, float q
     }
 }
 
+// The H-bond (energy.rs:303-307) and EEF1 solvation (solvation.rs:34-50) terms of a pair
+// within the cutoff, added to e: ei, yi the antigen atom's EEF1 parameters and reciprocal
+// lambda, ej, yj the candidate atom's; hb = they can form an H-bond.
+__device__ __forceinline__ float full_terms(float e, bool hb, const float4& ei, float yi, const float4& ej, float yj,
+                                            float r2, float ir) {
+    if (hb && r2 <= HB_CUTOFF_SQ) {
+        const float z = div_by(r2 * ir - HB_R0, HB_SIGMA, 1.0f / HB_SIGMA);
+        e += -HB_DEPTH * expf(-0.5f * z * z);
+    }
+    if (r2 < SOLV_CUTOFF_SQ && !(ej.y == 0.0f && ej.x == 0.0f)) {
+        const float r = r2 * ir;
+        const float xi = div_by(r, ei.z, yi), xj = div_by(r, ej.z, yj);
+        const float pi = ei.x * ej.y * expf(-(xi * xi)), pj = ej.x * ei.y * expf(-(xj * xj));
+        e -= __fmaf_rn(pj, ej.w, __fmul_rn(pi, ei.w));
+    }
+    return e;
+}
+// donor / acceptor roles of two atoms that make an H-bond (bit 0 donor, bit 1 acceptor)
+__device__ __forceinline__ bool hb_pair(int a, int b) { return (a & ((b & 1) << 1 | (b >> 1 & 1))) != 0; }
+
 // Energy of one pair within the cutoff (r2: the reference's rounding of r^2):
 // candidate atom b / bp, antigen atom a / ap, each (x, y, z, q sqrt(332)) and
 // (r_min_half, sqrt(epsilon), hydrophobic, AMBER type).  LJ + Coulomb + hydrophobic
-// (energy.rs:269-301), with FULL the H-bond (energy.rs:303-307) and EEF1 solvation
-// (solvation.rs:34-50: ei the antigen atom's, ej the candidate atom's) terms; the
-// first three are returned in lj, coul, hyd as well.
-template <bool FULL>
-__device__ __forceinline__ float pair_energy(const float4& b, const float4& bp, const float4& a, const float4& ap,
-                                             float r2, float& lj, float& coul, float& hyd) {
-    const float ir = rsqrtf(r2);
+// (energy.rs:269-301); ir = 1 / r for the further terms.
+__device__ __forceinline__ float pair_base(const float4& b, const float4& bp, const float4& a, const float4& ap,
+                                           float r2, float& ir) {
+    ir = rsqrtf(r2);
     const float ir2 = ir * ir;
     const float R = bp.x + ap.x;
     const float s2 = R * R * ir2;
     const float s6 = s2 * s2 * s2;
-    lj = (bp.y * ap.y) * (s6 * (s6 - 2.0f));
-    coul = (b.w * a.w) * ir;
-    hyd = (r2 < HYDRO_CUTOFF_SQ) ? HYDRO_BONUS * (bp.z * ap.z) : 0.0f;
-    float e = lj + coul + hyd;
-    if (FULL) {
-        const int bt = (int)bp.w, at = (int)ap.w;
-        if ((((c_hb[bt] & 1) && (c_hb[at] & 2)) || ((c_hb[bt] & 2) && (c_hb[at] & 1))) && r2 <= HB_CUTOFF_SQ) {
-            const float z = (r2 * ir - HB_R0) / HB_SIGMA;
-            e += -HB_DEPTH * expf(-0.5f * z * z);
-        }
-        const float4 ej = c_eef1[bt];
-        if (r2 < SOLV_CUTOFF_SQ && !(ej.y == 0.0f && ej.x == 0.0f)) {
-            const float4 ei = c_eef1[at];
-            const float r = r2 * ir;
-            const float xi = r / ei.z, xj = r / ej.z;
-            e += -(ei.x * ej.y * expf(-(xi * xi)) * ei.w + ej.x * ei.y * expf(-(xj * xj)) * ej.w);
-        }
-    }
-    return e;
+    const float hyd = (r2 < HYDRO_CUTOFF_SQ) ? HYDRO_BONUS * (bp.z * ap.z) : 0.0f;
+    const float le = __fmul_rn(bp.y, ap.y), ls = __fmul_rn(s6, s6 - 2.0f), qq = __fmul_rn(b.w, a.w);
+    return __fmaf_rn(qq, ir, __fmul_rn(le, ls)) + hyd;
 }
 
 // One antigen atom (this lane's) against the n group atoms in shared memory, two
 // group atoms per step: dx = b - a in packed f32x2 arithmetic, r^2 = (dx*dx + dy*dy)
 // + dz*dz with the reference's roundings (scalar, never fused), hence its pair set;
 // the terms of the pairs within the cutoff (packed) are added in group-atom order.
-template <bool KAHAN, bool FULL, bool ABS, bool COUNT>
-__device__ __forceinline__ void group_pairs(const float4* __restrict__ pq, const float4* __restrict__ prm,
-                                            const GroupSmem& s, int n, int idx, Acc& acc) {
+// Returns the atom's sum over the group (f32, group-atom order).
+template <bool FULL, bool ABS, bool COUNT>
+__device__ __forceinline__ float group_pairs(const float4* __restrict__ pq, const float4* __restrict__ prm,
+                                            const GroupSmem& s, const GroupFull* gf, int n, int idx, Acc& acc) {
+    static_assert(!FULL || !ABS, "the full energy has no absolute sum");
     const float4 a = __ldg(&pq[idx]);
     const float4 ap = __ldg(&prm[idx]);
     float part = 0.0f, pabs = 0.0f;
     int np = 0;
+    // FULL: this antigen atom's parameters, once for all group atoms (the type is the
+    // lane's: looked up per pair, its constant-table rows were fetched one distinct type
+    // after another)
+    float4 ei = make_float4(0.f, 0.f, 0.f, 0.f);
+    float yi = 0.0f;
+    int ahb = 0;
+    if (FULL) {
+        const int at = (int)ap.w;
+        ei = c_eef1[at];
+        yi = __frcp_rn(ei.z);
+        ahb = c_hb[at];
+    }
     auto term = [&](int j, float r2) {
-        float lj, coul, hyd;
-        const float e = pair_energy<FULL>(s.pos[j], s.prm[j], a, ap, r2, lj, coul, hyd);
-        part += e;
-        if (ABS) pabs += fabsf(lj) + fabsf(coul) + fabsf(hyd);
+        float ir;
+        const float e = pair_base(s.pos[j], s.prm[j], a, ap, r2, ir);
+        part += full_terms(e, hb_pair(gf->hb[j], ahb), ei, yi, gf->eef[j], gf->rl[j], r2, ir);
         if (COUNT) ++np;
     };
     const uint64_t ax = f2_pack(a.x, a.x), ay = f2_pack(a.y, a.y), az = f2_pack(a.z, a.z);
@@ -251,63 +283,92 @@ __device__ __forceinline__ void group_pairs(const float4* __restrict__ pq, const
             if (COUNT) np += (int)ina + (int)inb;
         }
     }
-    acc_add<KAHAN>(acc, part);
     if (ABS) acc.abs_s += pabs;
     if (COUNT) acc.pairs += np;
+    return part;
 }
 
-// Everything one warp does for one group already in shared memory (n atoms): centre
-// and radius, warp-uniform walk over the culled grid columns, sphere prefilter into
-// the queue, batched pair evaluation.  Accumulates into the lane's acc.
-template <bool KAHAN, bool FULL, bool ABS, bool COUNT>
-__device__ __forceinline__ void score_group(const AgView* __restrict__ Ap, GroupSmem& s, int n, int lane,
-                                            unsigned lt, Acc& acc) {
-    const float4* __restrict__ pq = Ap->pq;
-    const float4* __restrict__ prm = Ap->prm;
-    const int* __restrict__ cell_start = Ap->grid.cell_start;
+// The grid columns within 10 A + group radius of a group's centre (group atoms in shared
+// memory, all lanes call).
+struct GroupCols {
+    float cx, cy, cz, reach2;  // centre, squared reach
+    float ux, uy, uz, rc2;     // the same in cell units
+    int i0, j0, nj, ncol;
+    // atom range of column `col` (x-major): its z-run of cells within reach (empty: ra0 = ra1)
+    __device__ __forceinline__ void range(const AgView* __restrict__ Ap, int col, int& ra0, int& ra1) const {
+        ra0 = ra1 = 0;
+        if (col >= ncol) return;
+        const int i = i0 + col / nj, j = j0 + col % nj;
+        const float ddx = fmaxf(fmaxf((float)i - ux, ux - (float)(i + 1)), 0.0f);
+        const float ddy = fmaxf(fmaxf((float)j - uy, uy - (float)(j + 1)), 0.0f);
+        const float rem2 = rc2 - ddx * ddx - ddy * ddy;
+        if (!(rem2 >= 0.0f)) return;
+        const int gny = Ap->grid.ny, gnz = Ap->grid.nz;
+        const float rem = sqrtf(rem2);
+        const int k0 = max(0, (int)floorf(uz - rem)), k1 = min(gnz - 1, (int)floorf(uz + rem));
+        if (k0 <= k1) {
+            const int base = (i * gny + j) * gnz;
+            ra0 = __ldg(&Ap->grid.cell_start[base + k0]);
+            ra1 = __ldg(&Ap->grid.cell_start[base + k1 + 1]);
+        }
+    }
+};
+__device__ __forceinline__ GroupCols group_columns(const AgView* __restrict__ Ap, const GroupSmem& s, int n, int lane) {
+    GroupCols c;
     const float inv = Ap->grid.inv;
-    const int ox = Ap->grid.ox, oy = Ap->grid.oy, oz = Ap->grid.oz;
-    const int gnx = Ap->grid.nx, gny = Ap->grid.ny, gnz = Ap->grid.nz;
-    // group centre and radius
     float px = 0.f, py = 0.f, pz = 0.f;
     if (lane < n) {
         const float4 p = s.pos[lane];
         px = p.x; py = p.y; pz = p.z;
     }
     const float inv_n = 1.0f / (float)n;
-    const float cx = warp_sum_f(px) * inv_n, cy = warp_sum_f(py) * inv_n, cz = warp_sum_f(pz) * inv_n;
-    const float dgx = px - cx, dgy = py - cy, dgz = pz - cz;
+    c.cx = warp_sum_f(px) * inv_n;
+    c.cy = warp_sum_f(py) * inv_n;
+    c.cz = warp_sum_f(pz) * inv_n;
+    const float dgx = px - c.cx, dgy = py - c.cy, dgz = pz - c.cz;
     const float rad2 = warp_max_f(lane < n ? dgx * dgx + dgy * dgy + dgz * dgz : 0.0f);
     const float reach = 10.01f + sqrtf(rad2) * 1.0001f + 1e-3f;
-    const float reach2 = reach * reach;
-    // grid columns within reach of the centre (cell units)
-    const float ux = cx * inv - (float)ox, uy = cy * inv - (float)oy, uz = cz * inv - (float)oz;
-    const float rc = reach * inv, rc2 = rc * rc;
-    const int i0 = max(0, (int)floorf(ux - rc)), i1 = min(gnx - 1, (int)floorf(ux + rc));
-    const int j0 = max(0, (int)floorf(uy - rc)), j1 = min(gny - 1, (int)floorf(uy + rc));
-    // the columns (i, j) in x-major order, 32 at a time: each lane finds one column's
-    // atom range (z-run of cells within reach) in parallel, then the warp takes the
-    // non-empty ranges in column order
-    const int nj = j1 - j0 + 1;
-    const int ncol = (i1 >= i0 && j1 >= j0) ? (i1 - i0 + 1) * nj : 0;
+    c.reach2 = reach * reach;
+    c.ux = c.cx * inv - (float)Ap->grid.ox;
+    c.uy = c.cy * inv - (float)Ap->grid.oy;
+    c.uz = c.cz * inv - (float)Ap->grid.oz;
+    const float rc = reach * inv;
+    c.rc2 = rc * rc;
+    c.i0 = max(0, (int)floorf(c.ux - rc));
+    c.j0 = max(0, (int)floorf(c.uy - rc));
+    const int i1 = min(Ap->grid.nx - 1, (int)floorf(c.ux + rc)), j1 = min(Ap->grid.ny - 1, (int)floorf(c.uy + rc));
+    c.nj = j1 - c.j0 + 1;
+    c.ncol = (i1 >= c.i0 && j1 >= c.j0) ? (i1 - c.i0 + 1) * c.nj : 0;
+    return c;
+}
+// FULL scoring: the group atoms' further parameters (prm visible to the warp)
+__device__ __forceinline__ void group_full(const GroupSmem& s, GroupFull* gf, int n, int lane) {
+    if (lane < n) {
+        const int t = (int)s.prm[lane].w;
+        const float4 e = c_eef1[t];
+        gf->eef[lane] = e;
+        gf->rl[lane] = __frcp_rn(e.z);
+        gf->hb[lane] = c_hb[t];
+    }
+    __syncwarp();
+}
+
+// Everything one warp does for one group already in shared memory (n atoms): centre
+// and radius, warp-uniform walk over the culled grid columns, sphere prefilter into
+// the queue, batched pair evaluation.  Accumulates into the lane's acc.
+template <bool KAHAN, bool FULL, bool ABS, bool COUNT>
+__device__ __forceinline__ void score_group(const AgView* __restrict__ Ap, GroupSmem& s, GroupFull* gf, int n,
+                                            int lane, unsigned lt, Acc& acc) {
+    const float4* __restrict__ pq = Ap->pq;
+    const float4* __restrict__ prm = Ap->prm;
+    const GroupCols cols = group_columns(Ap, s, n, lane);
+    const float reach2 = cols.reach2, cx = cols.cx, cy = cols.cy, cz = cols.cz;
+    const int ncol = cols.ncol;
+    if (FULL) group_full(s, gf, n, lane);
     int qn = 0;
     for (int c0 = 0; c0 < ncol; c0 += 32) {
         int ra0 = 0, ra1 = 0;
-        if (c0 + lane < ncol) {
-            const int i = i0 + (c0 + lane) / nj, j = j0 + (c0 + lane) % nj;
-            const float ddx = fmaxf(fmaxf((float)i - ux, ux - (float)(i + 1)), 0.0f);
-            const float ddy = fmaxf(fmaxf((float)j - uy, uy - (float)(j + 1)), 0.0f);
-            const float rem2 = rc2 - ddx * ddx - ddy * ddy;
-            if (rem2 >= 0.0f) {
-                const float rem = sqrtf(rem2);
-                const int k0 = max(0, (int)floorf(uz - rem)), k1 = min(gnz - 1, (int)floorf(uz + rem));
-                if (k0 <= k1) {
-                    const int base = (i * gny + j) * gnz;
-                    ra0 = __ldg(&cell_start[base + k0]);
-                    ra1 = __ldg(&cell_start[base + k1 + 1]);
-                }
-            }
-        }
+        cols.range(Ap, c0 + lane, ra0, ra1);
         unsigned live = __ballot_sync(0xffffffffu, ra1 > ra0);
         while (live) {
             const int src = __ffs(live) - 1;
@@ -326,7 +387,7 @@ __device__ __forceinline__ void score_group(const AgView* __restrict__ Ap, Group
                 qn += __popc(m);
                 __syncwarp();
                 if (qn >= 32) {
-                    group_pairs<KAHAN, FULL, ABS, COUNT>(pq, prm, s, n, s.q[lane], acc);
+                    acc_add<KAHAN>(acc, group_pairs<FULL, ABS, COUNT>(pq, prm, s, gf, n, s.q[lane], acc));
                     __syncwarp();
                     if (lane < qn - 32) s.q[lane] = s.q[32 + lane];
                     qn -= 32;
@@ -335,9 +396,163 @@ __device__ __forceinline__ void score_group(const AgView* __restrict__ Ap, Group
             }
         }
     }
-    if (lane < qn) group_pairs<KAHAN, FULL, ABS, COUNT>(pq, prm, s, n, s.q[lane], acc);
+    if (lane < qn) acc_add<KAHAN>(acc, group_pairs<FULL, ABS, COUNT>(pq, prm, s, gf, n, s.q[lane], acc));
     __syncwarp();
 }
 
+// The full energy of one group by a team of TEAM warps (warp `rank`; sync(): the team's
+// barrier): what score_group's lanes sum, in the same order, with the work shared.  The
+// columns' atom ranges are concatenated; the warps prefilter 32 atoms of the concatenation
+// each (up to TEAM_SEG chunks a segment), place the passing ones in the team's list -- the
+// single warp's queue -- and evaluate its batches of 32 in turn into the team's slots;
+// warp 0 adds the slots to its acc, batch after batch, so every lane of it sums exactly
+// the terms it would sum alone.  Result in warp 0's acc.
+constexpr int TEAM_SEG = 32;
+struct TeamSmem {
+    float part[TEAM_SEG + 1][32];
+    int list[TEAM_SEG * 32 + 32];  // queued atoms: the last segment's rest, then this one's
+    int found[TEAM_SEG][32];       // passing atoms of each chunk
+    int count[TEAM_SEG];
+};
+template <bool KAHAN, int TEAM, class Sync>
+__device__ __forceinline__ void score_group_team(const AgView* __restrict__ Ap, GroupSmem& s, GroupFull* gf, int n,
+                                                 int lane, unsigned lt, Acc& acc, int rank, TeamSmem& T, Sync sync) {
+    const float4* __restrict__ pq = Ap->pq;
+    const float4* __restrict__ prm = Ap->prm;
+    const GroupCols cols = group_columns(Ap, s, n, lane);
+    group_full(s, gf, n, lane);
+    int qn = 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < cols.ncol; c0 += 32) {
+        int ra0 = 0, ra1 = 0;
+        cols.range(Ap, c0 + lane, ra0, ra1);
+        const int len = ra1 - ra0;
+        int incl = len;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        const int tot = __shfl_sync(0xffffffffu, incl, 31);
+        const bool last_cols = c0 + 32 >= cols.ncol;
+        int f0 = 0;
+        do {  // (once when tot = 0: the last segment closes the sums)
+            const int chunks = min(TEAM_SEG, (tot - f0 + 31) / 32);
+#pragma unroll 1
+            for (int ch = rank; ch < chunks; ch += TEAM) {
+                const int f = f0 + ch * 32 + lane, fq = min(f, tot - 1);
+                int lo = 0;  // the first column whose inclusive prefix exceeds fq
+#pragma unroll
+                for (int step = 16; step > 0; step >>= 1) {
+                    const int v = __shfl_sync(0xffffffffu, incl, lo + step - 1);
+                    if (v <= fq) lo += step;
+                }
+                const int v_lo = __shfl_sync(0xffffffffu, incl, lo), len_lo = __shfl_sync(0xffffffffu, len, lo);
+                const int t = __shfl_sync(0xffffffffu, ra0, lo) + (fq - (v_lo - len_lo));
+                bool pass = false;
+                if (f < tot) {
+                    const float4 a = __ldg(&pq[t]);
+                    const float ex = a.x - cols.cx, ey = a.y - cols.cy, ez = a.z - cols.cz;
+                    pass = ex * ex + ey * ey + ez * ez <= cols.reach2;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, pass);
+                if (pass) T.found[ch][__popc(m & lt)] = t;
+                if (lane == 0) T.count[ch] = __popc(m);
+            }
+            sync();
+            int at = lane < chunks ? T.count[lane] : 0;  // inclusive prefix over the chunks
+            const int own = at;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, at, d);
+                if (lane >= d) at += v;
+            }
+            const int found = __shfl_sync(0xffffffffu, at, 31);
+#pragma unroll 1
+            for (int ch = rank; ch < chunks; ch += TEAM) {
+                const int cnt = __shfl_sync(0xffffffffu, own, ch), to = qn + __shfl_sync(0xffffffffu, at, ch) - cnt;
+                if (lane < cnt) T.list[to + lane] = T.found[ch][lane];
+            }
+            qn += found;
+            f0 += TEAM_SEG * 32;
+            const bool last = last_cols && f0 >= tot;
+            sync();
+            const int full = qn / 32, rest = qn - full * 32, batches = full + (last && rest ? 1 : 0);
+#pragma unroll 1
+            for (int b = rank; b < batches; b += TEAM) {
+                if (b * 32 + lane < qn)
+                    T.part[b][lane] = group_pairs<true, false, false>(pq, prm, s, gf, n, T.list[b * 32 + lane], acc);
+            }
+            sync();
+            if (rank == 0) {
+#pragma unroll 1
+                for (int b = 0; b < batches; ++b)
+                    if (b * 32 + lane < qn) acc_add<KAHAN>(acc, T.part[b][lane]);
+                if (lane < rest && full) T.list[lane] = T.list[full * 32 + lane];
+            }
+            qn = rest;
+            if (!last) sync();  // the list's rest and the slots
+        } while (f0 < tot);
+    }
+    sync();  // the next group reuses the team's memory
+}
+
+// ---- candidate sums, by one warp ------------------------------------------------------
+// v[r0] + .. + v[r1 - 1] in order (without v[skip]); the loads of 32 run in parallel; on
+// every lane.
+__device__ __forceinline__ double warp_ordered_sum(const double* __restrict__ v, int r0, int r1, int skip = -1) {
+    const int lane = threadIdx.x & 31;
+    double e = 0.0;
+    for (int base = r0; base < r1; base += 32) {
+        const int r = base + lane;
+        const double x = r < r1 && r != skip ? v[r] : 0.0;
+        const int m = min(32, r1 - base);
+        for (int i = 0; i < m; ++i) e += __shfl_sync(0xffffffffu, x, i);
+    }
+    return e;
+}
+
+// disulfide_energy (allatom.rs:155-180) of residues r0 .. r1-1, f32 in the reference's
+// pair order: Gaussian well between every pair of Cys SG atoms (topology atom 5).
+// Residue sub (>= 0) is taken as amino acid sub_aa with its SG at sub_sg.  The lanes find
+// the Cys residues and test one Cys's partners at a time; on every lane.
+static __device__ __noinline__ float warp_disulfide(const StateView& st, int r0, int r1, int sub, int sub_aa, float4 sub_sg) {
+    const int lane = threadIdx.x & 31;
+    float ds = 0.0f;
+    for (int bi = r0; bi < r1; bi += 32) {
+        const int ri = bi + lane;
+        const bool ci = ri < r1 && (ri == sub ? sub_aa : (int)st.res_aa[ri]) == CYS;
+        for (unsigned mi = __ballot_sync(0xffffffffu, ci); mi; mi &= mi - 1) {
+            const int i = bi + __ffs(mi) - 1;
+            const float4 pi = i == sub ? sub_sg : st.res_pos[(size_t)i * SLOT_STRIDE + 5];
+            for (int bj = bi; bj < r1; bj += 32) {
+                const int j = bj + lane;
+                float t = 0.0f;
+                bool in = j > i && j < r1 && (j == sub ? sub_aa : (int)st.res_aa[j]) == CYS;
+                if (in) {
+                    const float4 pj = j == sub ? sub_sg : st.res_pos[(size_t)j * SLOT_STRIDE + 5];
+                    const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
+                    in = !(d > 4.0f);
+                    if (in) {
+                        const float z = xdiv(xsub(d, 2.05f), 0.4f);
+                        t = xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z)));
+                    }
+                }
+                for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1)
+                    ds = xsub(ds, __shfl_sync(0xffffffffu, t, __ffs(m) - 1));
+            }
+        }
+    }
+    return ds;
+}
+
+// the candidate's energy from its residues' (full: with its disulfide term)
+__device__ __forceinline__ double warp_candidate_sum(const StateView& st, int c, const double* __restrict__ res_e,
+                                                     int full) {
+    const int r0 = st.cand_res_off[c], r1 = st.cand_res_off[c + 1];
+    double e = warp_ordered_sum(res_e, r0, r1);
+    if (full) e += (double)warp_disulfide(st, r0, r1, -1, 0, make_float4(0.f, 0.f, 0.f, 0.f));
+    return e;
+}
 
 }  // namespace binder
