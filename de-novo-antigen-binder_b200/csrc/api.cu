@@ -230,6 +230,7 @@ struct binder_ctx {
     HBuf<double> h_energy;
     HBuf<uint32_t> h_err;
     size_t last_n_cand = 0;
+    long long last_n_ab = 0;  // atoms per candidate of a uniform batch (0: ctx->off holds the offsets)
     bool last_batch_valid = false;
     State st;
     // per-phase event timing of binder_block: a ring of 4 events per block
@@ -539,17 +540,19 @@ int ensure_dropin(binder_ctx* ctx, const binder_atom_cloud* ag) {
 
 int grid_ctas(binder_ctx* ctx, int n_cand) { return std::min(n_cand, ctx->num_sms * 8); }
 
-// Score n_cand ragged candidates already in ctx->cand / ctx->off against the drop-in antigen.
-int score_resident_batch(binder_ctx* ctx, int n_cand, bool want_abs) {
+// Score n_cand candidates already in ctx->cand (n_ab atoms each, or ragged with the offsets
+// in ctx->off when n_ab = 0) against the drop-in antigen.
+int score_resident_batch(binder_ctx* ctx, int n_cand, long long n_ab, bool want_abs) {
     int s;
     CK(ctx->energy.ensure(n_cand), "alloc energy");
     if (want_abs) CK(ctx->energy_abs.ensure(n_cand), "alloc energy");
     if ((s = clear_err(ctx))) return s;
     ScoreOut o{ctx->energy.p, want_abs ? ctx->energy_abs.p : nullptr, nullptr, nullptr, ctx->errf.p};
-    launch_score_flat(ctx->stream, ctx->cand.p, ctx->off.p, n_cand, ctx->d_dropin_view.p, nullptr,
-                      ctx->params.accumulate, o, grid_ctas(ctx, n_cand), 256);
+    launch_score_flat(ctx->stream, ctx->cand.p, n_ab ? nullptr : ctx->off.p, n_ab, n_cand, ctx->d_dropin_view.p,
+                      nullptr, ctx->params.accumulate, o, grid_ctas(ctx, n_cand));
     LAUNCHED("score_flat");
     ctx->last_n_cand = (size_t)n_cand;
+    ctx->last_n_ab = n_ab;
     ctx->last_batch_valid = true;
     return BINDER_OK;
 }
@@ -587,10 +590,7 @@ int score_batch_common(binder_ctx* ctx, const binder_atom_cloud* antigen, const 
     CK(ctx->cand.ensure(used * 8), "alloc candidates");
     CK(cudaMemcpyAsync(ctx->cand.p, candidates, used * sizeof(binder_gpu_atom), cudaMemcpyHostToDevice, ctx->stream),
        "candidates H2D");
-    CK(ctx->off.ensure(n_cand + 1), "alloc offsets");
-    launch_uniform_offsets(ctx->stream, ctx->off.p, (int)n_cand, (long long)n_ab);
-    LAUNCHED("uniform_offsets");
-    if ((s = score_resident_batch(ctx, (int)n_cand, out_abs != nullptr))) return s;
+    if ((s = score_resident_batch(ctx, (int)n_cand, (long long)n_ab, out_abs != nullptr))) return s;
     return fetch_energies(ctx, (int)n_cand, out64, out_abs, out32);
 }
 
@@ -787,7 +787,7 @@ int binder_score_batch_ragged(binder_ctx* ctx, const binder_atom_cloud* antigen,
                            ctx->stream),
            "candidates H2D");
     if ((s = upload(ctx, ctx->off, (const long long*)offsets, n_cand + 1, "offsets H2D"))) return s;
-    if ((s = score_resident_batch(ctx, (int)n_cand, out_abs != nullptr))) return s;
+    if ((s = score_resident_batch(ctx, (int)n_cand, 0, out_abs != nullptr))) return s;
     return fetch_energies(ctx, (int)n_cand, out, out_abs, nullptr);
 }
 
@@ -807,8 +807,8 @@ int binder_last_pair_count(binder_ctx* ctx, int64_t* out_pairs) {
     CK(cudaMemsetAsync(ctx->pairs.p, 0, sizeof(long long), ctx->stream), "memset");
     if ((s = clear_err(ctx))) return s;
     ScoreOut o{ctx->energy.p, nullptr, nullptr, ctx->pairs.p, ctx->errf.p};
-    launch_score_flat(ctx->stream, ctx->cand.p, ctx->off.p, n_cand, ctx->d_dropin_view.p, nullptr, 0, o,
-                      grid_ctas(ctx, n_cand), 256);
+    launch_score_flat(ctx->stream, ctx->cand.p, ctx->last_n_ab ? nullptr : ctx->off.p, ctx->last_n_ab, n_cand,
+                      ctx->d_dropin_view.p, nullptr, 0, o, grid_ctas(ctx, n_cand));
     LAUNCHED("score_flat_count");
     long long h = 0;
     CK(cudaMemcpyAsync(&h, ctx->pairs.p, sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream), "D2H");
@@ -950,8 +950,8 @@ int binder_forces_allatom(binder_ctx* ctx, const binder_atom_cloud* antigen, con
     CK(ctx->force.ensure(3 * n_atoms), "alloc");
     if ((s = clear_err(ctx))) return s;
     ScoreOut o{ctx->energy.p, nullptr, ctx->force.p, nullptr, ctx->errf.p};
-    launch_score_flat(ctx->stream, ctx->cand.p, ctx->off.p, (int)n_cand, ctx->d_dropin_view.p, nullptr,
-                      ctx->params.accumulate, o, grid_ctas(ctx, (int)n_cand), 256);
+    launch_score_flat(ctx->stream, ctx->cand.p, ctx->off.p, 0, (int)n_cand, ctx->d_dropin_view.p, nullptr,
+                      ctx->params.accumulate, o, grid_ctas(ctx, (int)n_cand));
     LAUNCHED("score_flat_force");
     ctx->last_batch_valid = false;
     if (n_atoms)

@@ -48,9 +48,10 @@ struct ScoreOut {
     long long* pairs;     // pair counter (may be null)
     uint32_t* err;        // error flags
 };
-// flat GpuAtom candidates (8 floats per atom), ragged offsets (n_cand + 1)
-int launch_score_flat(cudaStream_t s, const float* atoms, const long long* offsets, int n_cand, const AgView* ags,
-                      const int* cand_ag, int accumulate, const ScoreOut& out, int grid_ctas, int block);
+// flat GpuAtom candidates (8 floats per atom): ragged offsets (n_cand + 1), or n_ab atoms
+// each (offsets null)
+int launch_score_flat(cudaStream_t s, const float* atoms, const long long* offsets, long long n_ab, int n_cand,
+                      const AgView* ags, const int* cand_ag, int accumulate, const ScoreOut& out, int grid_ctas);
 // resident state (slot layout); full = add H-bond + EEF1 + disulfide.  Persistent
 // warps over a residue work queue; per-residue FP64 energies summed per candidate.
 struct StateScoreScratch {
@@ -83,7 +84,6 @@ int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, i
 void launch_score_full_residues(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, uint32_t* err,
                                 const StateScoreScratch& scr, int grid_ctas, int warps_per_cta);
 
-void launch_uniform_offsets(cudaStream_t s, long long* off, int n_cand, long long n_ab);
 
 // ---- k_topk.cu ----
 // idx_list (may be null): segment entries are energies[idx_list[j]] and report idx_list[j]

@@ -110,7 +110,7 @@ __device__ __forceinline__ float warp_max_f(float v) {
 }
 
 // ---- grouped scoring: one warp per group of <= 16 nearby candidate atoms ----------
-// A group (a residue of the resident state, or 8 consecutive GpuAtoms) sits in
+// A group (a residue of the resident state, or a few consecutive GpuAtoms) sits in
 // shared memory.  The warp walks the grid columns within 10 A + group radius of
 // the group centre (warp-uniform loop, lanes stride a column's contiguous atom
 // range), keeps the antigen atoms that pass a sphere test in a per-warp queue, and
@@ -118,7 +118,6 @@ __device__ __forceinline__ float warp_max_f(float v) {
 // pair math never runs on idle lanes.  Every lane visits its antigen atoms in
 // increasing grid order, which keeps the sums deterministic.
 constexpr int GMAX = 16;
-constexpr int FLAT_GROUP = 8;
 
 // Group atom coordinates also as separate x / y / z arrays, so that the pair test
 // reads two atoms' coordinates as one 8-byte word; entries n..GMAX-1 hold GROUP_PAD.
