@@ -239,8 +239,10 @@ struct binder_ctx {
     int ev_blocks = 0;
     int last_k = 0;
     bool async_pending = false;
-    // launch shapes (autotuned) and the CUDA graph of the search block
+    // launch shapes (by the state's size until set or autotuned) and the CUDA graph of the
+    // search block
     LaunchCfg cfg;
+    bool cfg_chosen = false;  // set or autotuned by the caller
     cudaGraphExec_t block_graph = nullptr;
     std::vector<uint64_t> block_graph_sig;  // what the captured launches baked in
     int block_graph_launches = 0;
@@ -1198,6 +1200,7 @@ int set_state_meta(binder_ctx* ctx, const std::vector<int>& off, const std::vect
     CK(S.res_abs.ensure(std::max(total, 1)), "alloc");
     S.order_valid = false;
     S.meta_epoch = ctx->ag_epoch;
+    if (!ctx->cfg_chosen) ctx->cfg = default_launch_cfg(total);
     return BINDER_OK;
 }
 }  // namespace
@@ -1436,15 +1439,16 @@ int enqueue_diffuse(binder_ctx* ctx, int n_steps, uint32_t step0, int with_noise
     } else {
         S.order_valid = false;  // residues move: the cell order is stale
     }
-    // order 3 (work-balanced tasks) is built by the flat kernel for its next launch
-    int order_mode = ctx->cfg.cg_order;
-    if (order_mode == 3 && (!ctx->cfg.cg_flat || !S.cg_bal.p)) order_mode = 1;
     int max_ag = 0, max_cells = 0;
     for (const auto& a : ctx->ags) {
         const GridView& gv = a->view.ca_grid;
         max_ag = std::max(max_ag, a->n_res);
         max_cells = std::max(max_cells, gv.nx * gv.ny * gv.nz);
     }
+    // order 3 (work-balanced tasks) is built by the flat kernel for its next launch (the flat
+    // form takes antigens of at most 65536 Calphas, see launch_diffuse)
+    int order_mode = ctx->cfg.cg_order;
+    if (order_mode == 3 && (!ctx->cfg.cg_flat || !S.cg_bal.p || max_ag > 65536)) order_mode = 1;
     // the antigen every candidate probes, if they share one (staged in shared memory)
     int stage_ag = S.h_cand_ag.empty() ? -1 : S.h_cand_ag[0];
     for (int a : S.h_cand_ag)
@@ -1777,6 +1781,7 @@ int binder_set_launch_cfg(binder_ctx* ctx, const binder_launch_cfg* c) {
     ctx->cfg.score_order = c->score_order;
     ctx->cfg.cg_queue = c->cg_queue;
     ctx->cfg.cg_flat = c->cg_flat;
+    ctx->cfg_chosen = true;
     return BINDER_OK;
 }
 
@@ -1791,6 +1796,7 @@ int binder_autotune(binder_ctx* ctx, int reps, binder_launch_cfg* out) {
     for (const auto& e : ctx->tune_cache)
         if (e.first == key) {
             ctx->cfg = e.second;
+            ctx->cfg_chosen = true;
             return out ? binder_get_launch_cfg(ctx, out) : BINDER_OK;
         }
     if ((s = clear_err(ctx))) return s;
@@ -1853,6 +1859,7 @@ int binder_autotune(binder_ctx* ctx, int reps, binder_launch_cfg* out) {
     CK(cudaMemcpyAsync(S.res_pos.p, saved.p, n_slots * sizeof(float4), cudaMemcpyDeviceToDevice, ctx->stream), "copy");
     CK(cudaStreamSynchronize(ctx->stream), "synchronize");
     ctx->cfg = best;
+    ctx->cfg_chosen = true;
     if (s) return s;
     if ((s = check_err(ctx))) return s;
     tune_cache_store(ctx, key, best);

@@ -11,6 +11,8 @@
 //
 // Precision: f32 pair terms, per-lane compensated (Kahan) sums, FP64 warp-shuffle and
 // fixed-order FP64 sums above them (deterministic).
+#include <algorithm>
+
 #include "kernels.h"
 #include "score.cuh"
 #include "topk.cuh"
@@ -626,13 +628,9 @@ static void score_residues_nw(cudaStream_t s, int g, const StateView& st, const 
         st, ags, scr.order, scr.queue, count ? nullptr : scr.res_e, scr.res_abs, o.pairs, o.err)
     if (count) BINDER_R(true, false, false, true, 1);
     else if (full) {
-        if (full_team(st, g, NW)) {
-            if (team_bytes > 32 * 1024)
-                cudaFuncSetAttribute(k_score_residues<NW, true, true, false, false, 4>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)team_bytes);
-            BINDER_R(true, true, false, false, 4);
-        } else {
-            BINDER_R(true, true, false, false, 1);
+        if constexpr (NW == NW_SCORE) {
+            if (full_team(st, g, NW)) BINDER_R(true, true, false, false, 4);
+            else BINDER_R(true, true, false, false, 1);
         }
     }
     else if (abs_) { if (kahan) BINDER_R(true, false, true, false, 1); else BINDER_R(false, false, true, false, 1); }
@@ -649,10 +647,13 @@ static void score_residues(cudaStream_t s, const StateView& st, const AgView* ag
     }
 }
 
+// The full energy takes CTAs of 8 warps whatever the plain score's shape (its 79 registers
+// a thread leave room for 24 warps per SM that way, for 16 in CTAs of 16).
 void launch_score_full_residues(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, uint32_t* err,
                                 const StateScoreScratch& scr, int grid_ctas, int warps_per_cta) {
     const ScoreOut o{nullptr, nullptr, nullptr, nullptr, err};
-    score_residues(s, st, ags, accumulate == 0, true, false, false, o, scr, grid_ctas, warps_per_cta);
+    score_residues_nw<NW_SCORE>(s, std::max(1, grid_ctas * warps_per_cta / NW_SCORE), st, ags, accumulate == 0, true,
+                                false, false, o, scr);
 }
 
 int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, int full,
@@ -661,7 +662,8 @@ int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, i
     if (st.n_cand <= 0) return 0;
     const bool kahan = accumulate == 0, abs_ = o.abs_sum != nullptr, count = o.pairs != nullptr;
     const int g = grid_ctas > 0 ? grid_ctas : 148 * 4;
-    score_residues(s, st, ags, kahan, full, abs_, count, o, scr, g, warps_per_cta);
+    if (full && !count) launch_score_full_residues(s, st, ags, accumulate, o.err, scr, g, warps_per_cta);
+    else score_residues(s, st, ags, kahan, false, abs_, count, o, scr, g, warps_per_cta);
     if (!count && tk && !abs_) {
         if (tk->defer) return 1;  // the sums and the selection come later (launch_sum_select)
         if (tk->mid) cudaEventRecord(tk->mid, s);

@@ -11,16 +11,33 @@ namespace binder {
 // depend on them: every residue is computed by the same lanes with the same
 // arithmetic whatever the grid).
 struct LaunchCfg {
-    int score_warps = 8;         // warps per CTA of the persistent scoring kernel (4, 8, 16)
-    int score_ctas_per_sm = 4;   // persistent scoring CTAs per SM
-    int cg_warps = 8;            // warps per CTA of the gradient-step kernel (2, 4, 8)
+    int score_warps = 16;        // warps per CTA of the persistent scoring kernel (4, 8, 16)
+    int score_ctas_per_sm = 2;   // persistent scoring CTAs per SM
+    int cg_warps = 4;            // warps per CTA of the gradient-step kernel (2, 4, 8)
     int cg_lanes = 8;            // lanes per residue of the gradient-step kernel (4, 8)
-    int cg_order = 1;            // residue order of the gradient-step kernel: 0 cell, 1 candidate, 2 strided
-    int score_order = 0;         // work-queue order of the scoring kernel: 0 cell, 1 residue index
-    int cg_queue = 1;            // gradient-step kernel: 0 static grid, 1 persistent CTAs on a work queue
-    int cg_flat = 0;             // gradient-step kernel: 0 lane groups (cg_lanes per residue), 8 / 16 / 32 the
+    int cg_order = 3;            // residue order of the gradient-step kernel: 0 cell, 1 candidate, 2 strided,
+                                 // 3 work-balanced tasks
+    int score_order = 1;         // work-queue order of the scoring kernel: 0 cell, 1 residue index
+    int cg_queue = 0;            // gradient-step kernel: 0 static grid, 1 persistent CTAs on a work queue
+    int cg_flat = 8;             // gradient-step kernel: 0 lane groups (cg_lanes per residue), 4 / 8 / 16 / 32 the
                                  // flat form with that many residues per warp
 };
+
+// The shapes of a state of total_res residues when the caller neither set nor tuned them.
+// Gradient steps (10, us): the flat form with work-balanced tasks beats the lane groups at
+// every size -- 1280 residues 50 (4 a warp; 8 a warp 54) against 72, 9000 66 (8) against
+// 113, 20480 73 against 133, 81 k residues of 8 antigens 226 with 8 warps on the work queue
+// (297 with 4 warps static) against 376.  Scores in residue order: the cell order's better
+// locality (68 against 73 us at 20480) does not pay for its three sorting launches (17 us).
+inline LaunchCfg default_launch_cfg(int total_res) {
+    LaunchCfg c;
+    if (total_res < 4096) c.cg_flat = 4;
+    if (total_res >= 32768) {
+        c.cg_warps = 8;
+        c.cg_queue = 1;
+    }
+    return c;
+}
 
 // ---- k_grid.cu: SpatialHashGrid ----
 void launch_cell_coords(cudaStream_t s, const float* x, const float* y, const float* z, int n, float inv, int4* cells,
