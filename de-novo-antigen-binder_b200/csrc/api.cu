@@ -181,7 +181,7 @@ struct MlpState {
     DBuf<__nv_bfloat16> X, Xt, H1, H1t, H2, H2t, dY, dYt, dZ2, dZ2t, dZ1t, S1, S2;
     DBuf<float> Y, part, feat, ca, target;
     DBuf<uint8_t> aa;
-    DBuf<int> ag, action, ref, idx;
+    DBuf<int> ag, action, ref;
     DBuf<double> loss;
     DBuf<MlpTuple> tuples;
     size_t n_tuples = 0;
@@ -2454,7 +2454,6 @@ int mlp_reserve(binder_ctx* ctx, int rows) {
     CK(M.ag.ensure(c), "mlp alloc");
     CK(M.action.ensure(c), "mlp alloc");
     CK(M.ref.ensure(c), "mlp alloc");
-    CK(M.idx.ensure(c), "mlp alloc");
     M.cap = cap;
     return BINDER_OK;
 }
@@ -2462,7 +2461,7 @@ int mlp_reserve(binder_ctx* ctx, int rows) {
 constexpr int MLP_KSPLIT = 512;  // batch rows per split-K slice of the weight-gradient GEMMs
 
 int gemm(binder_ctx* ctx, const GemmArgs& g, const char* what) {
-    CK(launch_gemm_tc(ctx->stream, g, ctx->errf.p), what);
+    CK(launch_gemm_tc(ctx->stream, &g, 1, ctx->errf.p), what);
     ctx->launches++;
     return BINDER_OK;
 }
@@ -2497,39 +2496,17 @@ int mlp_forward_dev(binder_ctx* ctx, int m, bool train) {
     return gemm(ctx, g, "mlp layer 3");
 }
 
-// dW = G^T * A over the batch: G^T [rows][mp] and A^T [n][mp] (BF16), split-K
-// partials reduced in a fixed order into grad (FP32 [rows][n]).
-int mlp_weight_grad(binder_ctx* ctx, const __nv_bfloat16* Gt, int rows, const __nv_bfloat16* At, int n, int mp,
-                    float* grad) {
-    MlpState& M = ctx->mlp;
-    const int slices = (mp + MLP_KSPLIT - 1) / MLP_KSPLIT;
-    const long long stride = (long long)rows * n;
-    CK(M.part.ensure((size_t)slices * stride), "mlp alloc");
-    GemmArgs g;
-    g.a = Gt; g.lda = mp; g.m = rows;
-    g.b = At; g.ldb = mp; g.n = n; g.k = mp; g.k_split = MLP_KSPLIT;
-    g.e.mode = EPI_PARTIAL; g.e.c = M.part.p; g.e.ldc = n; g.e.part_stride = stride;
-    g.e.n_valid = n; g.e.m_valid = rows;
-    int s = gemm(ctx, g, "mlp weight grad");
-    if (s) return s;
-    launch_reduce_partials(ctx->stream, (int)stride, slices, stride, M.part.p, grad);
-    LAUNCHED("mlp reduce");
-    return BINDER_OK;
-}
-
 // Loss and gradient of the batch in M.X / M.action / M.target (m rows; reference
-// outputs in M.ref when with_ref) into M.g.
-int mlp_backward_dev(binder_ctx* ctx, int m, float delta, bool with_ref) {
+// outputs in M.ref when with_ref): the bias entries of M.g, the weight gradients as
+// split-K partials (launch_update sums them).
+int mlp_backward_dev(binder_ctx* ctx, int m, float delta, bool with_ref, MlpPartials& part) {
     MlpState& M = ctx->mlp;
     const int mp = round_up(m, 128);
     int s;
     launch_mlp_loss(ctx->stream, m, mp, M.Y.p, M.action.p, with_ref ? M.ref.p : nullptr, M.target.p, delta, M.dY.p,
                     M.dYt.p, M.loss.p);
     LAUNCHED("mlp loss");
-    // layer 3: dW3 = dY^T H2, db3 = colsum dY, dZ2 = (dY W3) * silu'(Z2)
-    if ((s = mlp_weight_grad(ctx, M.dYt.p, MLP_OUT_PAD, M.H2t.p, MLP_H, mp, M.g.p + MLP_OFF_W3))) return s;
-    launch_rowsum_bf16(ctx->stream, MLP_OUT_PAD, mp, mp, M.dYt.p, M.g.p + MLP_OFF_B3);
-    LAUNCHED("mlp bias grad");
+    // layer 3: dZ2 = (dY W3) * silu'(Z2)
     GemmArgs g;
     g.a = M.dY.p; g.lda = MLP_OUT_PAD; g.m = mp;
     g.b = M.w3t.p; g.ldb = MLP_OUT_PAD; g.n = MLP_H; g.k = MLP_OUT_PAD; g.k_split = 64;
@@ -2538,16 +2515,32 @@ int mlp_backward_dev(binder_ctx* ctx, int m, float delta, bool with_ref) {
     g.e.ht = M.dZ2t.p; g.e.ldht = mp; g.e.ht_rows = mp;
     g.e.n_valid = MLP_H; g.e.m_valid = m;
     if ((s = gemm(ctx, g, "mlp dZ2"))) return s;
-    // layer 2: dW2 = dZ2^T H1, db2, dZ1 = (dZ2 W2) * silu'(Z1)
-    if ((s = mlp_weight_grad(ctx, M.dZ2t.p, MLP_H, M.H1t.p, MLP_H, mp, M.g.p + MLP_OFF_W2))) return s;
-    launch_rowsum_bf16(ctx->stream, MLP_H, mp, mp, M.dZ2t.p, M.g.p + MLP_OFF_B2);
-    LAUNCHED("mlp bias grad");
+    // layer 2: dZ1 = (dZ2 W2) * silu'(Z1)
     g.a = M.dZ2.p; g.lda = MLP_H; g.b = M.w2t.p; g.ldb = MLP_H; g.k = MLP_H; g.k_split = MLP_H;
     g.e.sp = M.S1.p; g.e.h = nullptr; g.e.ht = M.dZ1t.p;
     if ((s = gemm(ctx, g, "mlp dZ1"))) return s;
-    // layer 1: dW1 = dZ1^T X, db1
-    if ((s = mlp_weight_grad(ctx, M.dZ1t.p, MLP_H, M.Xt.p, MLP_K1, mp, M.g.p + MLP_OFF_W1))) return s;
-    launch_rowsum_bf16(ctx->stream, MLP_H, mp, mp, M.dZ1t.p, M.g.p + MLP_OFF_B1);
+    // dW = G^T A over the batch of all three layers (G^T [rows][mp], A^T [n][mp], BF16):
+    // dW1 = dZ1^T X, dW2 = dZ2^T H1, dW3 = dY^T H2; and the bias gradients, G^T's row sums
+    const int slices = (mp + MLP_KSPLIT - 1) / MLP_KSPLIT;
+    const size_t n1 = (size_t)MLP_H * MLP_K1, n2 = (size_t)MLP_H * MLP_H, n3 = (size_t)MLP_OUT_PAD * MLP_H;
+    CK(M.part.ensure(slices * (n1 + n2 + n3)), "mlp alloc");
+    part = MlpPartials{{M.part.p, M.part.p + slices * n1, M.part.p + slices * (n1 + n2)}, slices};
+    GemmArgs dw[3];
+    const __nv_bfloat16* gt[3] = {M.dZ1t.p, M.dZ2t.p, M.dYt.p};
+    const __nv_bfloat16* at[3] = {M.Xt.p, M.H1t.p, M.H2t.p};
+    const int rows[3] = {MLP_H, MLP_H, MLP_OUT_PAD}, cols[3] = {MLP_K1, MLP_H, MLP_H};
+    for (int l = 0; l < 3; ++l) {
+        dw[l].a = gt[l]; dw[l].lda = mp; dw[l].m = rows[l];
+        dw[l].b = at[l]; dw[l].ldb = mp; dw[l].n = cols[l]; dw[l].k = mp; dw[l].k_split = MLP_KSPLIT;
+        dw[l].e.mode = EPI_PARTIAL; dw[l].e.c = const_cast<float*>(part.p[l]); dw[l].e.ldc = cols[l];
+        dw[l].e.part_stride = (long long)rows[l] * cols[l];
+        dw[l].e.n_valid = cols[l]; dw[l].e.m_valid = rows[l];
+    }
+    CK(launch_gemm_tc(ctx->stream, dw, 3, ctx->errf.p), "mlp weight grad");
+    ctx->launches++;
+    launch_rowsum_bf16(ctx->stream, RowSums{{gt[0], gt[1], gt[2]},
+                                            {M.g.p + MLP_OFF_B1, M.g.p + MLP_OFF_B2, M.g.p + MLP_OFF_B3},
+                                            {rows[0], rows[1], rows[2]}, mp});
     LAUNCHED("mlp bias grad");
     return BINDER_OK;
 }
@@ -2692,8 +2685,12 @@ int binder_mlp_loss_grad(binder_ctx* ctx, size_t n, const float* features, const
     launch_transpose_bf16(ctx->stream, mp, MLP_K1, M.X.p, M.Xt.p);
     LAUNCHED("mlp transpose");
     CK(cudaMemsetAsync(M.loss.p, 0, sizeof(double), ctx->stream), "mlp memset");
-    if ((s = mlp_forward_dev(ctx, (int)n, true)) || (s = mlp_backward_dev(ctx, (int)n, huber_delta, ref != nullptr)))
+    MlpPartials part;
+    if ((s = mlp_forward_dev(ctx, (int)n, true)) ||
+        (s = mlp_backward_dev(ctx, (int)n, huber_delta, ref != nullptr, part)))
         return s;
+    launch_update(ctx->stream, part, M.w.p, M.g.p, M.m1.p, M.m2.p, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, M.bf16(), false);
+    LAUNCHED("mlp gradient");
     double loss = 0.0;
     CK(cudaMemcpyAsync(&loss, M.loss.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "mlp D2H");
     if (out_grad)
@@ -2754,11 +2751,8 @@ int binder_mlp_train(binder_ctx* ctx, int n_steps, int batch, float lr, float hu
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     double* loss_base = M.loss.p;
     for (int step = 0; step < n_steps; ++step) {
-        launch_draw_batch(ctx->stream, batch, (int)std::min<size_t>(M.n_tuples, INT32_MAX), seed, (uint32_t)M.adam_t,
-                          M.idx.p);
-        LAUNCHED("mlp draw batch");
-        launch_gather_tuples(ctx->stream, batch, M.idx.p, M.tuples.p, M.ca.p, M.aa.p, M.ag.p, M.action.p, M.ref.p,
-                             M.target.p);
+        launch_gather_tuples(ctx->stream, batch, (int)std::min<size_t>(M.n_tuples, INT32_MAX), seed,
+                             (uint32_t)M.adam_t, M.tuples.p, M.ca.p, M.aa.p, M.ag.p, M.action.p, M.ref.p, M.target.p);
         LAUNCHED("mlp gather");
         launch_features(ctx->stream, batch, mp, M.ca.p, M.aa.p, M.ag.p, ctx->d_views.p, M.X.p);
         LAUNCHED("features");
@@ -2766,14 +2760,14 @@ int binder_mlp_train(binder_ctx* ctx, int n_steps, int batch, float lr, float hu
         LAUNCHED("mlp transpose");
         M.loss.p = loss_base + step;  // per-step loss slot
         s = mlp_forward_dev(ctx, batch, true);
-        if (!s) s = mlp_backward_dev(ctx, batch, huber_delta, true);
+        MlpPartials part;
+        if (!s) s = mlp_backward_dev(ctx, batch, huber_delta, true, part);
         M.loss.p = loss_base;
         if (s) return s;
         M.adam_t += 1;
         const float bc1 = 1.0f - std::pow(b1, (float)M.adam_t), bc2 = 1.0f - std::pow(b2, (float)M.adam_t);
-        launch_adam(ctx->stream, MLP_N_PARAMS, M.w.p, M.g.p, M.m1.p, M.m2.p, lr, b1, b2, eps, bc1, bc2);
-        LAUNCHED("mlp adam");
-        if ((s = mlp_pack(ctx))) return s;
+        launch_update(ctx->stream, part, M.w.p, M.g.p, M.m1.p, M.m2.p, lr, b1, b2, eps, bc1, bc2, M.bf16(), true);
+        LAUNCHED("mlp update");
     }
     if (out_losses && n_steps > 0)
         CK(cudaMemcpyAsync(out_losses, loss_base, (size_t)n_steps * sizeof(double), cudaMemcpyDeviceToHost,

@@ -152,8 +152,9 @@ __device__ __forceinline__ void tc_commit(uint64_t* b) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(b))
                  : "memory");
 }
-// 32 lanes x 8 consecutive FP32 columns: thread t of the warp gets lane (base lane + t)
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8]) {
+// 32 lanes x 8 consecutive FP32 columns: thread t of the warp gets lane (base lane + t);
+// the registers are valid after tc_ld_wait
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, float* v) {
     uint32_t r[8];
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -184,89 +185,103 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 __device__ __forceinline__ float sigmoid_fast(float z) { return rcp_approx(1.0f + __expf(-z)); }
 
 // ---- C[M x N] = A[M x K] * B[N x K]^T on the tensor cores ----------------------------
-// One CTA of 256 threads per 128-row tile of A (blockIdx.x) and K slice (blockIdx.y,
-// split-K); the whole N (16..256, multiple of 16) in one tensor-memory accumulator.
-// A rows >= m and K beyond the slice are zero-filled in shared memory.  Warps w and
-// w + 4 read the accumulator lanes 32 (w % 4) .. +31 and split its columns.
-constexpr int G_M = 128, G_K = 64, G_THREADS = 256;
+// One CTA of 256 threads per 128-row tile of A, 64-column tile of the outputs and K
+// slice (split-K), its accumulator in tensor memory; up to three GEMMs in one launch (the
+// weight gradients), their CTAs numbered one after another.  A rows >= m and K beyond the
+// slice are zero-filled in shared memory.  Warps w and w + 4 read the accumulator lanes
+// 32 (w % 4) .. +31 and split its columns.
+// These GEMMs are small (8192 x 256 x 192 and the like), so what bounds them is one CTA's
+// chain of loads, MMAs and epilogue: 64-column tiles give 4 times the CTAs and a quarter of
+// the epilogue each, four stages keep three chunks of K in flight (training step of 8192
+// rows: forward and data-gradient GEMMs 27 us each, now GEMM_A; weight gradients 43 + 43 +
+// 25 us, now GEMM_B in one launch).  Every output sums over K in the same order as before.
+constexpr int G_M = 128, G_K = 64, G_N = 64, G_THREADS = 256, G_STAGES = 4;
 constexpr int G_STAGE_A = G_M * G_K * 2;                       // 16 KB
-__host__ __device__ constexpr int gemm_stage_bytes(int n) { return G_STAGE_A + n * G_K * 2; }
-__host__ __device__ constexpr int gemm_smem_bytes(int n) { return 2 * gemm_stage_bytes(n) + 1024; }
+constexpr int G_STAGE = G_STAGE_A + G_N * G_K * 2;
+constexpr int G_SMEM = G_STAGES * G_STAGE + 1024;
+struct GemmGroup {
+    GemmArgs g[3];
+    int first[4];  // first CTA of each GEMM, then the total
+};
 
 // core-matrix offset of (row r, 8-element K group kg) inside a stage operand
 __device__ __forceinline__ uint32_t cm_off(int r, int kg) { return (uint32_t)((r >> 3) * 1024 + kg * 128 + (r & 7) * 16); }
 
-__global__ void __launch_bounds__(G_THREADS) k_gemm_tc(GemmArgs g, uint32_t* __restrict__ err) {
+__global__ void __launch_bounds__(G_THREADS) k_gemm_tc(const __grid_constant__ GemmGroup group,
+                                                        uint32_t* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char g_smem[];
-    __shared__ __align__(8) uint64_t s_bar[2];
+    __shared__ __align__(8) uint64_t s_bar[G_STAGES];
     __shared__ uint32_t s_tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * G_M;
-    const int k_begin = blockIdx.y * g.k_split;
+    const int which = (int)blockIdx.x >= group.first[2] ? 2 : (int)blockIdx.x >= group.first[1] ? 1 : 0;
+    const GemmArgs& g = group.g[which];
+    // CTA -> (row tile, K slice, column tile), columns fastest (they share the rows of A)
+    const int n_tiles = (g.n + G_N - 1) / G_N, m_tiles = (g.m + G_M - 1) / G_M;
+    int cta = (int)blockIdx.x - group.first[which];
+    const int n0 = cta % n_tiles * G_N;
+    cta /= n_tiles;
+    const int m0 = cta % m_tiles * G_M, slice = cta / m_tiles;
+    const int nt = min(G_N, g.n - n0);  // columns of this tile (16, 32, 48 or 64)
+    const int k_begin = slice * g.k_split;
     const int k_end = min(g.k, k_begin + g.k_split);
     const int n_chunks = (k_end - k_begin + G_K - 1) / G_K;
     const uint32_t base = (smem_u32(g_smem) + 1023u) & ~1023u;
-    const int stage_bytes = gemm_stage_bytes(g.n);
-    const uint32_t ncols = g.n <= 32 ? 32u : (g.n <= 64 ? 64u : (g.n <= 128 ? 128u : 256u));
+    const uint32_t ncols = nt <= 32 ? 32u : 64u;
 
     if (warp == 0) {
         tmem_alloc(&s_tmem, ncols);
         tmem_relinquish();
     }
-    if (tid == 0) {
-        mbar_init(&s_bar[0], 1);
-        mbar_init(&s_bar[1], 1);
-    }
+    if (tid == 0)
+        for (int i = 0; i < G_STAGES; ++i) mbar_init(&s_bar[i], 1);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t idesc = idesc_bf16(G_M, g.n);
+    const uint32_t idesc = idesc_bf16(G_M, nt);
 
-    auto load_chunk = [&](int c, int st) {
-        const int k0 = k_begin + c * G_K;
-        const uint32_t sa = base + st * stage_bytes, sb = sa + G_STAGE_A;
-        for (int p = tid; p < G_M * 8; p += G_THREADS) {
-            const int r = p >> 3, kg = p & 7, k = k0 + kg * 8;
-            const bool ok = m0 + r < g.m && k < k_end;
-            const __nv_bfloat16* src = ok ? g.a + (size_t)(m0 + r) * g.lda + k : g.a;
-            cp_async16(sa + cm_off(r, kg), src, ok);
-        }
-        for (int p = tid; p < g.n * 8; p += G_THREADS) {
-            const int r = p >> 3, kg = p & 7, k = k0 + kg * 8;
-            const bool ok = k < k_end;
-            const __nv_bfloat16* src = ok ? g.b + (size_t)r * g.ldb + k : g.b;
-            cp_async16(sb + cm_off(r, kg), src, ok);
+    auto load_chunk = [&](int c) {  // (a group is committed for chunks past the end, too)
+        if (c < n_chunks) {
+            const int k0 = k_begin + c * G_K;
+            const uint32_t sa = base + (c % G_STAGES) * G_STAGE, sb = sa + G_STAGE_A;
+#pragma unroll
+            for (int p = tid; p < G_M * 8; p += G_THREADS) {
+                const int r = p >> 3, kg = p & 7, k = k0 + kg * 8;
+                const bool ok = m0 + r < g.m && k < k_end;
+                const __nv_bfloat16* src = ok ? g.a + (size_t)(m0 + r) * g.lda + k : g.a;
+                cp_async16(sa + cm_off(r, kg), src, ok);
+            }
+            for (int p = tid; p < nt * 8; p += G_THREADS) {
+                const int r = p >> 3, kg = p & 7, k = k0 + kg * 8;
+                const bool ok = k < k_end;
+                const __nv_bfloat16* src = ok ? g.b + (size_t)(n0 + r) * g.ldb + k : g.b;
+                cp_async16(sb + cm_off(r, kg), src, ok);
+            }
         }
         cp_async_commit();
     };
 
     bool ok = true;
-    if (n_chunks > 0) load_chunk(0, 0);
+    for (int c = 0; c < G_STAGES - 1; ++c) load_chunk(c);
     for (int c = 0; c < n_chunks && ok; ++c) {
-        const int st = c & 1;
-        if (c + 1 < n_chunks) {
-            // stage st^1 was read by the MMAs of chunk c-1: wait for them before refilling it
-            if (c >= 1) ok = mbar_wait(&s_bar[st ^ 1], ((c - 1) >> 1) & 1);
-            if (!ok) break;
-            load_chunk(c + 1, st ^ 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
+        cp_async_wait<G_STAGES - 2>();
         fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t sa = base + st * stage_bytes, sb = sa + G_STAGE_A;
+            const uint32_t sa = base + (c % G_STAGES) * G_STAGE, sb = sa + G_STAGE_A;
             const int kc = min(G_K, k_end - (k_begin + c * G_K));
             for (int j = 0; j < kc / 16; ++j)
                 tc_mma(tmem, smem_desc(sa + 256 * j, 128, 1024), smem_desc(sb + 256 * j, 128, 1024), idesc,
                        (c > 0 || j > 0) ? 1u : 0u);
-            tc_commit(&s_bar[st]);
+            tc_commit(&s_bar[c % G_STAGES]);
         }
+        // the next chunk's stage was read by the MMAs of chunk c-1: wait for them first
+        if (c >= 1 && c + G_STAGES - 1 < n_chunks) ok = mbar_wait(&s_bar[(c - 1) % G_STAGES], ((c - 1) / G_STAGES) & 1);
+        if (ok) load_chunk(c + G_STAGES - 1);
     }
-    if (ok && n_chunks > 0) ok = mbar_wait(&s_bar[(n_chunks - 1) & 1], ((n_chunks - 1) >> 1) & 1);
+    cp_async_wait<0>();
+    if (ok && n_chunks > 0) ok = mbar_wait(&s_bar[(n_chunks - 1) % G_STAGES], ((n_chunks - 1) / G_STAGES) & 1);
     // every thread saw the same waits; a thread that gave up raises the flag
     if (!ok && err) atomicOr(err, ERRF_TIMEOUT);
     tc_fence_after();
@@ -277,19 +292,19 @@ __global__ void __launch_bounds__(G_THREADS) k_gemm_tc(GemmArgs g, uint32_t* __r
     const int row = m0 + wl * 32 + lane;
     const bool row_ok = row < g.e.m_valid;
     const GemmEpi& e = g.e;
-    const int n8 = g.n / 8;                        // column groups of 8
+    const int n8 = nt / 8;                         // column groups of 8
     const int cg0 = (n8 * half) / 2, cg1 = (n8 * (half + 1)) / 2;
     for (int cgi = cg0; cgi < cg1 && ok; ++cgi) {
-        const int c0 = cgi * 8;
+        const int c0 = n0 + cgi * 8;
         float v[8];
-        if (n_chunks > 0) tc_ld8(tmem + ((uint32_t)(wl * 32) << 16) + (uint32_t)c0, v);
+        if (n_chunks > 0) tc_ld8(tmem + ((uint32_t)(wl * 32) << 16) + (uint32_t)(cgi * 8), v);
         else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = 0.0f;
         }
         if (e.mode == EPI_F32 || e.mode == EPI_PARTIAL) {
             if (row_ok) {
-                float* out = e.c + (e.mode == EPI_PARTIAL ? (size_t)blockIdx.y * e.part_stride : 0) +
+                float* out = e.c + (e.mode == EPI_PARTIAL ? (size_t)slice * e.part_stride : 0) +
                              (size_t)row * e.ldc;
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
@@ -344,16 +359,28 @@ cudaError_t launch_wait_selftest(cudaStream_t s, uint32_t max_polls, uint32_t* e
     return cudaGetLastError();
 }
 
-cudaError_t launch_gemm_tc(cudaStream_t s, const GemmArgs& g, uint32_t* err) {
-    if (g.n < 16 || g.n > 256 || g.n % 16 || g.k % 16 || g.lda % 8 || g.ldb % 8 || g.k_split % G_K)
-        return cudaErrorInvalidValue;
-    const int smem = gemm_smem_bytes(g.n);
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+cudaError_t launch_gemm_tc(cudaStream_t s, const GemmArgs* g, int count, uint32_t* err) {
+    if (count < 1 || count > 3) return cudaErrorInvalidValue;
+    GemmGroup group;
+    int ctas = 0;
+    for (int i = 0; i < 3; ++i) {
+        group.first[i] = ctas;
+        if (i >= count) {
+            group.first[i] = INT32_MAX;  // no CTA
+            continue;
+        }
+        if (g[i].n < 16 || g[i].n > 256 || g[i].n % 16 || g[i].k % 16 || g[i].lda % 8 || g[i].ldb % 8 ||
+            g[i].k_split % G_K)
+            return cudaErrorInvalidValue;
+        group.g[i] = g[i];
+        const int m_tiles = (g[i].m + G_M - 1) / G_M, k_slices = (g[i].k + g[i].k_split - 1) / g[i].k_split;
+        ctas += std::max(0, m_tiles * k_slices) * ((g[i].n + G_N - 1) / G_N);
+    }
+    group.first[3] = ctas;
+    if (ctas == 0) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, G_SMEM);
     if (e) return e;
-    const int m_tiles = (g.m + G_M - 1) / G_M;
-    const int k_slices = (g.k + g.k_split - 1) / g.k_split;
-    if (m_tiles <= 0 || k_slices <= 0) return cudaSuccess;
-    k_gemm_tc<<<dim3(m_tiles, k_slices), G_THREADS, smem, s>>>(g, err);
+    k_gemm_tc<<<ctas, G_THREADS, G_SMEM, s>>>(group, err);
     return cudaGetLastError();
 }
 
@@ -383,48 +410,97 @@ __global__ void k_mlp_loss(int m, int m_pad, const float* __restrict__ Y, const 
             g = fminf(fmaxf(d, -delta), delta) / (float)m;
         }
     }
+    __align__(16) __nv_bfloat16 row[MLP_OUT_PAD];
+#pragma unroll
     for (int j = 0; j < MLP_OUT_PAD; ++j) {
-        const __nv_bfloat16 v = __float2bfloat16_rn(j == a ? g : (j == b ? -g : 0.0f));
-        dY[(size_t)r * MLP_OUT_PAD + j] = v;
-        dYt[(size_t)j * m_pad + r] = v;
+        row[j] = __float2bfloat16_rn(j == a ? g : (j == b ? -g : 0.0f));
+        dYt[(size_t)j * m_pad + r] = row[j];
     }
+#pragma unroll
+    for (int j = 0; j < MLP_OUT_PAD; j += 8) *(uint4*)(dY + (size_t)r * MLP_OUT_PAD + j) = *(const uint4*)(row + j);
     // warp sum in fixed order, one atomic per warp
     for (int o = 16; o; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)l / (double)m);
 }
 
-// out[j] = sum over k < m of G[j][k] (BF16 rows), one warp per j, fixed order
-__global__ void k_rowsum_bf16(int rows, int m, int ld, const __nv_bfloat16* __restrict__ G, float* __restrict__ out) {
-    const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (j >= rows) return;
+// out[j] = sum over k < m of G[j][k] (BF16 rows) for the rows of up to three matrices (the
+// bias gradients), one CTA per row: 256 threads stage 4096 columns at a time, then the
+// first warp's lane l adds k = l, l + 32, .. and the lanes are folded, a fixed order.  (A
+// warp reading its 2-byte entries from global memory: 11 us for 256 rows of 8192.)
+constexpr int RS_COLS = 4096;
+__global__ void __launch_bounds__(256) k_rowsum_bf16(RowSums rs) {
+    __shared__ __align__(16) __nv_bfloat16 s_row[RS_COLS];
+    int j = blockIdx.x, w = 0;
+    while (j >= rs.rows[w]) j -= rs.rows[w++];
+    const __nv_bfloat16* G = rs.g[w] + (size_t)j * rs.m;
+    const int tid = threadIdx.x;
     float s = 0.0f;
-    for (int k = lane; k < m; k += 32) s += __bfloat162float(G[(size_t)j * ld + k]);
+    for (int k0 = 0; k0 < rs.m; k0 += RS_COLS) {
+        const int n = min(RS_COLS, rs.m - k0);  // a multiple of 128: rows are padded to the GEMM tile
+        for (int i = tid * 8; i < n; i += 256 * 8) *(uint4*)(s_row + i) = *(const uint4*)(G + k0 + i);
+        __syncthreads();
+        if (tid < 32) {
+#pragma unroll 8
+            for (int k = tid; k < n; k += 32) s += __bfloat162float(s_row[k]);
+        }
+        __syncthreads();
+    }
+    if (tid >= 32) return;
     for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) out[j] = s;
+    if (tid == 0) rs.out[w][j] = s;
 }
 
-// out[i] = sum over s < n_part of part[s * stride + i], fixed order
-__global__ void k_reduce_partials(int n, int n_part, long long stride, const float* __restrict__ part,
-                                  float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.0f;
-    for (int p = 0; p < n_part; ++p) s += part[(size_t)p * stride + i];
-    out[i] = s;
+// The weight gradients from their split-K partials (summed slice after slice) into g
+// (whose bias entries are there already), and with ADAM the update (Kingma & Ba 2015) of
+// the FP32 master parameters and of their BF16 copies: row-major, transposed and in
+// fragment order.  One thread per parameter (three reductions, the update and the packing
+// took five launches).
+__device__ __forceinline__ void store_frag(uint4* f, int K, int n, int k, __nv_bfloat16 v) {
+    const int g = n & 7, hi = n >> 3 & 1, c = k & 7, half = k >> 3 & 1;
+    ((__nv_bfloat16*)&f[frag_index(n >> 4, k >> 4, g * 4 + (c >> 1), K)])[(half * 2 + hi) * 2 + (c & 1)] = v;
 }
-
-// Adam (Kingma & Ba 2015) on the flat FP32 parameter vector
-__global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
-                       float* __restrict__ m2, float lr, float b1, float b2, float eps, float bc1, float bc2) {
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_update(MlpPartials part, float* __restrict__ w, float* __restrict__ g,
+                                                float* __restrict__ m1, float* __restrict__ m2, float lr, float b1,
+                                                float b2, float eps, float bc1, float bc2, MlpBf16 o) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
+    if (i >= MLP_N_PARAMS) return;
+    const int l = i < MLP_OFF_B1 ? 0 : i >= MLP_OFF_W2 && i < MLP_OFF_B2 ? 1 : i >= MLP_OFF_W3 && i < MLP_OFF_B3 ? 2 : -1;
+    const int t = l == 0 ? i - MLP_OFF_W1 : l == 1 ? i - MLP_OFF_W2 : i - MLP_OFF_W3;
+    float gi;
+    if (l >= 0) {
+        const float* p = part.p[l] + t;
+        const size_t stride = l == 0 ? MLP_H * MLP_K1 : l == 1 ? MLP_H * MLP_H : MLP_OUT_PAD * MLP_H;
+        gi = 0.0f;
+#pragma unroll 8
+        for (int q = 0; q < part.slices; ++q) gi += p[q * stride];
+        g[i] = gi;
+    } else {
+        gi = g[i];
+    }
+    if (!ADAM) return;
     const float a = b1 * m1[i] + (1.0f - b1) * gi;
     const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
     m1[i] = a;
     m2[i] = b;
-    w[i] -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+    float x = w[i];
+    x -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+    w[i] = x;
+    const __nv_bfloat16 v = __float2bfloat16_rn(x);
+    if (l == 0) {
+        o.w1[t] = v;
+        store_frag(o.f1, MLP_K1, t / MLP_K1, t % MLP_K1, v);
+    } else if (l == 1) {
+        const int n = t / MLP_H, k = t % MLP_H;
+        o.w2[t] = v;
+        o.w2t[(size_t)k * MLP_H + n] = v;
+        store_frag(o.f2, MLP_H, n, k, v);
+    } else if (l == 2) {
+        const int n = t / MLP_H, k = t % MLP_H;
+        o.w3[t] = v;
+        o.w3t[(size_t)k * MLP_OUT_PAD + n] = v;
+        store_frag(o.f3, MLP_H, n, k, v);
+    }
 }
 
 // 16-byte fragment-order element (mt, s, lane) of W [N][K] at w (FP32 master copy)
@@ -475,12 +551,15 @@ __global__ void k_pack_weights(const float* __restrict__ p, MlpBf16 o) {
 // output, target.  A mutation is a query without amino acid (MLP_NO_AA) whose
 // energy change is predicted as y[new] - y[old]; a rotamer move queries with its
 // amino acid and is predicted by y[20 + rotamer].
-__global__ void k_gather_tuples(int m, const int* __restrict__ idx, const MlpTuple* __restrict__ tup,
+// The rows are drawn with the Philox generator: row r takes tuple
+// (u n_tuples) >> 32.
+__global__ void k_gather_tuples(int m, int n_tuples, uint64_t seed, uint32_t step, const MlpTuple* __restrict__ tup,
                                 float* __restrict__ ca, uint8_t* __restrict__ aa, int* __restrict__ ag,
                                 int* __restrict__ action, int* __restrict__ ref, float* __restrict__ target) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= m) return;
-    const MlpTuple t = tup[idx[r]];
+    const U4 u = philox((uint32_t)r, step, 0xB47Cu, 0u, (uint32_t)seed, (uint32_t)(seed >> 32));
+    const MlpTuple t = tup[(int)(((uint64_t)u.x * (uint32_t)n_tuples) >> 32)];
     const bool mut = t.action < N_AA;
     ca[3 * r] = t.x;
     ca[3 * r + 1] = t.y;
@@ -490,13 +569,6 @@ __global__ void k_gather_tuples(int m, const int* __restrict__ idx, const MlpTup
     action[r] = t.action;
     ref[r] = mut ? (int)t.aa : -1;
     target[r] = t.delta_e;
-}
-// minibatch indices drawn with the Philox generator: idx[r] = uniform in [0, n_tuples)
-__global__ void k_draw_batch(int m, int n_tuples, uint64_t seed, uint32_t step, int* __restrict__ idx) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= m) return;
-    const U4 u = philox((uint32_t)r, step, 0xB47Cu, 0u, (uint32_t)seed, (uint32_t)(seed >> 32));
-    idx[r] = (int)(((uint64_t)u.x * (uint32_t)n_tuples) >> 32);
 }
 
 // ---- launchers ----------------------------------------------------------------------
@@ -516,26 +588,24 @@ void launch_mlp_loss(cudaStream_t s, int m, int m_pad, const float* Y, const int
     if (m_pad > 0)
         k_mlp_loss<<<(m_pad + 255) / 256, 256, 0, s>>>(m, m_pad, Y, action, ref, target, delta, dY, dYt, loss);
 }
-void launch_rowsum_bf16(cudaStream_t s, int rows, int m, int ld, const __nv_bfloat16* G, float* out) {
-    if (rows > 0) k_rowsum_bf16<<<(rows + 7) / 8, 256, 0, s>>>(rows, m, ld, G, out);
+void launch_rowsum_bf16(cudaStream_t s, const RowSums& rs) {
+    const int rows = rs.rows[0] + rs.rows[1] + rs.rows[2];
+    if (rows > 0) k_rowsum_bf16<<<rows, 256, 0, s>>>(rs);
 }
-void launch_reduce_partials(cudaStream_t s, int n, int n_part, long long stride, const float* part, float* out) {
-    if (n > 0) k_reduce_partials<<<(n + 255) / 256, 256, 0, s>>>(n, n_part, stride, part, out);
-}
-void launch_adam(cudaStream_t s, int n, float* w, const float* g, float* m1, float* m2, float lr, float b1, float b2,
-                 float eps, float bc1, float bc2) {
-    if (n > 0) k_adam<<<(n + 255) / 256, 256, 0, s>>>(n, w, g, m1, m2, lr, b1, b2, eps, bc1, bc2);
+void launch_update(cudaStream_t s, const MlpPartials& part, float* w, float* g, float* m1, float* m2, float lr,
+                   float b1, float b2, float eps, float bc1, float bc2, const MlpBf16& o, bool adam) {
+    const int n = (MLP_N_PARAMS + 255) / 256;
+    if (adam) k_update<true><<<n, 256, 0, s>>>(part, w, g, m1, m2, lr, b1, b2, eps, bc1, bc2, o);
+    else k_update<false><<<n, 256, 0, s>>>(part, w, g, m1, m2, lr, b1, b2, eps, bc1, bc2, o);
 }
 void launch_pack_weights(cudaStream_t s, const float* p, const MlpBf16& o) {
     const int n = std::max(MLP_H * MLP_K1, std::max(MLP_H * MLP_H, MLP_OUT_PAD * MLP_H));
     k_pack_weights<<<(n + 255) / 256, 256, 0, s>>>(p, o);
 }
-void launch_gather_tuples(cudaStream_t s, int m, const int* idx, const MlpTuple* tup, float* ca, uint8_t* aa, int* ag,
-                          int* action, int* ref, float* target) {
-    if (m > 0) k_gather_tuples<<<(m + 255) / 256, 256, 0, s>>>(m, idx, tup, ca, aa, ag, action, ref, target);
-}
-void launch_draw_batch(cudaStream_t s, int m, int n_tuples, uint64_t seed, uint32_t step, int* idx) {
-    if (m > 0) k_draw_batch<<<(m + 255) / 256, 256, 0, s>>>(m, n_tuples, seed, step, idx);
+void launch_gather_tuples(cudaStream_t s, int m, int n_tuples, uint64_t seed, uint32_t step, const MlpTuple* tup,
+                          float* ca, uint8_t* aa, int* ag, int* action, int* ref, float* target) {
+    if (m > 0)
+        k_gather_tuples<<<(m + 255) / 256, 256, 0, s>>>(m, n_tuples, seed, step, tup, ca, aa, ag, action, ref, target);
 }
 
 }  // namespace binder
