@@ -66,6 +66,16 @@ constexpr int AN_WARPS = 8;
 constexpr int AN_THREADS = AN_WARPS * 32;
 constexpr int STAGE_CAP = 64;                        // staged in-cutoff terms per warp (ACC = float)
 constexpr int HIT_CAP = 96;                          // in-cutoff entries a warp's scan holds (ACC = double)
+// Skins of the residues' lists: a residue's first, and the most a residue that outruns its
+// list gets (twice the last).  600 steps of 64 candidates and the rest of run_allatom: 12.35
+// ms with at most 4 A, 12.8 with 5, 12.6 with 3 (longer lists cost every step, shorter ones
+// more builds).  Fv chains take wide ones from the start (7.5 ms for 32 pairs x 20 steps
+// with 4 and 8 A, 7.9 with 2 and 5): their backbone moves swing 60 residues at a time, and
+// an energy inside the skin costs a fifth of a scan.
+template <bool FV>
+constexpr float AN_SKIN = FV ? 4.0f : 2.0f;
+template <bool FV>
+constexpr float AN_SKIN_MAX = FV ? 8.0f : 4.0f;
 constexpr int EL = 8;                                // lanes per Calpha energy (ACC = double)
 constexpr int MASK_WORDS = ANNEAL_MAX_RES / 32;      // residue bit masks of a candidate
 constexpr int AN_IN = 32;                            // in-cutoff entries of the force a residue holds per round
@@ -127,7 +137,8 @@ struct AnSmem {
     float mbias[LRN ? MLP_BIASES : 1];        // the network's biases b1 | b2 | b3
     __align__(16) unsigned char tile[LRN ? MT_BYTES : 16];  // the network tile
     __align__(16) uint16_t cglist[RT * CG_LIST_MAX];  // Verlet lists of the Langevin force
-    uint8_t ptaa[RT];
+    uint8_t ptaa[RT], dirty[RT];              // dirty: the list was built in this launch
+    unsigned char cysid[W][RT];               // Cys residues of a warp's disulfide sum
 };
 // Entries of each staged x / y / z array: room for the pad, a multiple of 4.
 __host__ __device__ inline int anneal_xyz_len(int G) { return G > 0 ? (G + 4) & ~3 : 0; }
@@ -348,47 +359,52 @@ __device__ __noinline__ double warp_scan_energy(F3 ca, int aa, float2* hits) {
 }
 
 // disulfide_energy (allatom.rs:155-180) over the SG atoms (topology atom 5) of the
-// residues in the bit mask cysw, pairs in residue order, by one warp: lanes test the
-// partners of one Cys at a time and the in-range terms are subtracted in order (the
-// result is on every lane).  sweep: residues take their slots as the sweep sees them
-// (their proposal when accepted, their rejection rebuild when rejected, else the state)
+// residues in the bit mask cysw, pairs in residue order, by one warp: the lanes list the
+// Cys residues, test 32 pairs at a time and the in-range terms are subtracted in order
+// (the result is on every lane).  sweep: residues take their slots as the sweep sees
+// them (their proposal when accepted, their rejection rebuild when rejected, else the state)
 // and residue `sub` (>= 0) its proposal; else every residue is read from the state.
 template <class L, class ACC>
 __device__ __noinline__ ACC warp_disulfide(bool sweep, int words, int sub) {
     L& S = an_smem<L>();
-    const unsigned* cys = S.cysw;
     const int lane = threadIdx.x & 31;
-    int k = 0;
-    for (int w = 0; w < words; ++w) k += __popc(cys[w]);
     ACC e = 0;
+    int k = 0;
+    unsigned char* ids = S.cysid[threadIdx.x >> 5];
+    __syncwarp();
+#pragma unroll 1
+    for (int w = 0; w < words; ++w) {
+        const unsigned m = S.cysw[w];
+        if (m >> lane & 1u) ids[k + __popc(m & ((1u << lane) - 1u))] = (unsigned char)(w * 32 + lane);
+        k += __popc(m);
+    }
     if (k < 2) return e;
+    __syncwarp();
     auto sg = [&](int j) -> float4 {
         const int s = sweep ? (j == sub ? (int)SEL_PROP : S.sel[j] & 3) : (int)SEL_KEEP;
         return (s == SEL_PROP ? S.prop : s == SEL_REJ ? S.rej : S.pos)[j * SLOT_STRIDE + 5];
     };
-    for (int wi = 0; wi < words; ++wi)
-        for (unsigned mi = cys[wi]; mi; mi &= mi - 1) {
-            const int i = wi * 32 + __ffs(mi) - 1;
-            const float4 pi = sg(i);
-            for (int wj = wi; wj < words; ++wj) {
-                const unsigned mj = cys[wj];
-                if (!mj) continue;
-                const int j = wj * 32 + lane;
-                float t = 0.0f;
-                bool in = false;
-                if (j > i && (mj >> lane & 1u)) {
-                    const float4 pj = sg(j);
-                    const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
-                    in = !(d > 4.0f);
-                    if (in) {
-                        const float z = xdiv(xsub(d, 2.05f), 0.4f);
-                        t = xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z)));
-                    }
-                }
-                for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1)
-                    e -= (ACC)__shfl_sync(0xffffffffu, t, __ffs(m) - 1);
+    int i = 0, left = lane;  // this lane's pair: (i, i + 1 + left)
+    const int pairs = k * (k - 1) / 2;
+#pragma unroll 1
+    for (int p0 = 0; p0 < pairs; p0 += 32, left += 32) {
+        float t = 0.0f;
+        bool in = false;
+        if (p0 + lane < pairs) {
+            while (left >= k - 1 - i) {
+                left -= k - 1 - i;
+                ++i;
+            }
+            const float4 pi = sg(ids[i]), pj = sg(ids[i + 1 + left]);
+            const float d = xsqrt(xdist2(xsub(pi.x, pj.x), xsub(pi.y, pj.y), xsub(pi.z, pj.z)));
+            in = !(d > 4.0f);
+            if (in) {
+                const float z = xdiv(xsub(d, 2.05f), 0.4f);
+                t = xmul(4.0f, mc_exp(xmul(xmul(-0.5f, z), z)));
             }
         }
+        for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1) e -= (ACC)__shfl_sync(0xffffffffu, t, __ffs(m) - 1);
+    }
     return e;
 }
 
@@ -830,7 +846,9 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
     if (n <= 0 || n > L::RT) return;
     const int words = (n + 31) >> 5;  // of a residue bit mask
     const uint32_t cid = st.cand_id[c];
-    if (tid == 0) S.ag = ags[st.cand_ag[c]];
+    const int c_ag = st.cand_ag[c];
+    const int epoch = st.ag_epoch && st.cg_meta && st.cg_list && st.cg_centre ? *st.ag_epoch : -2;
+    if (tid == 0) S.ag = ags[c_ag];
     __syncthreads();
     const AgView& A = S.ag;
     const int nag = A.n_res;
@@ -906,8 +924,13 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
         S.chi[r] = chi;
         S.trig[2 * r] = st.res_trig[2 * (r0 + r)];
         S.trig[2 * r + 1] = st.res_trig[2 * (r0 + r) + 1];
-        S.cgnl[r] = -1;
-        S.cgcentre[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // the residue's list of an earlier launch, if it was built for this antigen set and antigen
+        const int4 meta = epoch >= 0 ? st.cg_meta[r0 + r] : make_int4(-1, -1, -1, -1);
+        const bool kept = epoch >= 0 && meta.z == epoch && meta.y == c_ag && meta.x >= 0 && meta.x <= CG_LIST_MAX &&
+                          nag <= 65536;
+        S.cgnl[r] = kept ? meta.x : -1;
+        S.cgcentre[r] = kept ? st.cg_centre[r0 + r] : make_float4(0.f, 0.f, 0.f, 0.f);
+        S.dirty[r] = 0;
         if (EXT) {
             // rotamer index of the state: the library entry whose chi it holds, else -1
             int k = -1;
@@ -919,6 +942,10 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
         }
     }
     __syncthreads();
+    for (int r = warp; r < n; r += W) {
+        const int nl = S.cgnl[r];
+        for (int j = lane; j < nl; j += 32) S.cglist[r * CG_LIST_MAX + j] = (uint16_t)st.cg_list[(size_t)(r0 + r) * CG_LIST_MAX + j];
+    }
     if (tid == 0 && cells_staged) {  // the list builds read the staged copies through the view
         S.ag.ca_pq = s_cgq;
         S.ag.ca_prm = s_cgp;
@@ -1009,14 +1036,20 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
                         const int rq = __shfl_sync(0xffffffffu, rr, q);
                         const F3 cq = f3(S.pos[(size_t)rq * SLOT_STRIDE + 1]);
                         const int nq = S.cgnl[rq];
-                        const float sq = nq < 0 ? CG_SKIN : fminf(2.0f * S.cgcentre[rq].w, CG_SKIN_MAX);
+                        float sq = nq < 0 ? AN_SKIN<FV> : fminf(2.0f * S.cgcentre[rq].w, AN_SKIN_MAX<FV>);
                         __syncwarp();
-                        const int len = nag <= 65536 ? build_cg_list_warp<uint16_t>(A.ca_grid, A.ca_pq, cq, lane,
-                                                                                     S.cglist + (size_t)rq * CG_LIST_MAX, sq)
-                                                     : CG_LIST_MAX + 1;
+                        int len = CG_LIST_MAX + 1;
+                        for (;;) {  // one that overflows the list (deep in the antigen) is built again with 1 A
+                            if (nag <= 65536)
+                                len = build_cg_list_warp<uint16_t>(A.ca_grid, A.ca_pq, cq, lane,
+                                                                   S.cglist + (size_t)rq * CG_LIST_MAX, sq);
+                            if (len <= CG_LIST_MAX || sq <= 1.0f) break;
+                            sq = 1.0f;
+                        }
                         if (lane == q) {
                             S.cgcentre[rq] = make_float4(cq.x, cq.y, cq.z, sq);
                             S.cgnl[rq] = len;
+                            S.dirty[rq] = 1;
                         }
                     }
                     __syncwarp();
@@ -1477,6 +1510,16 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
         st.res_chi[r0 + r] = S.chi[r];
         st.res_trig[2 * (r0 + r)] = S.trig[2 * r];
         st.res_trig[2 * (r0 + r) + 1] = S.trig[2 * r + 1];
+    }
+    for (int r = warp; epoch >= 0 && r < n; r += W) {  // lists built here, for the next launch
+        if (!S.dirty[r]) continue;
+        const int nl = S.cgnl[r];
+        for (int j = lane; j < min(nl, CG_LIST_MAX); j += 32)
+            st.cg_list[(size_t)(r0 + r) * CG_LIST_MAX + j] = S.cglist[r * CG_LIST_MAX + j];
+        if (lane == 0) {
+            st.cg_centre[r0 + r] = S.cgcentre[r];
+            st.cg_meta[r0 + r] = make_int4(nl, c_ag, epoch, 0);
+        }
     }
     if (stats && (n_mc || n_bb)) {  // the decisions are spread over the lanes of warp 0
         atomicAdd((unsigned long long*)&stats[4 * c], (unsigned long long)n_mc);

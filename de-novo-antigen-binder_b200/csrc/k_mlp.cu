@@ -193,8 +193,8 @@ __device__ __forceinline__ float sigmoid_fast(float z) { return rcp_approx(1.0f 
 // These GEMMs are small (8192 x 256 x 192 and the like), so what bounds them is one CTA's
 // chain of loads, MMAs and epilogue: 64-column tiles give 4 times the CTAs and a quarter of
 // the epilogue each, four stages keep three chunks of K in flight (training step of 8192
-// rows: forward and data-gradient GEMMs 27 us each, now GEMM_A; weight gradients 43 + 43 +
-// 25 us, now GEMM_B in one launch).  Every output sums over K in the same order as before.
+// rows: forward and data-gradient GEMMs 27 us each, now 18; weight gradients 43 + 43 +
+// 25 us, now 34 in one launch).  Every output sums over K in the same order as before.
 constexpr int G_M = 128, G_K = 64, G_N = 64, G_THREADS = 256, G_STAGES = 4;
 constexpr int G_STAGE_A = G_M * G_K * 2;                       // 16 KB
 constexpr int G_STAGE = G_STAGE_A + G_N * G_K * 2;
