@@ -1518,7 +1518,8 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
             st.cg_list[(size_t)(r0 + r) * CG_LIST_MAX + j] = S.cglist[r * CG_LIST_MAX + j];
         if (lane == 0) {
             st.cg_centre[r0 + r] = S.cgcentre[r];
-            st.cg_meta[r0 + r] = make_int4(nl, c_ag, epoch, 0);
+            // the gradient steps take a kept list's skin for at least CG_SKIN: a narrower one stays here
+            st.cg_meta[r0 + r] = make_int4(S.cgcentre[r].w >= CG_SKIN ? nl : -1, c_ag, epoch, 0);
         }
     }
     if (stats && (n_mc || n_bb)) {  // the decisions are spread over the lanes of warp 0
