@@ -95,7 +95,7 @@ struct Antigen {
     DBuf<float> x, y, z, q, rmh, eps;
     DBuf<uint8_t> hyd, type;
     GridBuf grid;
-    DBuf<float4> pq, prm;
+    DBuf<float4> pq, prm, box;
     DBuf<float> cax, cay, caz;
     DBuf<uint8_t> caa;
     GridBuf ca_grid;
@@ -469,11 +469,13 @@ int build_antigen_atoms(binder_ctx* ctx, Antigen& A, const float* x, const float
     if ((s = build_grid(ctx, A.x.p, A.y.p, A.z.p, (int)n, ctx->params.score_cell, A.grid))) return s;
     CK(A.pq.ensure(n), "antigen alloc");
     CK(A.prm.ensure(n), "antigen alloc");
+    CK(A.box.ensure(2 * ((n + 31) / 32)), "antigen alloc");
     launch_gather_atoms(ctx->stream, A.grid.sorted_idx.p, (int)n, A.x.p, A.y.p, A.z.p, A.q.p, A.rmh.p, A.eps.p,
-                        A.hyd.p, type ? A.type.p : nullptr, A.pq.p, A.prm.p);
+                        A.hyd.p, type ? A.type.p : nullptr, A.pq.p, A.prm.p, A.box.p);
     if (n > 0) LAUNCHED("gather_atoms");
     A.view.pq = A.pq.p;
     A.view.prm = A.prm.p;
+    A.view.box = A.box.p;
     A.view.grid = A.grid.view;
     A.view.n_atoms = (int)n;
     return BINDER_OK;
@@ -1467,7 +1469,8 @@ int enqueue_diffuse(binder_ctx* ctx, int n_steps, uint32_t step0, int with_noise
 StateScoreScratch score_scratch(binder_ctx* ctx) {
     State& S = ctx->st;
     const bool cell = S.order_valid && ctx->cfg.score_order == 0;
-    return StateScoreScratch{cell ? S.order.p : nullptr, S.queue.p, S.res_e.p, S.res_abs.p};
+    return StateScoreScratch{cell ? S.order.p : nullptr, S.queue.p, S.res_e.p, S.res_abs.p,
+                             cell ? nullptr : S.cg_bal.p};
 }
 
 int persistent_ctas(binder_ctx* ctx) { return ctx->num_sms * ctx->cfg.score_ctas_per_sm; }

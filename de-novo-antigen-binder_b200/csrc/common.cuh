@@ -77,6 +77,11 @@ __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
 __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -84,6 +89,21 @@ __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
 }
 __device__ __forceinline__ float f2_lo(uint64_t v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float f2_hi(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+// The same in packed arithmetic: a product rounded on its own is fma(d, d, -0) with a -0
+// that the code generator cannot see (it comes from memory), which no add can be fused into.
+__device__ __forceinline__ void f2_dist2(uint64_t dx, uint64_t dy, uint64_t dz, uint64_t neg0, float& lo, float& hi) {
+    const uint64_t d = f2_add(f2_add(f2_fma(dx, dx, neg0), f2_fma(dy, dy, neg0)), f2_fma(dz, dz, neg0));
+    lo = f2_lo(d);
+    hi = f2_hi(d);
+}
+// 1 / sqrt(x) of a normal x: the instruction of rsqrtf without the scaling around it that
+// only denormal x needs (three operations each).  Every r^2 whose result is used is at
+// least MIN_R_SQ.
+__device__ __forceinline__ float rsqrt_normal(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 // the reference's r^2 of both elements of packed differences (scalar, never fused)
 __device__ __forceinline__ void f2_dist2(uint64_t dx, uint64_t dy, uint64_t dz, float& lo, float& hi) {
     lo = xdist2(f2_lo(dx), f2_lo(dy), f2_lo(dz));
@@ -153,6 +173,7 @@ struct AgView {
     // all atoms, sorted by score-grid cell (ascending original index within a cell)
     const float4* pq;   // x, y, z, q*sqrt(332)
     const float4* prm;  // r_min_half, sqrt(epsilon), hydrophobic (0/1), atom type
+    const float4* box;  // lowest, highest coordinates of each 32 consecutive atoms
     GridView grid;
     int n_atoms;
     // Calpha cloud (run_allatom ag_ca, diffusion.rs:994-1002) sorted by CA-grid cell

@@ -99,13 +99,31 @@ __global__ void k_gather_atoms(const int* __restrict__ sorted_idx, int n, const 
                                const float* __restrict__ y, const float* __restrict__ z, const float* __restrict__ q,
                                const float* __restrict__ rmh, const float* __restrict__ eps,
                                const uint8_t* __restrict__ hyd, const uint8_t* __restrict__ type,
-                               float4* __restrict__ pq, float4* __restrict__ prm) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    int i = sorted_idx[j];
-    const float sqrt_k = 18.220867f;  // sqrt(332) rounded to f32
-    pq[j] = make_float4(x[i], y[i], z[i], q[i] * sqrt_k);
-    prm[j] = make_float4(rmh[i], sqrtf(eps[i]), hyd[i] == 1 ? 1.0f : 0.0f, type ? (float)type[i] : 0.0f);
+                               float4* __restrict__ pq, float4* __restrict__ prm, float4* __restrict__ box) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const float inf = __int_as_float(0x7f800000);
+    float3 lo = make_float3(inf, inf, inf), hi = make_float3(-inf, -inf, -inf);
+    if (j < n) {
+        const int i = sorted_idx[j];
+        const float sqrt_k = 18.220867f;  // sqrt(332) rounded to f32
+        pq[j] = make_float4(x[i], y[i], z[i], q[i] * sqrt_k);
+        prm[j] = make_float4(rmh[i], sqrtf(eps[i]), hyd[i] == 1 ? 1.0f : 0.0f, type ? (float)type[i] : 0.0f);
+        lo = hi = make_float3(x[i], y[i], z[i]);
+    }
+    // the box of the warp's 32 atoms (AgView::box)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
+        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
+        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
+        hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
+        hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
+        hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
+    }
+    if ((j & 31) == 0 && j < n) {
+        box[2 * (j >> 5)] = make_float4(lo.x, lo.y, lo.z, 0.f);
+        box[2 * (j >> 5) + 1] = make_float4(hi.x, hi.y, hi.z, 0.f);
+    }
 }
 
 // Residue-level Calpha records (ResidueCloud::push, atom.rs:221-231) in grid order.
@@ -181,8 +199,8 @@ void launch_stable_scatter(cudaStream_t s, const int4* cells, int n, int* cursor
 }
 void launch_gather_atoms(cudaStream_t s, const int* sorted_idx, int n, const float* x, const float* y,
                          const float* z, const float* q, const float* rmh, const float* eps, const uint8_t* hyd,
-                         const uint8_t* type, float4* pq, float4* prm) {
-    if (n > 0) k_gather_atoms<<<nblk(n, 256), 256, 0, s>>>(sorted_idx, n, x, y, z, q, rmh, eps, hyd, type, pq, prm);
+                         const uint8_t* type, float4* pq, float4* prm, float4* box) {
+    if (n > 0) k_gather_atoms<<<nblk(n, 256), 256, 0, s>>>(sorted_idx, n, x, y, z, q, rmh, eps, hyd, type, pq, prm, box);
 }
 void launch_gather_ca(cudaStream_t s, const int* sorted_idx, int n, const float* x, const float* y, const float* z,
                       const uint8_t* aa, const float4* res_tab, float inv, float4* pq, float4* prm, int4* cells) {

@@ -227,9 +227,9 @@ __global__ void __launch_bounds__(MAT_WARPS * 32) k_mature(StateView st, const A
             const int t = warp, aa = s_aa[t], na = c_topo_n[aa];
             if (lane < na) {
                 const float4 p = s_pos[t][lane];
-                const float4 m = c_slot_prm[aa][lane];
+                const float4 m = g_slot_prm[aa][lane];
                 g.pos[lane] = make_float4(p.x, p.y, p.z, m.x);
-                g.prm[lane] = make_float4(m.y, m.z, m.w, (float)c_slot_type[aa][lane]);
+                g.prm[lane] = make_float4(m.y, m.z, m.w, (float)g_slot_type[aa][lane]);
                 group_xyz(g, lane, na, p.x, p.y, p.z);
                 group_prm(g, lane, na, m.x, m.y, m.z, m.w);
             } else {
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(FVP_WARPS * 32) k_fv_pair(StateView st, double
     const int l0 = st.cand_res_off[2 * i + 1], nl = st.cand_res_off[2 * i + 2] - l0;
     __shared__ float4 s_c[2][FVP_MAX_RES];  // residue centroid, radius
     __shared__ unsigned char s_aa[2][FVP_MAX_RES];
-    __shared__ float4 s_prm[N_AA * SLOT_STRIDE];  // c_slot_prm, type, EEF1 parameters
+    __shared__ float4 s_prm[N_AA * SLOT_STRIDE];  // g_slot_prm, type, EEF1 parameters
     __shared__ unsigned char s_type[N_AA * SLOT_STRIDE];
     __shared__ float4 s_eef[16];
     __shared__ float s_rl[16];
@@ -315,8 +315,8 @@ __global__ void __launch_bounds__(FVP_WARPS * 32) k_fv_pair(StateView st, double
         return;
     }
     for (int t = tid; t < N_AA * SLOT_STRIDE; t += blockDim.x) {
-        s_prm[t] = (&c_slot_prm[0][0])[t];
-        s_type[t] = (unsigned char)(&c_slot_type[0][0])[t];
+        s_prm[t] = (&g_slot_prm[0][0])[t];
+        s_type[t] = (unsigned char)(&g_slot_type[0][0])[t];
     }
     if (tid < 16) {
         s_eef[tid] = c_eef1[tid];
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(VAL_THREADS) k_validate(StateView st, int* __r
             const int aa = st.res_aa[r0 + i], na = s_topo_n[aa];
             if ((int)threadIdx.x < na) {
                 const float4 p = st.res_pos[(size_t)(r0 + i) * SLOT_STRIDE + threadIdx.x];
-                at[base + threadIdx.x] = make_float4(p.x, p.y, p.z, c_slot_prm[aa][threadIdx.x].y);
+                at[base + threadIdx.x] = make_float4(p.x, p.y, p.z, g_slot_prm[aa][threadIdx.x].y);
                 res[base + threadIdx.x] = i;
             }
             base += na;

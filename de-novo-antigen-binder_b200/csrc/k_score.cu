@@ -23,36 +23,38 @@ cudaError_t score_init_tables() { return score_tables_init(); }
 
 struct SrcStateG {
     StateView st;
-    __device__ int ag(int c) const { return st.cand_ag[c]; }
-    __device__ int n_groups(int c) const { return st.cand_res_off[c + 1] - st.cand_res_off[c]; }
-    __device__ int load(int c, int g, int lane, GroupSmem& s, bool& bad) const {
-        const int r = st.cand_res_off[c] + g;
+    // residue r: its atoms into the group (the loads of its amino acid and positions are issued
+    // together: the slots beyond its atoms are read and dropped)
+    __device__ int load(int r, int lane, GroupSmem& s, bool& bad) const {
         const int aa = st.res_aa[r];
+        const float4 p = lane < SLOTS ? st.res_pos[(size_t)r * SLOT_STRIDE + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
         const int n = c_topo_n[aa];
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
         if (lane < n) {
-            const float4 p = st.res_pos[(size_t)r * SLOT_STRIDE + lane];
-            const float4 m = c_slot_prm[aa][lane];
+            m = g_slot_prm[aa][lane];
             bad = !finite3(p.x, p.y, p.z);
             s.pos[lane] = make_float4(p.x, p.y, p.z, m.x);
-            s.prm[lane] = make_float4(m.y, m.z, m.w, (float)c_slot_type[aa][lane]);
-            group_xyz(s, lane, n, p.x, p.y, p.z);
-            group_prm(s, lane, n, m.x, m.y, m.z, m.w);
-        } else {
-            group_xyz(s, lane, n, 0.f, 0.f, 0.f);
-            group_prm(s, lane, n, 0.f, 0.f, 0.f, 0.f);
+            s.prm[lane] = make_float4(m.y, m.z, m.w, (float)g_slot_type[aa][lane]);
         }
+        group_xyz(s, lane, n, p.x, p.y, p.z);
+        group_prm(s, lane, n, m.x, m.y, m.z, m.w);
         return n;
     }
 };
 
 // Resident state: persistent teams of TEAM warps take residues from a work queue (an
-// atomic counter; residues in index order, or in Calpha-cell order so that neighbouring
-// warps share antigen atoms in L1 -- whichever the autotuner timed faster) and
-// write one FP64 energy per residue; k_sum_residues adds a candidate's residues in
-// index order.  No CTA barrier: teams never wait for each other.
+// atomic counter) and write one FP64 energy per residue; k_sum_residues adds a candidate's
+// residues in index order.  No CTA barrier: teams never wait for each other.  The residues
+// come in Calpha-cell order, so that neighbouring warps share antigen atoms in L1, or by the
+// gradient steps' work bands, heaviest first, or in index order while those bands are not
+// filled -- cell order or not as the autotuner timed it.  A warp evaluates only four or five
+// residues of about 11 us each (20480 residues, 4736 warps), so the launch's end is decided by
+// what comes last: heaviest first 61 -> 57 us, and claiming a residue ahead (to hide the
+// counter's latency) cost more than it hid (60 us).
 template <int NW, bool KAHAN, bool FULL, bool ABS, bool COUNT, int TEAM>
 __global__ void __launch_bounds__(NW * 32) k_score_residues(StateView st, const AgView* __restrict__ ags,
-                                                             const int* __restrict__ order, int* __restrict__ queue,
+                                                             const int* __restrict__ order, const int* __restrict__ bal,
+                                                             int* __restrict__ queue,
                                                              double* __restrict__ res_e, double* __restrict__ res_abs,
                                                              long long* __restrict__ pair_count,
                                                              uint32_t* __restrict__ err) {
@@ -69,6 +71,18 @@ __global__ void __launch_bounds__(NW * 32) k_score_residues(StateView st, const 
     SrcStateG src{st};
     auto sync = [team] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(TEAM * 32) : "memory"); };
     int my_pairs = 0;
+    // lane b: residues in the work bands 0 .. b; the buckets are taken when they hold every residue
+    int band_end = 0, parity = 0;
+    if (bal) {
+        parity = __ldg(&bal[0]) & 1;
+        band_end = lane < CG_BAL_BINS ? __ldg(&bal[2 + CG_BAL_BINS * parity + lane]) : 0;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, band_end, d);
+            if (lane >= d) band_end += v;
+        }
+        if (__shfl_sync(0xffffffffu, band_end, 31) != st.total_res) bal = nullptr;
+    }
     for (;;) {
         int gi = 0;
         if (lane == 0 && rank == 0) gi = atomicAdd(queue, 1);
@@ -81,21 +95,26 @@ __global__ void __launch_bounds__(NW * 32) k_score_residues(StateView st, const 
             gi = __shfl_sync(0xffffffffu, gi, 0);
         }
         if (gi >= st.total_res) break;
-        const int r = order ? order[gi] : gi;
-        const int c = st.res_cand[r];
+        int r = gi;
+        if (order) {
+            r = order[gi];
+        } else if (bal) {
+            const int b = __popc(__ballot_sync(0xffffffffu, lane < CG_BAL_BINS && band_end <= gi));
+            const int below = __shfl_sync(0xffffffffu, band_end, max(b - 1, 0));
+            r = __ldg(bal + CG_BAL_HEADER + (size_t)(parity * CG_BAL_BINS + b) * st.total_res + gi - (b ? below : 0));
+        }
+        const AgView* Ap = &ags[st.cand_ag[st.res_cand[r]]];
         bool bad = false;
-        const int n = src.load(c, r - st.cand_res_off[c], lane, s, bad);
+        const int n = src.load(r, lane, s, bad);
         Acc acc = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0};
         if (__any_sync(0xffffffffu, bad)) {
             if (lane == 0) atomicOr(err, ERRF_NAN);
         } else if (n > 0) {
             __syncwarp();
             if constexpr (TEAM > 1)
-                score_group_team<KAHAN, TEAM>(&ags[st.cand_ag[c]], s, &gfs[warp], n, lane, lt, acc, rank, teams[team],
-                                              sync);
+                score_group_team<KAHAN, TEAM>(Ap, s, &gfs[warp], n, lane, lt, acc, rank, teams[team], sync);
             else
-                score_group<KAHAN, FULL, ABS, COUNT>(&ags[st.cand_ag[c]], s, FULL ? &gfs[warp] : nullptr, n, lane, lt,
-                                                     acc);
+                score_group<KAHAN, FULL, ABS, COUNT>(Ap, s, FULL ? &gfs[warp] : nullptr, n, lane, lt, acc);
         }
         __syncwarp();
         if (rank == 0) {
@@ -299,7 +318,7 @@ __global__ void __launch_bounds__(NW * 32) k_force_flat(FlatAtoms src, int n_can
                     const float4 apq = __ldg(&pq[t]);
                     const float4 aprm = __ldg(&prm[t]);
                     const float dx = b.x - apq.x, dy = b.y - apq.y, dz = b.z - apq.z;
-                    const float ir = rsqrtf(r2);
+                    const float ir = rsqrt_normal(r2);
                     const float ir2 = ir * ir;
                     const float R = b.rmh + aprm.x;
                     const float s2 = R * R * ir2;
@@ -625,7 +644,7 @@ static void score_residues_nw(cudaStream_t s, int g, const StateView& st, const 
     constexpr size_t team_bytes = NW / 4 * sizeof(TeamSmem);
 #define BINDER_R(K, FU, A, C, T)                                                                                 \
     k_score_residues<NW, K, FU, A, C, T><<<g, NW * 32, T > 1 ? team_bytes : 0, s>>>(                            \
-        st, ags, scr.order, scr.queue, count ? nullptr : scr.res_e, scr.res_abs, o.pairs, o.err)
+        st, ags, scr.order, scr.bal, scr.queue, count ? nullptr : scr.res_e, scr.res_abs, o.pairs, o.err)
     if (count) BINDER_R(true, false, false, true, 1);
     else if (full) {
         if constexpr (NW == NW_SCORE) {

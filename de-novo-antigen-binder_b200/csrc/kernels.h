@@ -47,7 +47,7 @@ void launch_exclusive_scan(cudaStream_t s, const int* counts, int n, int* out);
 void launch_stable_scatter(cudaStream_t s, const int4* cells, int n, int* cursor, int* sorted_idx);
 void launch_gather_atoms(cudaStream_t s, const int* sorted_idx, int n, const float* x, const float* y,
                          const float* z, const float* q, const float* rmh, const float* eps, const uint8_t* hyd,
-                         const uint8_t* type, float4* pq, float4* prm);
+                         const uint8_t* type, float4* pq, float4* prm, float4* box);
 void launch_gather_ca(cudaStream_t s, const int* sorted_idx, int n, const float* x, const float* y, const float* z,
                       const uint8_t* aa, const float4* res_tab, float inv, float4* pq, float4* prm, int4* cells);
 void launch_nb_count(cudaStream_t s, const GridView& g, const float* px, const float* py, const float* pz, int n_q,
@@ -76,6 +76,7 @@ struct StateScoreScratch {
     int* queue;        // work counter, queue[2] the done count (left zero by queue_retire)
     double* res_e;     // total_res
     double* res_abs;   // total_res (abs sums)
+    const int* bal = nullptr;  // residues by the gradient steps' work bands (cg_bal_*), heaviest first
 };
 // Survivor selection fused into the candidate sums of launch_score_state (k <= 64,
 // every segment at most 4096 candidates, listed in ascending candidate index;

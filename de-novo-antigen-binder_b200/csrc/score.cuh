@@ -14,8 +14,8 @@
 
 namespace binder {
 
-static __constant__ float4 c_slot_prm[N_AA][SLOT_STRIDE];  // q*sqrt(332), r_min_half, sqrt(eps), hydrophobic
-static __constant__ int c_slot_type[N_AA][SLOT_STRIDE];
+static __device__ float4 g_slot_prm[N_AA][SLOT_STRIDE];  // q*sqrt(332), r_min_half, sqrt(eps), hydrophobic
+static __device__ int g_slot_type[N_AA][SLOT_STRIDE];
 static __constant__ int c_topo_n[N_AA];
 static __constant__ float4 c_eef1[16];  // dg_ref, vol, lambda, 1/(PI32*lambda^3)
 static __constant__ int c_hb[16];       // bit0 donor, bit1 acceptor
@@ -46,8 +46,8 @@ static cudaError_t score_tables_init() {
         hb[t] = BT_HB[t];
     }
     cudaError_t e;
-    if ((e = cudaMemcpyToSymbol(c_slot_prm, slot, sizeof(slot))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_slot_type, stype, sizeof(stype))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(g_slot_prm, slot, sizeof(slot))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(g_slot_type, stype, sizeof(stype))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_topo_n, BT_TOPO_N, sizeof(BT_TOPO_N))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_eef1, eef, sizeof(eef))) != cudaSuccess) return e;
     return cudaMemcpyToSymbol(c_hb, hb, sizeof(hb));
@@ -111,30 +111,26 @@ __device__ __forceinline__ float warp_max_f(float v) {
 
 // ---- grouped scoring: one warp per group of <= 16 nearby candidate atoms ----------
 // A group (a residue of the resident state, or a few consecutive GpuAtoms) sits in
-// shared memory.  The warp walks the grid columns within 10 A + group radius of
-// the group centre (warp-uniform loop, lanes stride a column's contiguous atom
-// range), keeps the antigen atoms that pass a sphere test in a per-warp queue, and
-// evaluates full batches of 32 queued atoms against every group atom — so the
-// pair math never runs on idle lanes.  Every lane visits its antigen atoms in
-// increasing grid order, which keeps the sums deterministic.
+// shared memory.  The warp takes the antigen's blocks of 32 atoms whose boxes come within
+// 10 A + group radius of the group centre (warp-uniform loop, one atom per lane), keeps the
+// atoms that pass a sphere test in a per-warp queue, and evaluates full batches of 32 queued
+// atoms against every group atom — so the pair math never runs on idle lanes.  Every lane
+// visits its antigen atoms in increasing grid order, which keeps the sums deterministic.
 constexpr int GMAX = 16;
 
-// Group atom coordinates also as separate x / y / z arrays, so that the pair test
-// reads two atoms' coordinates as one 8-byte word; entries n..GMAX-1 hold GROUP_PAD.
+// Two group atoms side by side, as group_pairs reads them (16-byte loads, both atoms'
+// values of a field one 8-byte word): coordinates, r_min_half, sqrt(epsilon),
+// charge * sqrt(332), hydrophobic.  Entries past the group hold GROUP_PAD coordinates
+// and zero parameters (finite terms, never added).  nz holds -0 (f2_dist2).
 constexpr float GROUP_PAD = 1e30f;  // its squared distance to any atom overflows to +inf
+struct __align__(16) GroupTwo {
+    float x[2], y[2], z[2], rm[2], se[2], qs[2], hy[2], nz[2];
+};
 
 struct GroupSmem {
     float4 pos[GMAX];  // x, y, z, q*sqrt(332)
     float4 prm[GMAX];  // r_min_half, sqrt(epsilon), hydrophobic, AMBER type
-    __align__(8) float sx[GMAX];
-    __align__(8) float sy[GMAX];
-    __align__(8) float sz[GMAX];
-    // charge * sqrt(332), r_min_half, sqrt(epsilon), hydrophobic as separate arrays too,
-    // so that the pair terms read two atoms' parameters as one 8-byte word
-    __align__(8) float sqs[GMAX];
-    __align__(8) float srm[GMAX];
-    __align__(8) float sse[GMAX];
-    __align__(8) float shy[GMAX];
+    GroupTwo two[GMAX / 2];
     int q[64];         // queued antigen atom indices
 };
 // FULL scoring: the group atoms' EEF1 parameters (c_eef1), reciprocal lambdas and H-bond
@@ -157,24 +153,22 @@ __device__ __forceinline__ float div_by(float r, float d, float y) {
 }
 
 __device__ __forceinline__ void group_xyz(GroupSmem& s, int lane, int n, float x, float y, float z) {
-    if (lane < n) {
-        s.sx[lane] = x;
-        s.sy[lane] = y;
-        s.sz[lane] = z;
-    } else if (lane < GMAX) {
-        s.sx[lane] = s.sy[lane] = s.sz[lane] = GROUP_PAD;
-    }
+    if (lane >= GMAX) return;
+    GroupTwo& g = s.two[lane >> 1];
+    const int i = lane & 1;
+    g.x[i] = lane < n ? x : GROUP_PAD;
+    g.y[i] = lane < n ? y : GROUP_PAD;
+    g.z[i] = lane < n ? z : GROUP_PAD;
+    g.nz[i] = -0.0f;
 }
-// the parameter arrays of group atom `lane` (pads: zeros, finite terms never added)
 __device__ __forceinline__ void group_prm(GroupSmem& s, int lane, int n, float qs, float rmh, float se, float hy) {
-    if (lane < n) {
-        s.sqs[lane] = qs;
-        s.srm[lane] = rmh;
-        s.sse[lane] = se;
-        s.shy[lane] = hy;
-    } else if (lane < GMAX) {
-        s.sqs[lane] = s.srm[lane] = s.sse[lane] = s.shy[lane] = 0.0f;
-    }
+    if (lane >= GMAX) return;
+    GroupTwo& g = s.two[lane >> 1];
+    const int i = lane & 1;
+    g.qs[i] = lane < n ? qs : 0.0f;
+    g.rm[i] = lane < n ? rmh : 0.0f;
+    g.se[i] = lane < n ? se : 0.0f;
+    g.hy[i] = lane < n ? hy : 0.0f;
 }
 
 // The H-bond (energy.rs:303-307) and EEF1 solvation (solvation.rs:34-50) terms of a pair
@@ -203,7 +197,7 @@ __device__ __forceinline__ bool hb_pair(int a, int b) { return (a & ((b & 1) << 
 // (energy.rs:269-301); ir = 1 / r for the further terms.
 __device__ __forceinline__ float pair_base(const float4& b, const float4& bp, const float4& a, const float4& ap,
                                            float r2, float& ir) {
-    ir = rsqrtf(r2);
+    ir = rsqrt_normal(r2);
     const float ir2 = ir * ir;
     const float R = bp.x + ap.x;
     const float s2 = R * R * ir2;
@@ -215,7 +209,7 @@ __device__ __forceinline__ float pair_base(const float4& b, const float4& bp, co
 
 // One antigen atom (this lane's) against the n group atoms in shared memory, two
 // group atoms per step: dx = b - a in packed f32x2 arithmetic, r^2 = (dx*dx + dy*dy)
-// + dz*dz with the reference's roundings (scalar, never fused), hence its pair set;
+// + dz*dz with the reference's roundings (never fused), hence its pair set;
 // the terms of the pairs within the cutoff (packed) are added in group-atom order.
 // Returns the atom's sum over the group (f32, group-atom order).
 template <bool FULL, bool ABS, bool COUNT>
@@ -247,29 +241,33 @@ __device__ __forceinline__ float group_pairs(const float4* __restrict__ pq, cons
     const uint64_t ax = f2_pack(a.x, a.x), ay = f2_pack(a.y, a.y), az = f2_pack(a.z, a.z);
     const uint64_t aq = f2_pack(a.w, a.w), arm = f2_pack(ap.x, ap.x), ase = f2_pack(ap.y, ap.y);
     const uint64_t ahy = f2_pack(HYDRO_BONUS * ap.z, HYDRO_BONUS * ap.z), two = f2_pack(2.0f, 2.0f);
+    const uint64_t neg0 = *(const uint64_t*)s.two[0].nz;
 #pragma unroll 1
     for (int j = 0; j < n; j += 2) {
-        const uint64_t dx = f2_sub(*(const uint64_t*)&s.sx[j], ax);
-        const uint64_t dy = f2_sub(*(const uint64_t*)&s.sy[j], ay);
-        const uint64_t dz = f2_sub(*(const uint64_t*)&s.sz[j], az);
+        const ulonglong2* g = (const ulonglong2*)&s.two[j >> 1];
+        const ulonglong2 xy = g[0], zr = g[1];
+        const uint64_t dx = f2_sub(xy.x, ax);
+        const uint64_t dy = f2_sub(xy.y, ay);
+        const uint64_t dz = f2_sub(zr.x, az);
         float r2a, r2b;
-        f2_dist2(dx, dy, dz, r2a, r2b);
+        f2_dist2(dx, dy, dz, neg0, r2a, r2b);
         const bool ina = r2a <= CUTOFF_SQ && r2a >= MIN_R_SQ;
         const bool inb = r2b <= CUTOFF_SQ && r2b >= MIN_R_SQ;  // j + 1 = n: a pad, +inf
         if (FULL) {
             if (ina) term(j, r2a);
             if (inb) term(j + 1, r2b);
-        } else if (ina || inb) {
+        } else {
             // both pairs' terms in packed f32x2 arithmetic; an out-of-range element is
             // computed but never added
-            const uint64_t ir = f2_pack(rsqrtf(r2a), rsqrtf(r2b));
+            const ulonglong2 sq = g[2];
+            const uint64_t ir = f2_pack(rsqrt_normal(r2a), rsqrt_normal(r2b));
             const uint64_t ir2 = f2_mul(ir, ir);
-            const uint64_t R = f2_add(*(const uint64_t*)&s.srm[j], arm);
+            const uint64_t R = f2_add(zr.y, arm);
             const uint64_t s2 = f2_mul(f2_mul(R, R), ir2);
             const uint64_t s6 = f2_mul(f2_mul(s2, s2), s2);
-            const uint64_t lj = f2_mul(f2_mul(*(const uint64_t*)&s.sse[j], ase), f2_mul(s6, f2_sub(s6, two)));
-            const uint64_t coul = f2_mul(f2_mul(*(const uint64_t*)&s.sqs[j], aq), ir);
-            const uint64_t hy = f2_mul(*(const uint64_t*)&s.shy[j], ahy);
+            const uint64_t lj = f2_mul(f2_mul(sq.x, ase), f2_mul(s6, f2_sub(s6, two)));
+            const uint64_t coul = f2_mul(f2_mul(sq.y, aq), ir);
+            const uint64_t hy = f2_mul(((const uint64_t*)g)[6], ahy);
             const float hya = r2a < HYDRO_CUTOFF_SQ ? f2_lo(hy) : 0.0f;
             const float hyb = r2b < HYDRO_CUTOFF_SQ ? f2_hi(hy) : 0.0f;
             const uint64_t e = f2_add(f2_add(lj, coul), f2_pack(hya, hyb));
@@ -287,34 +285,30 @@ __device__ __forceinline__ float group_pairs(const float4* __restrict__ pq, cons
     return part;
 }
 
-// The grid columns within 10 A + group radius of a group's centre (group atoms in shared
-// memory, all lanes call).
-struct GroupCols {
+// The antigen atoms near a group: those within 10 A + group radius of its centre, among the
+// blocks b0 .. b1-1 of 32 atoms each (AgView::box; a block is taken or left by its box).
+struct GroupReach {
     float cx, cy, cz, reach2;  // centre, squared reach
-    float ux, uy, uz, rc2;     // the same in cell units
-    int i0, j0, nj, ncol;
-    // atom range of column `col` (x-major): its z-run of cells within reach (empty: ra0 = ra1)
-    __device__ __forceinline__ void range(const AgView* __restrict__ Ap, int col, int& ra0, int& ra1) const {
-        ra0 = ra1 = 0;
-        if (col >= ncol) return;
-        const int i = i0 + col / nj, j = j0 + col % nj;
-        const float ddx = fmaxf(fmaxf((float)i - ux, ux - (float)(i + 1)), 0.0f);
-        const float ddy = fmaxf(fmaxf((float)j - uy, uy - (float)(j + 1)), 0.0f);
-        const float rem2 = rc2 - ddx * ddx - ddy * ddy;
-        if (!(rem2 >= 0.0f)) return;
-        const int gny = Ap->grid.ny, gnz = Ap->grid.nz;
-        const float rem = sqrtf(rem2);
-        const int k0 = max(0, (int)floorf(uz - rem)), k1 = min(gnz - 1, (int)floorf(uz + rem));
-        if (k0 <= k1) {
-            const int base = (i * gny + j) * gnz;
-            ra0 = __ldg(&Ap->grid.cell_start[base + k0]);
-            ra1 = __ldg(&Ap->grid.cell_start[base + k1 + 1]);
-        }
+    int b0, b1;
+    __device__ __forceinline__ bool within(float ex, float ey, float ez) const {
+        return __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex))) <= reach2;
+    }
+    __device__ __forceinline__ bool atom(const float4& a) const { return within(a.x - cx, a.y - cy, a.z - cz); }
+    // false only if no atom of the block is within reach (each operation is monotonic in the
+    // atom's distance along an axis, rounding included)
+    __device__ __forceinline__ bool block(const AgView* __restrict__ Ap, int b) const {
+        if (b >= b1) return false;
+        const float4 lo = __ldg(&Ap->box[2 * b]), hi = __ldg(&Ap->box[2 * b + 1]);
+        return within(fmaxf(fmaxf(lo.x - cx, cx - hi.x), 0.0f), fmaxf(fmaxf(lo.y - cy, cy - hi.y), 0.0f),
+                      fmaxf(fmaxf(lo.z - cz, cz - hi.z), 0.0f));
     }
 };
-__device__ __forceinline__ GroupCols group_columns(const AgView* __restrict__ Ap, const GroupSmem& s, int n, int lane) {
-    GroupCols c;
-    const float inv = Ap->grid.inv;
+// Blocks from which a group looks at those of its x-slab of the grid only (two dependent
+// loads that a smaller antigen's few boxes do not repay).
+constexpr int SLAB_BLOCKS = 128;
+// (group atoms in shared memory, all lanes call)
+__device__ __forceinline__ GroupReach group_reach(const AgView* __restrict__ Ap, const GroupSmem& s, int n, int lane) {
+    GroupReach c;
     float px = 0.f, py = 0.f, pz = 0.f;
     if (lane < n) {
         const float4 p = s.pos[lane];
@@ -328,16 +322,19 @@ __device__ __forceinline__ GroupCols group_columns(const AgView* __restrict__ Ap
     const float rad2 = warp_max_f(lane < n ? dgx * dgx + dgy * dgy + dgz * dgz : 0.0f);
     const float reach = 10.01f + sqrtf(rad2) * 1.0001f + 1e-3f;
     c.reach2 = reach * reach;
-    c.ux = c.cx * inv - (float)Ap->grid.ox;
-    c.uy = c.cy * inv - (float)Ap->grid.oy;
-    c.uz = c.cz * inv - (float)Ap->grid.oz;
-    const float rc = reach * inv;
-    c.rc2 = rc * rc;
-    c.i0 = max(0, (int)floorf(c.ux - rc));
-    c.j0 = max(0, (int)floorf(c.uy - rc));
-    const int i1 = min(Ap->grid.nx - 1, (int)floorf(c.ux + rc)), j1 = min(Ap->grid.ny - 1, (int)floorf(c.uy + rc));
-    c.nj = j1 - c.j0 + 1;
-    c.ncol = (i1 >= c.i0 && j1 >= c.j0) ? (i1 - c.i0 + 1) * c.nj : 0;
+    c.b0 = 0;
+    c.b1 = (Ap->n_atoms + 31) >> 5;
+    if (c.b1 > SLAB_BLOCKS) {
+        const GridView& g = Ap->grid;
+        const float ux = c.cx * g.inv - (float)g.ox, rc = reach * g.inv;
+        const int i0 = max(0, (int)floorf(ux - rc)), i1 = min(g.nx - 1, (int)floorf(ux + rc));
+        if (i0 <= i1) {
+            c.b0 = __ldg(&g.cell_start[i0 * g.ny * g.nz]) >> 5;
+            c.b1 = (__ldg(&g.cell_start[(i1 + 1) * g.ny * g.nz]) + 31) >> 5;
+        } else {
+            c.b1 = 0;
+        }
+    }
     return c;
 }
 // FULL scoring: the group atoms' further parameters (prm visible to the warp)
@@ -353,45 +350,35 @@ __device__ __forceinline__ void group_full(const GroupSmem& s, GroupFull* gf, in
 }
 
 // Everything one warp does for one group already in shared memory (n atoms): centre
-// and radius, warp-uniform walk over the culled grid columns, sphere prefilter into
-// the queue, batched pair evaluation.  Accumulates into the lane's acc.
+// and radius, the antigen's blocks that come near it (32 boxes at a time), their atoms
+// within reach into the queue, batched pair evaluation.  Accumulates into the lane's acc.
+// The blocks are in the atoms' grid order and hold 32 atoms each, aligned: one test per
+// block, where walking the grid's columns took divisions, a square root and two dependent
+// loads per 32 columns and partly filled steps at their ends (one peptide of 60 atoms
+// against 2500, whole call: 60 us, 52 us now; long launches change little).
 template <bool KAHAN, bool FULL, bool ABS, bool COUNT>
 __device__ __forceinline__ void score_group(const AgView* __restrict__ Ap, GroupSmem& s, GroupFull* gf, int n,
                                             int lane, unsigned lt, Acc& acc) {
     const float4* __restrict__ pq = Ap->pq;
     const float4* __restrict__ prm = Ap->prm;
-    const GroupCols cols = group_columns(Ap, s, n, lane);
-    const float reach2 = cols.reach2, cx = cols.cx, cy = cols.cy, cz = cols.cz;
-    const int ncol = cols.ncol;
+    const int n_atoms = Ap->n_atoms;
+    const GroupReach near = group_reach(Ap, s, n, lane);
     if (FULL) group_full(s, gf, n, lane);
     int qn = 0;
-    for (int c0 = 0; c0 < ncol; c0 += 32) {
-        int ra0 = 0, ra1 = 0;
-        cols.range(Ap, c0 + lane, ra0, ra1);
-        unsigned live = __ballot_sync(0xffffffffu, ra1 > ra0);
-        while (live) {
-            const int src = __ffs(live) - 1;
-            live &= live - 1;
-            const int a0 = __shfl_sync(0xffffffffu, ra0, src), a1 = __shfl_sync(0xffffffffu, ra1, src);
-            for (int t0 = a0; t0 < a1; t0 += 32) {
-                const int t = t0 + lane;
-                bool pass = false;
-                if (t < a1) {
-                    const float4 a = __ldg(&pq[t]);
-                    const float ex = a.x - cx, ey = a.y - cy, ez = a.z - cz;
-                    pass = ex * ex + ey * ey + ez * ez <= reach2;
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, pass);
-                if (pass) s.q[qn + __popc(m & lt)] = t;
-                qn += __popc(m);
+    for (int w0 = near.b0; w0 < near.b1; w0 += 32) {
+        for (unsigned live = __ballot_sync(0xffffffffu, near.block(Ap, w0 + lane)); live; live &= live - 1) {
+            const int t = (w0 + __ffs(live) - 1) * 32 + lane;
+            const bool pass = t < n_atoms && near.atom(__ldg(&pq[t]));
+            const unsigned m = __ballot_sync(0xffffffffu, pass);
+            if (pass) s.q[qn + __popc(m & lt)] = t;
+            qn += __popc(m);
+            __syncwarp();
+            if (qn >= 32) {
+                acc_add<KAHAN>(acc, group_pairs<FULL, ABS, COUNT>(pq, prm, s, gf, n, s.q[lane], acc));
                 __syncwarp();
-                if (qn >= 32) {
-                    acc_add<KAHAN>(acc, group_pairs<FULL, ABS, COUNT>(pq, prm, s, gf, n, s.q[lane], acc));
-                    __syncwarp();
-                    if (lane < qn - 32) s.q[lane] = s.q[32 + lane];
-                    qn -= 32;
-                    __syncwarp();
-                }
+                if (lane < qn - 32) s.q[lane] = s.q[32 + lane];
+                qn -= 32;
+                __syncwarp();
             }
         }
     }
@@ -400,17 +387,16 @@ __device__ __forceinline__ void score_group(const AgView* __restrict__ Ap, Group
 }
 
 // The full energy of one group by a team of TEAM warps (warp `rank`; sync(): the team's
-// barrier): what score_group's lanes sum, in the same order, with the work shared.  The
-// columns' atom ranges are concatenated; the warps prefilter 32 atoms of the concatenation
-// each (up to TEAM_SEG chunks a segment), place the passing ones in the team's list -- the
-// single warp's queue -- and evaluate its batches of 32 in turn into the team's slots;
-// warp 0 adds the slots to its acc, batch after batch, so every lane of it sums exactly
-// the terms it would sum alone.  Result in warp 0's acc.
+// barrier): what score_group's lanes sum, in the same order, with the work shared.  Of the
+// blocks of 32 boxes that come near the group, the warps take one each in turn, place the
+// atoms within reach in the team's list -- the single warp's queue -- and evaluate its
+// batches of 32 in turn into the team's slots; warp 0 adds the slots to its acc, batch after
+// batch, so every lane of it sums exactly the terms it would sum alone.  Result in warp 0's acc.
 constexpr int TEAM_SEG = 32;
 struct TeamSmem {
     float part[TEAM_SEG + 1][32];
     int list[TEAM_SEG * 32 + 32];  // queued atoms: the last segment's rest, then this one's
-    int found[TEAM_SEG][32];       // passing atoms of each chunk
+    int found[TEAM_SEG][32];       // passing atoms of each block
     int count[TEAM_SEG];
 };
 template <bool KAHAN, int TEAM, class Sync>
@@ -418,80 +404,55 @@ __device__ __forceinline__ void score_group_team(const AgView* __restrict__ Ap, 
                                                  int lane, unsigned lt, Acc& acc, int rank, TeamSmem& T, Sync sync) {
     const float4* __restrict__ pq = Ap->pq;
     const float4* __restrict__ prm = Ap->prm;
-    const GroupCols cols = group_columns(Ap, s, n, lane);
+    const int n_atoms = Ap->n_atoms;
+    const GroupReach near = group_reach(Ap, s, n, lane);
     group_full(s, gf, n, lane);
     int qn = 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < cols.ncol; c0 += 32) {
-        int ra0 = 0, ra1 = 0;
-        cols.range(Ap, c0 + lane, ra0, ra1);
-        const int len = ra1 - ra0;
-        int incl = len;
+    for (int w0 = near.b0; w0 < near.b1; w0 += 32) {
+        const unsigned live = __ballot_sync(0xffffffffu, near.block(Ap, w0 + lane));
+        const int chunks = __popc(live);
+        int ch = 0;
+        for (unsigned m = live; m; m &= m - 1, ++ch) {
+            if (ch % TEAM != rank) continue;
+            const int t = (w0 + __ffs(m) - 1) * 32 + lane;
+            const bool pass = t < n_atoms && near.atom(__ldg(&pq[t]));
+            const unsigned pm = __ballot_sync(0xffffffffu, pass);
+            if (pass) T.found[ch][__popc(pm & lt)] = t;
+            if (lane == 0) T.count[ch] = __popc(pm);
+        }
+        sync();
+        int at = lane < chunks ? T.count[lane] : 0;  // inclusive prefix over the blocks
+        const int own = at;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += v;
+            const int v = __shfl_up_sync(0xffffffffu, at, d);
+            if (lane >= d) at += v;
         }
-        const int tot = __shfl_sync(0xffffffffu, incl, 31);
-        const bool last_cols = c0 + 32 >= cols.ncol;
-        int f0 = 0;
-        do {  // (once when tot = 0: the last segment closes the sums)
-            const int chunks = min(TEAM_SEG, (tot - f0 + 31) / 32);
+        const int found = __shfl_sync(0xffffffffu, at, 31);
 #pragma unroll 1
-            for (int ch = rank; ch < chunks; ch += TEAM) {
-                const int f = f0 + ch * 32 + lane, fq = min(f, tot - 1);
-                int lo = 0;  // the first column whose inclusive prefix exceeds fq
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int v = __shfl_sync(0xffffffffu, incl, lo + step - 1);
-                    if (v <= fq) lo += step;
-                }
-                const int v_lo = __shfl_sync(0xffffffffu, incl, lo), len_lo = __shfl_sync(0xffffffffu, len, lo);
-                const int t = __shfl_sync(0xffffffffu, ra0, lo) + (fq - (v_lo - len_lo));
-                bool pass = false;
-                if (f < tot) {
-                    const float4 a = __ldg(&pq[t]);
-                    const float ex = a.x - cols.cx, ey = a.y - cols.cy, ez = a.z - cols.cz;
-                    pass = ex * ex + ey * ey + ez * ez <= cols.reach2;
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, pass);
-                if (pass) T.found[ch][__popc(m & lt)] = t;
-                if (lane == 0) T.count[ch] = __popc(m);
-            }
-            sync();
-            int at = lane < chunks ? T.count[lane] : 0;  // inclusive prefix over the chunks
-            const int own = at;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, at, d);
-                if (lane >= d) at += v;
-            }
-            const int found = __shfl_sync(0xffffffffu, at, 31);
+        for (int ch = rank; ch < chunks; ch += TEAM) {
+            const int cnt = __shfl_sync(0xffffffffu, own, ch), to = qn + __shfl_sync(0xffffffffu, at, ch) - cnt;
+            if (lane < cnt) T.list[to + lane] = T.found[ch][lane];
+        }
+        qn += found;
+        const bool last = w0 + 32 >= near.b1;
+        sync();
+        const int full = qn / 32, rest = qn - full * 32, batches = full + (last && rest ? 1 : 0);
 #pragma unroll 1
-            for (int ch = rank; ch < chunks; ch += TEAM) {
-                const int cnt = __shfl_sync(0xffffffffu, own, ch), to = qn + __shfl_sync(0xffffffffu, at, ch) - cnt;
-                if (lane < cnt) T.list[to + lane] = T.found[ch][lane];
-            }
-            qn += found;
-            f0 += TEAM_SEG * 32;
-            const bool last = last_cols && f0 >= tot;
-            sync();
-            const int full = qn / 32, rest = qn - full * 32, batches = full + (last && rest ? 1 : 0);
+        for (int b = rank; b < batches; b += TEAM) {
+            if (b * 32 + lane < qn)
+                T.part[b][lane] = group_pairs<true, false, false>(pq, prm, s, gf, n, T.list[b * 32 + lane], acc);
+        }
+        sync();
+        if (rank == 0) {
 #pragma unroll 1
-            for (int b = rank; b < batches; b += TEAM) {
-                if (b * 32 + lane < qn)
-                    T.part[b][lane] = group_pairs<true, false, false>(pq, prm, s, gf, n, T.list[b * 32 + lane], acc);
-            }
-            sync();
-            if (rank == 0) {
-#pragma unroll 1
-                for (int b = 0; b < batches; ++b)
-                    if (b * 32 + lane < qn) acc_add<KAHAN>(acc, T.part[b][lane]);
-                if (lane < rest && full) T.list[lane] = T.list[full * 32 + lane];
-            }
-            qn = rest;
-            if (!last) sync();  // the list's rest and the slots
-        } while (f0 < tot);
+            for (int b = 0; b < batches; ++b)
+                if (b * 32 + lane < qn) acc_add<KAHAN>(acc, T.part[b][lane]);
+            if (lane < rest && full) T.list[lane] = T.list[full * 32 + lane];
+        }
+        qn = rest;
+        if (!last) sync();  // the list's rest and the slots
     }
     sync();  // the next group reuses the team's memory
 }
