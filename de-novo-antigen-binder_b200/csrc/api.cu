@@ -89,6 +89,33 @@ struct GridBuf {
     GridView view{};
 };
 
+// The contents of the resident drop-in antigen, as the caller's arrays held them.
+struct DropinKey {
+    size_t n = 0;
+    bool typed = false;
+    std::vector<float> f;    // x, y, z, charge, r_min_half, epsilon
+    std::vector<uint8_t> b;  // hydrophobic, atom type
+
+    bool holds(const binder_atom_cloud* a) const {
+        const float* src[6] = {a->x, a->y, a->z, a->charge, a->r_min_half, a->epsilon};
+        if (a->n != n || (a->atom_type != nullptr) != typed) return false;
+        for (int k = 0; k < 6; ++k)
+            if (n && std::memcmp(src[k], f.data() + k * n, n * sizeof(float))) return false;
+        return !n || (!std::memcmp(a->hydrophobic, b.data(), n) && (!typed || !std::memcmp(a->atom_type, b.data() + n, n)));
+    }
+    void set(const binder_atom_cloud* a) {
+        const float* src[6] = {a->x, a->y, a->z, a->charge, a->r_min_half, a->epsilon};
+        n = a->n;
+        typed = a->atom_type != nullptr;
+        f.resize(6 * n);
+        b.resize((typed ? 2 : 1) * n);
+        if (!n) return;
+        for (int k = 0; k < 6; ++k) std::memcpy(f.data() + k * n, src[k], n * sizeof(float));
+        std::memcpy(b.data(), a->hydrophobic, n);
+        if (typed) std::memcpy(b.data() + n, a->atom_type, n);
+    }
+};
+
 // One resident antigen: all-atom records + score grid, Calpha cloud + CG grid.
 struct Antigen {
     int n_atoms = 0, n_res = 0;
@@ -208,7 +235,7 @@ struct binder_ctx {
     Antigen dropin;
     DBuf<AgView> d_dropin_view;
     bool dropin_valid = false;
-    std::vector<float> dropin_key;
+    DropinKey dropin_key;
     // resident search antigens
     std::vector<std::unique_ptr<Antigen>> ags;
     DBuf<AgView> d_views;
@@ -512,32 +539,26 @@ int validate_cloud(binder_ctx* ctx, const binder_atom_cloud* c, const char* what
     return BINDER_OK;
 }
 
-// Upload the drop-in antigen when its contents differ from the resident copy.
+// Upload the drop-in antigen when its contents differ from the resident copy (compared where
+// they lie: packing 2500 atoms into one key first took 20 us of every call).  A failure leaves
+// no copy of the caller's memory in flight.
 int ensure_dropin(binder_ctx* ctx, const binder_atom_cloud* ag) {
     int s = validate_cloud(ctx, ag, "antigen");
-    if (s) return s;
-    const size_t n = ag->n;
-    std::vector<float> key;
-    key.reserve(n * 7 + 2);
-    key.push_back((float)n);
-    key.push_back(ag->atom_type ? 1.0f : 0.0f);
-    for (size_t i = 0; i < n; ++i) {
-        key.push_back(ag->x[i]); key.push_back(ag->y[i]); key.push_back(ag->z[i]);
-        key.push_back(ag->charge[i]); key.push_back(ag->r_min_half[i]); key.push_back(ag->epsilon[i]);
-        key.push_back((float)ag->hydrophobic[i] + (ag->atom_type ? 256.0f * ag->atom_type[i] : 0.0f));
+    if (!s && ctx->dropin_valid && ctx->dropin_key.holds(ag)) return BINDER_OK;
+    if (!s) {
+        ctx->dropin_valid = false;
+        s = build_antigen_atoms(ctx, ctx->dropin, ag->x, ag->y, ag->z, ag->charge, ag->r_min_half, ag->epsilon,
+                                ag->hydrophobic, ag->atom_type, ag->n);
     }
-    if (ctx->dropin_valid && key.size() == ctx->dropin_key.size() &&
-        std::memcmp(key.data(), ctx->dropin_key.data(), key.size() * sizeof(float)) == 0)
-        return BINDER_OK;
-    ctx->dropin_valid = false;
-    if ((s = build_antigen_atoms(ctx, ctx->dropin, ag->x, ag->y, ag->z, ag->charge, ag->r_min_half, ag->epsilon,
-                                 ag->hydrophobic, ag->atom_type, n)))
+    if (s) {
+        cudaStreamSynchronize(ctx->stream);
         return s;
+    }
     CK(ctx->d_dropin_view.ensure(1), "view alloc");
     CK(cudaMemcpyAsync(ctx->d_dropin_view.p, &ctx->dropin.view, sizeof(AgView), cudaMemcpyHostToDevice, ctx->stream),
        "view H2D");
     CK(cudaStreamSynchronize(ctx->stream), "synchronize");
-    ctx->dropin_key.swap(key);
+    ctx->dropin_key.set(ag);
     ctx->dropin_valid = true;
     return BINDER_OK;
 }
@@ -589,11 +610,12 @@ int score_batch_common(binder_ctx* ctx, const binder_atom_cloud* antigen, const 
     if (!candidates) return fail(ctx, BINDER_ERR_ARG, "candidates is NULL");
     if (out_cap < n_cand) return fail(ctx, BINDER_ERR_CAPACITY, "out_cap %zu < n_cand %zu", out_cap, n_cand);
     if (n_cand > (size_t)INT32_MAX) return fail(ctx, BINDER_ERR_ARG, "too many candidates");
-    if ((s = ensure_dropin(ctx, antigen))) return s;
+    if ((s = validate_cloud(ctx, antigen, "antigen"))) return s;
     const size_t used = n_cand * n_ab;
     CK(ctx->cand.ensure(used * 8), "alloc candidates");
     CK(cudaMemcpyAsync(ctx->cand.p, candidates, used * sizeof(binder_gpu_atom), cudaMemcpyHostToDevice, ctx->stream),
        "candidates H2D");
+    if ((s = ensure_dropin(ctx, antigen))) return s;  // while the candidates are copied
     if ((s = score_resident_batch(ctx, (int)n_cand, (long long)n_ab, out_abs != nullptr))) return s;
     return fetch_energies(ctx, (int)n_cand, out64, out_abs, out32);
 }
@@ -784,12 +806,13 @@ int binder_score_batch_ragged(binder_ctx* ctx, const binder_atom_cloud* antigen,
         if (offsets[c + 1] < offsets[c]) return fail(ctx, BINDER_ERR_ARG, "offsets must be non-decreasing");
     const size_t n_atoms = (size_t)offsets[n_cand];
     if (n_atoms && !candidates) return fail(ctx, BINDER_ERR_ARG, "candidates is NULL");
-    if ((s = ensure_dropin(ctx, antigen))) return s;
+    if ((s = validate_cloud(ctx, antigen, "antigen"))) return s;
     CK(ctx->cand.ensure(n_atoms * 8), "alloc candidates");
     if (n_atoms)
         CK(cudaMemcpyAsync(ctx->cand.p, candidates, n_atoms * sizeof(binder_gpu_atom), cudaMemcpyHostToDevice,
                            ctx->stream),
            "candidates H2D");
+    if ((s = ensure_dropin(ctx, antigen))) return s;
     if ((s = upload(ctx, ctx->off, (const long long*)offsets, n_cand + 1, "offsets H2D"))) return s;
     if ((s = score_resident_batch(ctx, (int)n_cand, 0, out_abs != nullptr))) return s;
     return fetch_energies(ctx, (int)n_cand, out, out_abs, nullptr);
@@ -945,10 +968,11 @@ int binder_forces_allatom(binder_ctx* ctx, const binder_atom_cloud* antigen, con
     for (size_t c = 0; c < n_cand; ++c)
         if (offsets[c + 1] < offsets[c]) return fail(ctx, BINDER_ERR_ARG, "offsets must be non-decreasing");
     const size_t n_atoms = (size_t)offsets[n_cand];
-    if ((s = ensure_dropin(ctx, antigen))) return s;
+    if ((s = validate_cloud(ctx, antigen, "antigen"))) return s;
     CK(ctx->cand.ensure(n_atoms * 8), "alloc");
     if (n_atoms)
         CK(cudaMemcpyAsync(ctx->cand.p, candidates, n_atoms * 32, cudaMemcpyHostToDevice, ctx->stream), "H2D");
+    if ((s = ensure_dropin(ctx, antigen))) return s;
     if ((s = upload(ctx, ctx->off, (const long long*)offsets, n_cand + 1, "offsets H2D"))) return s;
     CK(ctx->energy.ensure(n_cand), "alloc");
     CK(ctx->force.ensure(3 * n_atoms), "alloc");
