@@ -298,7 +298,8 @@ int binder_block_io(binder_ctx* ctx, size_t n_cand, const int32_t* n_res, int32_
 
 /* ---- launch shapes and the autotuner (no reference counterpart) ----------------
    Results never depend on these: every residue is computed by the same lanes with
-   the same arithmetic whatever the grid. */
+   the same arithmetic whatever the grid.  Until the caller sets or tunes them they follow
+   the state's size. */
 typedef struct binder_launch_cfg {
     int32_t score_warps;        /* warps per CTA of the persistent scoring kernel: 4, 8, 16 */
     int32_t score_ctas_per_sm;  /* persistent scoring CTAs per SM: 1..32 */
@@ -312,7 +313,9 @@ typedef struct binder_launch_cfg {
                                    residues in work bands for the next, which deals them to its
                                    tasks heaviest first; no extra launch */
     int32_t score_order;        /* work-queue order of the scoring kernel: 0 by Calpha cell (three
-                                   sorting launches after every move), 1 residue index */
+                                   sorting launches after every move), 1 residue index, or the
+                                   work bands of cg_order 3, heaviest first, once they hold
+                                   the state's residues */
     int32_t cg_queue;           /* gradient-step kernel: 0 one CTA per residue batch, 1 persistent
                                    CTAs whose warps take residue batches from a work queue */
     int32_t cg_flat;            /* gradient-step kernel: 0 the lane-group form (cg_lanes lanes per
