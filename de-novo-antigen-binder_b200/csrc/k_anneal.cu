@@ -33,9 +33,9 @@
 // more per backbone move) and many candidates share an SM.  64 x 20 residues, 300-residue
 // antigen, 600 steps: 13.4 ms before (42 k cycles a step: lane-0 FP64 folds of every
 // energy, one thread scanning for Cys pairs, side chains built from divergent constant
-// tables and local memory, nine barriers), 9.5 ms now; 1024 x 20 residues, 60 steps:
-// 7.9 ms before, 4.2 ms now.  What is left is about 6.5 cycles per dependent instruction
-// (2.5 of fixed latency, 1 of shared memory, 0.8 of branches, 0.6-0.9 of instruction
+// tables and local memory, nine barriers), 9.5 ms so arranged, 9.1 ms with the lists kept
+// between launches and the skins below; 1024 x 20 residues, 60 steps: 7.9, 4.2, 4.1 ms.
+// What is left is about 6.5 cycles per dependent instruction (2.5 of fixed latency, 1 of shared memory, 0.8 of branches, 0.6-0.9 of instruction
 // fetch): the code is kept small -- one copy of each exponential, pair term and scan, no
 // unrolling (178 -> 122 KB) -- because several warps in different phases of unrolled code
 // waited for instructions more than for anything else (a 1024-candidate launch 5.5 -> 4.3 ms).
