@@ -1163,8 +1163,24 @@ int ensure_trig(binder_ctx* ctx) {
     return BINDER_OK;
 }
 
+// Verlet-list storage for every residue of the state (the gradient-step and Metropolis
+// kernels read and write all three arrays by residue).  Growing drops every kept list, the
+// old ones first: after a failed allocation no entry may point into the new storage.
+int ensure_lists(binder_ctx* ctx, int total) {
+    State& S = ctx->st;
+    const size_t n = (size_t)std::max(total, 1);
+    if (S.cg_meta.p && S.cg_meta.n >= n) return BINDER_OK;
+    S.cg_meta.release();
+    CK(S.cg_list.ensure(n * CG_LIST_CAP), "alloc");
+    CK(S.cg_centre.ensure(n), "alloc");
+    CK(S.cg_meta.ensure(n), "alloc");
+    CK(cudaMemsetAsync(S.cg_meta.p, 0xFF, S.cg_meta.n * sizeof(int4), ctx->stream), "memset");
+    return BINDER_OK;
+}
+
 // Candidate metadata of the resident state: residue offsets, antigen, Philox id,
-// per-antigen candidate groups, sort keys and scratch sizes.
+// per-antigen candidate groups, sort keys, list storage and scratch sizes.  The state is
+// empty until all of it has its size, so that no kernel runs on a half-grown one.
 int set_state_meta(binder_ctx* ctx, const std::vector<int>& off, const std::vector<int>& ag,
                    const std::vector<uint32_t>& ids, const std::vector<int>& orig) {
     State& S = ctx->st;
@@ -1184,8 +1200,7 @@ int set_state_meta(binder_ctx* ctx, const std::vector<int>& off, const std::vect
     std::vector<int> g_idx(n_cand);
     std::vector<long long> cur(g_off.begin(), g_off.end() - 1);
     for (size_t c = 0; c < n_cand; ++c) g_idx[cur[ag[c]]++] = (int)c;
-    S.n_cand = (int)n_cand;
-    S.total_res = total;
+    S.n_cand = S.total_res = 0;
     S.max_res = max_res;
     S.h_res_off = off;
     S.h_cand_ag = ag;
@@ -1224,6 +1239,9 @@ int set_state_meta(binder_ctx* ctx, const std::vector<int>& off, const std::vect
     CK(cudaMemsetAsync(S.queue.p, 0, 4 * sizeof(int), ctx->stream), "memset");
     CK(S.res_e.ensure(std::max(total, 1)), "alloc");
     CK(S.res_abs.ensure(std::max(total, 1)), "alloc");
+    if ((s = ensure_lists(ctx, total))) return s;
+    S.n_cand = (int)n_cand;
+    S.total_res = total;
     S.order_valid = false;
     S.meta_epoch = ctx->ag_epoch;
     if (!ctx->cfg_chosen) ctx->cfg = default_launch_cfg(total);
@@ -1277,12 +1295,6 @@ static int state_upload_impl(binder_ctx* ctx, size_t n_cand, const int32_t* n_re
         CK(cudaMemcpyAsync(S.res_chi.p, chi, (size_t)total * 16, cudaMemcpyHostToDevice, ctx->stream), "H2D");
         CK(cudaMemcpyAsync(S.stage.p, pos, (size_t)total * SLOTS * 3 * 4, cudaMemcpyHostToDevice, ctx->stream),
            "H2D");
-    }
-    if (S.cg_meta.n < (size_t)total || !S.cg_meta.p) {  // fresh list storage: every list invalid
-        CK(S.cg_list.ensure((size_t)total * CG_LIST_CAP), "alloc");
-        CK(S.cg_centre.ensure(total), "alloc");
-        CK(S.cg_meta.ensure(total), "alloc");
-        CK(cudaMemsetAsync(S.cg_meta.p, 0xFF, S.cg_meta.n * sizeof(int4), ctx->stream), "memset");
     }
     if (copy_data) {
         launch_pack_slots(ctx->stream, total, S.stage.p, S.res_pos.p);
@@ -1617,7 +1629,7 @@ std::vector<uint64_t> block_sig(binder_ctx* ctx, int n_steps, int k) {
     const void* ptrs[] = {S.cand_res_off.p, S.cand_ag.p, S.cand_id.p, S.res_aa.p, S.res_chi.p, S.res_pos.p,
                           S.res_trig.p, S.res_cand.p, S.ag_cand_idx.p, S.ag_cand_off.p, S.key_base.p, S.keys.p,
                           S.key_counts.p, S.key_cursor.p, S.order.p, S.cg_bal.p, S.queue.p, S.res_e.p,
-                          S.res_abs.p,
+                          S.res_abs.p, S.cg_list.p, S.cg_centre.p, S.cg_meta.p,
                           ctx->energy.p, ctx->topk.p, ctx->errf.p, ctx->d_views.p};
     for (const void* q : ptrs) v.push_back((uint64_t)(uintptr_t)q);
     unsigned char pb[sizeof(binder_params)];
