@@ -1286,10 +1286,18 @@ static int state_upload_impl(binder_ctx* ctx, size_t n_cand, const int32_t* n_re
     if (same_meta) S.order_valid = false;
     else if ((s = set_state_meta(ctx, off, ag, ids, orig))) return s;
     S.trig_valid = false;
-    CK(S.res_aa.ensure(total), "alloc");
-    CK(S.res_chi.ensure(total), "alloc");
-    CK(S.stage.ensure((size_t)total * SLOTS * 3), "alloc");
-    CK(S.res_pos.ensure((size_t)total * SLOT_STRIDE), "alloc");
+    auto grow = [&]() -> int {
+        CK(S.res_aa.ensure(total), "alloc");
+        CK(S.res_chi.ensure(total), "alloc");
+        CK(S.stage.ensure((size_t)total * SLOTS * 3), "alloc");
+        CK(S.res_pos.ensure((size_t)total * SLOT_STRIDE), "alloc");
+        CK(S.mc_stats.ensure(4 * n_cand), "alloc");
+        return BINDER_OK;
+    };
+    if ((s = grow())) {  // no state without its buffers
+        S.n_cand = S.total_res = 0;
+        return s;
+    }
     if (copy_data && total) {
         CK(cudaMemcpyAsync(S.res_aa.p, aa, (size_t)total, cudaMemcpyHostToDevice, ctx->stream), "H2D");
         CK(cudaMemcpyAsync(S.res_chi.p, chi, (size_t)total * 16, cudaMemcpyHostToDevice, ctx->stream), "H2D");
@@ -1300,7 +1308,6 @@ static int state_upload_impl(binder_ctx* ctx, size_t n_cand, const int32_t* n_re
         launch_pack_slots(ctx->stream, total, S.stage.p, S.res_pos.p);
         if (total) LAUNCHED("pack_slots");
     }
-    CK(S.mc_stats.ensure(4 * n_cand), "alloc");
     CK(cudaMemsetAsync(S.mc_stats.p, 0, 4 * n_cand * sizeof(long long), ctx->stream), "memset");
     if (sync) CK(cudaStreamSynchronize(ctx->stream), "synchronize");
     return BINDER_OK;

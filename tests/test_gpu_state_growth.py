@@ -42,3 +42,43 @@ def test_growing_selection(pkg, n_cand, n_res, copies, lane_groups):
             got.append(ctx.state_download() + (ctx.mc_stats(), e, top))
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("grow", ["upload", "select"])
+def test_no_state_without_its_buffers(pkg, grow):
+    """An allocation that fails while the state grows leaves either the old state or none:
+    the calls that follow are refused, and a later upload works."""
+    L = pkg.lib()
+    failed = 0
+    try:
+        for k in range(64):
+            with pkg.GpuContext.create(0, pkg.Params.defaults(shell_radius=18.0)) as ctx:
+                aa, chi, pos = _population(pkg, ctx, 12, 5)
+                ctx.state_upload(aa[:15], chi[:15], pos[:15], uniform_n_res=5)
+                ctx.diffuse(2)
+                L.binder_debug_fail_alloc(k)
+                try:
+                    if grow == "upload":
+                        ctx.state_upload(aa, chi, pos, uniform_n_res=5)
+                    else:
+                        ctx.state_select(np.arange(12) % 3)
+                except pkg.BinderError as e:
+                    assert e.status == 3  # BINDER_ERR_OOM
+                    failed += 1
+                    L.binder_debug_fail_alloc(-1)
+                    assert ctx.state_info()[0] in ((0,) if grow == "upload" else (0, 3))
+                    if ctx.state_info()[0] == 0:
+                        for call in (lambda: ctx.diffuse(2), lambda: ctx.diffuse(2, with_mc=True), ctx.score_state,
+                                     ctx.state_download, lambda: ctx.state_select([0])):
+                            with pytest.raises(pkg.BinderError) as ei:
+                                call()
+                            assert ei.value.status == 7  # BINDER_ERR_STATE
+                    ctx.state_upload(aa, chi, pos, uniform_n_res=5)
+                    assert np.array_equal(ctx.state_download()[2], pos)
+                    ctx.diffuse(2)
+                else:
+                    L.binder_debug_fail_alloc(-1)
+                    break
+    finally:
+        L.binder_debug_fail_alloc(-1)
+    assert failed >= (5 if grow == "upload" else 10) and failed < 63
