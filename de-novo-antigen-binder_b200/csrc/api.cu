@@ -540,18 +540,15 @@ int validate_cloud(binder_ctx* ctx, const binder_atom_cloud* c, const char* what
 }
 
 // Upload the drop-in antigen when its contents differ from the resident copy (compared where
-// they lie: packing 2500 atoms into one key first took 20 us of every call).  A failure leaves
-// no copy of the caller's memory in flight.
+// they lie: packing 2500 atoms into one key first took 20 us of every call).
 int ensure_dropin(binder_ctx* ctx, const binder_atom_cloud* ag) {
     int s = validate_cloud(ctx, ag, "antigen");
-    if (!s && ctx->dropin_valid && ctx->dropin_key.holds(ag)) return BINDER_OK;
-    if (!s) {
-        ctx->dropin_valid = false;
-        s = build_antigen_atoms(ctx, ctx->dropin, ag->x, ag->y, ag->z, ag->charge, ag->r_min_half, ag->epsilon,
-                                ag->hydrophobic, ag->atom_type, ag->n);
-    }
-    if (s) {
-        cudaStreamSynchronize(ctx->stream);
+    if (s) return s;
+    if (ctx->dropin_valid && ctx->dropin_key.holds(ag)) return BINDER_OK;
+    ctx->dropin_valid = false;
+    if ((s = build_antigen_atoms(ctx, ctx->dropin, ag->x, ag->y, ag->z, ag->charge, ag->r_min_half, ag->epsilon,
+                                 ag->hydrophobic, ag->atom_type, ag->n))) {
+        cudaStreamSynchronize(ctx->stream);  // no copy of the caller's arrays stays in flight
         return s;
     }
     CK(ctx->d_dropin_view.ensure(1), "view alloc");
@@ -565,13 +562,34 @@ int ensure_dropin(binder_ctx* ctx, const binder_atom_cloud* ag) {
 
 int grid_ctas(binder_ctx* ctx, int n_cand) { return std::min(n_cand, ctx->num_sms * 8); }
 
-// Score n_cand candidates already in ctx->cand (n_ab atoms each, or ragged with the offsets
-// in ctx->off when n_ab = 0) against the drop-in antigen.
-int score_resident_batch(binder_ctx* ctx, int n_cand, long long n_ab, bool want_abs) {
-    int s;
+// The buffers of a flat batch (offs: with ragged offsets), and the candidates' copy, the
+// first of the caller's arrays in flight: from here on nothing but a CUDA error returns
+// before a synchronisation.  The batch that binder_last_pair_count sees ends here.
+int begin_batch(binder_ctx* ctx, const binder_gpu_atom* candidates, size_t n_atoms, const int64_t* offs, int n_cand,
+                bool want_abs, bool want_force) {
+    ctx->last_batch_valid = false;
+    CK(ctx->cand.ensure(n_atoms * 8), "alloc candidates");
+    if (offs) CK(ctx->off.ensure((size_t)n_cand + 1), "alloc offsets");
     CK(ctx->energy.ensure(n_cand), "alloc energy");
     if (want_abs) CK(ctx->energy_abs.ensure(n_cand), "alloc energy");
-    if ((s = clear_err(ctx))) return s;
+    if (want_force) CK(ctx->force.ensure(3 * n_atoms), "alloc force");
+    CK(ctx->errf.ensure(1), "alloc err");
+    CK(ctx->h_energy.ensure(2 * (size_t)n_cand), "alloc host");
+    CK(ctx->h_err.ensure(1), "alloc host err");
+    if (n_atoms)
+        CK(cudaMemcpyAsync(ctx->cand.p, candidates, n_atoms * sizeof(binder_gpu_atom), cudaMemcpyHostToDevice,
+                           ctx->stream),
+           "candidates H2D");
+    if (offs)
+        CK(cudaMemcpyAsync(ctx->off.p, offs, ((size_t)n_cand + 1) * sizeof(int64_t), cudaMemcpyHostToDevice,
+                           ctx->stream),
+           "offsets H2D");
+    return clear_err(ctx);
+}
+
+// Score the batch of begin_batch (n_ab atoms per candidate, or ragged when n_ab = 0)
+// against the drop-in antigen.
+int score_resident_batch(binder_ctx* ctx, int n_cand, long long n_ab, bool want_abs) {
     ScoreOut o{ctx->energy.p, want_abs ? ctx->energy_abs.p : nullptr, nullptr, nullptr, ctx->errf.p};
     launch_score_flat(ctx->stream, ctx->cand.p, n_ab ? nullptr : ctx->off.p, n_ab, n_cand, ctx->d_dropin_view.p,
                       nullptr, ctx->params.accumulate, o, grid_ctas(ctx, n_cand));
@@ -610,12 +628,8 @@ int score_batch_common(binder_ctx* ctx, const binder_atom_cloud* antigen, const 
     if (!candidates) return fail(ctx, BINDER_ERR_ARG, "candidates is NULL");
     if (out_cap < n_cand) return fail(ctx, BINDER_ERR_CAPACITY, "out_cap %zu < n_cand %zu", out_cap, n_cand);
     if (n_cand > (size_t)INT32_MAX) return fail(ctx, BINDER_ERR_ARG, "too many candidates");
-    if ((s = validate_cloud(ctx, antigen, "antigen"))) return s;
-    const size_t used = n_cand * n_ab;
-    CK(ctx->cand.ensure(used * 8), "alloc candidates");
-    CK(cudaMemcpyAsync(ctx->cand.p, candidates, used * sizeof(binder_gpu_atom), cudaMemcpyHostToDevice, ctx->stream),
-       "candidates H2D");
-    if ((s = ensure_dropin(ctx, antigen))) return s;  // while the candidates are copied
+    if ((s = ensure_dropin(ctx, antigen))) return s;
+    if ((s = begin_batch(ctx, candidates, n_cand * n_ab, nullptr, (int)n_cand, out_abs != nullptr, false))) return s;
     if ((s = score_resident_batch(ctx, (int)n_cand, (long long)n_ab, out_abs != nullptr))) return s;
     return fetch_energies(ctx, (int)n_cand, out64, out_abs, out32);
 }
@@ -806,14 +820,8 @@ int binder_score_batch_ragged(binder_ctx* ctx, const binder_atom_cloud* antigen,
         if (offsets[c + 1] < offsets[c]) return fail(ctx, BINDER_ERR_ARG, "offsets must be non-decreasing");
     const size_t n_atoms = (size_t)offsets[n_cand];
     if (n_atoms && !candidates) return fail(ctx, BINDER_ERR_ARG, "candidates is NULL");
-    if ((s = validate_cloud(ctx, antigen, "antigen"))) return s;
-    CK(ctx->cand.ensure(n_atoms * 8), "alloc candidates");
-    if (n_atoms)
-        CK(cudaMemcpyAsync(ctx->cand.p, candidates, n_atoms * sizeof(binder_gpu_atom), cudaMemcpyHostToDevice,
-                           ctx->stream),
-           "candidates H2D");
     if ((s = ensure_dropin(ctx, antigen))) return s;
-    if ((s = upload(ctx, ctx->off, (const long long*)offsets, n_cand + 1, "offsets H2D"))) return s;
+    if ((s = begin_batch(ctx, candidates, n_atoms, offsets, (int)n_cand, out_abs != nullptr, false))) return s;
     if ((s = score_resident_batch(ctx, (int)n_cand, 0, out_abs != nullptr))) return s;
     return fetch_energies(ctx, (int)n_cand, out, out_abs, nullptr);
 }
@@ -968,20 +976,12 @@ int binder_forces_allatom(binder_ctx* ctx, const binder_atom_cloud* antigen, con
     for (size_t c = 0; c < n_cand; ++c)
         if (offsets[c + 1] < offsets[c]) return fail(ctx, BINDER_ERR_ARG, "offsets must be non-decreasing");
     const size_t n_atoms = (size_t)offsets[n_cand];
-    if ((s = validate_cloud(ctx, antigen, "antigen"))) return s;
-    CK(ctx->cand.ensure(n_atoms * 8), "alloc");
-    if (n_atoms)
-        CK(cudaMemcpyAsync(ctx->cand.p, candidates, n_atoms * 32, cudaMemcpyHostToDevice, ctx->stream), "H2D");
     if ((s = ensure_dropin(ctx, antigen))) return s;
-    if ((s = upload(ctx, ctx->off, (const long long*)offsets, n_cand + 1, "offsets H2D"))) return s;
-    CK(ctx->energy.ensure(n_cand), "alloc");
-    CK(ctx->force.ensure(3 * n_atoms), "alloc");
-    if ((s = clear_err(ctx))) return s;
+    if ((s = begin_batch(ctx, candidates, n_atoms, offsets, (int)n_cand, false, true))) return s;
     ScoreOut o{ctx->energy.p, nullptr, ctx->force.p, nullptr, ctx->errf.p};
     launch_score_flat(ctx->stream, ctx->cand.p, ctx->off.p, 0, (int)n_cand, ctx->d_dropin_view.p, nullptr,
                       ctx->params.accumulate, o, grid_ctas(ctx, (int)n_cand));
     LAUNCHED("score_flat_force");
-    ctx->last_batch_valid = false;
     if (n_atoms)
         CK(cudaMemcpyAsync(out_force, ctx->force.p, 3 * n_atoms * 4, cudaMemcpyDeviceToHost, ctx->stream), "D2H");
     return fetch_energies(ctx, (int)n_cand, out_e, nullptr, nullptr);
