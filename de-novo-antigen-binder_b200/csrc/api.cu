@@ -124,7 +124,7 @@ struct Antigen {
     GridBuf grid;
     DBuf<float4> pq, prm, box;
     DBuf<float> cax, cay, caz;
-    DBuf<uint8_t> caa;
+    DBuf<uint8_t> caa, ca_aa;
     GridBuf ca_grid;
     DBuf<float4> ca_pq, ca_prm, ca_atom, ca_atom_prm;
     DBuf<int4> ca_cell;
@@ -520,12 +520,15 @@ int build_antigen_ca(binder_ctx* ctx, Antigen& A, const float* x, const float* y
     CK(A.ca_pq.ensure(n), "ca alloc");
     CK(A.ca_prm.ensure(n), "ca alloc");
     CK(A.ca_cell.ensure(n), "ca alloc");
+    CK(A.ca_aa.ensure(n), "ca alloc");
     launch_gather_ca(ctx->stream, A.ca_grid.sorted_idx.p, (int)n, A.cax.p, A.cay.p, A.caz.p, A.caa.p,
-                     ctx->d_res_tab.p, A.ca_grid.view.inv, A.ca_pq.p, A.ca_prm.p, A.ca_cell.p);
+                     ctx->d_res_tab.p, A.ca_grid.view.inv, A.ca_pq.p, A.ca_prm.p, A.ca_cell.p,
+                     A.ca_aa.p);
     if (n > 0) LAUNCHED("gather_ca");
     A.view.ca_pq = A.ca_pq.p;
     A.view.ca_prm = A.ca_prm.p;
     A.view.ca_cell = A.ca_cell.p;
+    A.view.ca_aa = A.ca_aa.p;
     A.view.res_aa = A.caa.p;
     A.view.ca_grid = A.ca_grid.view;
     A.view.n_res = (int)n;

@@ -180,6 +180,7 @@ struct AgView {
     const float4* ca_pq;   // x, y, z, residue-level charge (atom.rs:55-63)
     const float4* ca_prm;  // residue-level epsilon, sigma, hydrophobic, 0
     const int4* ca_cell;   // CA-grid cell of each sorted Calpha
+    const uint8_t* ca_aa;  // amino acid of each sorted Calpha
     GridView ca_grid;
     // Calpha atoms in residue order with their AMBER parameters (diffusion.rs:440-446)
     const float4* ca_atom;      // x, y, z, partial charge

@@ -76,7 +76,6 @@ template <bool FV>
 constexpr float AN_SKIN = FV ? 4.0f : 2.0f;
 template <bool FV>
 constexpr float AN_SKIN_MAX = FV ? 8.0f : 4.0f;
-constexpr int EL = 8;                                // lanes per Calpha energy (ACC = double)
 constexpr int MASK_WORDS = ANNEAL_MAX_RES / 32;      // residue bit masks of a candidate
 constexpr int AN_IN = 32;                            // in-cutoff entries of the force a residue holds per round
 constexpr int AG_STAGE_MAX = 1024;                   // antigen Calphas staged in shared memory
@@ -85,14 +84,11 @@ enum : int { MV_NONE = 0, MV_ROT = 1, MV_MUT = 2 };
 enum : int { SEL_KEEP = 0, SEL_PROP = 1, SEL_REJ = 2, SEL_SIDE = 4 };  // SEL_SIDE: only the side chain was built
 enum : int { IS_DVALID = 0, IS_DECISION = 1, IS_CYSMV = 2, IS_NMV = 4, IS_NTASK = 5 };
 
-// What the Calpha energies read of the antigen: its Calphas' positions and amino acids
-// in list order (the CG grid's) and in scan order (list order when staged, else residue
-// order, map giving the residue of a list position).
+// What the Calpha energies read of the antigen: its Calphas in list (grid) order.
 struct AnEnv {
-    const float4 *lpos, *pos;
+    const float4* pos;
     const uint8_t* aa;
-    const float4* map;  // AgView::ca_prm (w = residue index bits), or null when list order = scan order
-    int n, np;          // antigen Calphas, Fv: partner residues
+    int n, np;  // antigen Calphas, Fv: partner residues
 };
 
 // Fixed part of a CTA's shared memory: candidates of up to RT residues, W warps, ACC
@@ -310,12 +306,22 @@ __device__ __noinline__ double ca_pair_sum(const float4 b, int bhb, const float4
     return e;
 }
 
-// Calpha energy of a Calpha at `ca` of amino acid `aa` against the scan-order Calphas,
-// in double, by one warp: two tests per lane and step, the in-cutoff ones queued and
-// their terms evaluated 32 at a time, the lanes' sums added by a butterfly (every lane
-// holds the result).
+// The double sum of a Calpha energy: the in-cutoff Calphas numbered in list (grid) order
+// (Fv: then the partner chain's), number h added to partial sum h % EL, and the partial
+// sums folded in a fixed order.  List and scan, alone or beside other tasks, give the same
+// bits (a Calpha's number does not depend on how it was found), so a run does not depend on
+// the lists that earlier launches left.
+constexpr int EL = 8;  // lanes per Calpha energy, a partial sum each
+struct ScanSum {
+    double e;  // partial sum lane % EL
+    int n;     // Calphas within the cutoff
+};
+
+// A Calpha at `ca` of amino acid `aa` against all antigen Calphas, in double, by one warp:
+// two tests per lane and step, the in-cutoff ones queued and their terms evaluated 32 at a
+// time.
 template <class L>
-__device__ __noinline__ double warp_scan_energy(F3 ca, int aa, float2* hits) {
+__device__ __noinline__ ScanSum warp_scan_energy(F3 ca, int aa, float2* hits) {
     L& S = an_smem<L>();
     const float4* pos = S.env.pos;
     const uint8_t* ag_aa = S.env.aa;
@@ -323,7 +329,7 @@ __device__ __noinline__ double warp_scan_energy(F3 ca, int aa, float2* hits) {
     const unsigned lt = (1u << lane) - 1u;
     const float4 b = S.ca_atom[aa];
     const int bhb = S.ca_hb[aa];
-    double e = 0.0;
+    ScanSum sum = {0.0, 0};
     int cnt = 0;
 #pragma unroll 1
     for (int base = 0; base < n; base += 64) {
@@ -338,24 +344,32 @@ __device__ __noinline__ double warp_scan_energy(F3 ca, int aa, float2* hits) {
         if (in0) hits[cnt + __popc(m0 & lt)] = make_float2(r0, __int_as_float(i0));
         if (in1) hits[c0 + __popc(m1 & lt)] = make_float2(r1, __int_as_float(i1));
         cnt = c0 + __popc(m1);
-        if (cnt > 32 || base + 64 >= n) {  // room for the next step's 64, or the end
+        const bool last = base + 64 >= n;
+        if (cnt > 32 || last) {  // room for the next step's 64, or the end
             __syncwarp();
+            int done = 0;
 #pragma unroll 1
-            do {
-                const int k = max(cnt - 32, 0) + lane;
-                if (k < cnt) {
-                    const float2 h = hits[k];
-                    const int t = ag_aa[__float_as_int(h.y)];
-                    e += ca_pair_sum(b, bhb, S.ca_atom[t], S.ca_hb[t], h.x);
+            for (; done + (last ? 0 : 31) < cnt; done += 32) {
+                double t = 0.0;
+                if (done + lane < cnt) {
+                    const float2 h = hits[done + lane];
+                    const int a = ag_aa[__float_as_int(h.y)];
+                    t = ca_pair_sum(b, bhb, S.ca_atom[a], S.ca_hb[a], h.x);
                 }
-                cnt = max(cnt - 32, 0);
-            } while (cnt > 32 || (cnt > 0 && base + 64 >= n));
-            __syncwarp();
+                __syncwarp();
+#pragma unroll
+                for (int o = 0; o < 32; o += EL) sum.e += __shfl_sync(0xffffffffu, t, (lane & (EL - 1)) + o);
+            }
+            sum.n += min(done, cnt);
+            if (!last) {  // the rest, fewer than 32, to the front
+                cnt -= done;
+                const float2 h = hits[done + lane];
+                __syncwarp();
+                if (lane < cnt) hits[lane] = h;
+            }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    return e;
+    return sum;
 }
 
 // disulfide_energy (allatom.rs:155-180) over the SG atoms (topology atom 5) of the
@@ -448,13 +462,11 @@ __device__ __noinline__ bool mh_accept(ACC de, float temp, float u, double lhr) 
 // acid for a rotamer query, none for a mutation query (the network's mutation
 // outputs then depend on the environment alone, the same before and after the
 // move); one warp per row (8 rows, 8 warps).  The environment counts come from the
-// residue's Verlet list when it still covers the Calpha and the antigen is staged,
-// else from all Calphas.
+// residue's Verlet list when it still covers the Calpha, else from all Calphas.
 template <class L>
 __device__ __forceinline__ void an_tile_features(const L& S, const MlpTile& T, const int* rows_of, int base, int rows) {
     const float4* agq = S.env.pos;
     const uint8_t* ag_aa = S.env.aa;
-    const bool listed = S.env.map == nullptr;  // list order = scan order
     const float* lg1p = S.lg1p;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = warp; i < MT_ROWS; i += AN_WARPS) {
@@ -471,7 +483,7 @@ __device__ __forceinline__ void an_tile_features(const L& S, const MlpTile& T, c
         const float4 cc = S.cgcentre[r];
         const int nl = S.cgnl[r];
         const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
-        if (listed && nl <= CG_LIST_MAX && mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f)) {
+        if (nl <= CG_LIST_MAX && mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f)) {
             const uint16_t* list = S.cglist + (size_t)r * CG_LIST_MAX;
             for (int j = lane; j < nl; j += 32) {
                 const int k = list[j];
@@ -737,18 +749,30 @@ __device__ __noinline__ double task_energies(int r, int aa, bool live) {
     const float mx = ca.x - cc.x, my = ca.y - cc.y, mz = ca.z - cc.z;
     const int nl = S.cgnl[r];
     const bool ok = live && nl <= CG_LIST_MAX && mx * mx + my * my + mz * mz <= (cc.w - 0.01f) * (cc.w - 0.01f);
-    // the group's in-cutoff candidates queued (r^2, amino acid), EL at a time evaluated one
-    // per lane
-    double e = 0.0;
-    const unsigned below = (1u << gl) - 1u;
     constexpr int CAP = HIT_CAP * EL / 32;
     float2* hits = S.hits + (threadIdx.x >> 5) * HIT_CAP;
+    double e = 0.0;  // the lane's partial sum
+    int first = 0;   // number of the group's next in-cutoff Calpha
+#pragma unroll 1
+    for (unsigned m = __ballot_sync(0xffffffffu, live && !ok && gl == 0); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const F3 c = {__shfl_sync(0xffffffffu, ca.x, src), __shfl_sync(0xffffffffu, ca.y, src),
+                      __shfl_sync(0xffffffffu, ca.z, src)};
+        const ScanSum v = warp_scan_energy<L>(c, __shfl_sync(0xffffffffu, aa, src), hits);
+        if ((lane & ~(EL - 1)) == src) {
+            e = v.e;
+            first = v.n;
+        }
+    }
+    __syncwarp();
+    // the group's in-cutoff candidates queued (r^2, amino acid), EL at a time evaluated one
+    // per lane
+    const unsigned below = (1u << gl) - 1u;
     float2* q = hits + (lane / EL) * CAP;
     int n_in = 0;
     const uint16_t* list = S.cglist + r * CG_LIST_MAX;
-    const float4* lpos = S.env.lpos;
+    const float4* pos = S.env.pos;
     const uint8_t* ag_aa = S.env.aa;
-    const float4* map = S.env.map;
     const int n_list = ok ? nl : 0, n_all = n_list + (L::FV && live ? S.env.np : 0);
     const int n_max = __reduce_max_sync(0xffffffffu, n_all);
 #pragma unroll 1
@@ -765,11 +789,11 @@ __device__ __noinline__ double task_energies(int r, int aa, bool live) {
                 a = S.ptq[i];
             } else {
                 i = list[j];
-                a = lpos[i];
+                a = pos[i];
             }
             r_sq = xdist2(xsub(ca.x, a.x), xsub(ca.y, a.y), xsub(ca.z, a.z));
             in = !(r_sq > CUTOFF_SQ || r_sq < MIN_R_SQ);
-            if (in) t = L::FV && j >= n_list ? S.ptaa[i] : ag_aa[map ? __float_as_int(map[i].w) : i];
+            if (in) t = L::FV && j >= n_list ? S.ptaa[i] : ag_aa[i];
         }
         const unsigned m = __ballot_sync(0xffffffffu, in) >> (lane & ~(EL - 1)) & ((1u << EL) - 1u);
         if (in) q[n_in + __popc(m & below)] = make_float2(r_sq, __int_as_float(t));
@@ -777,27 +801,21 @@ __device__ __noinline__ double task_energies(int r, int aa, bool live) {
         const int k_max = __reduce_max_sync(0xffffffffu, n_in);
         if (k_max + EL > CAP || j0 + EL >= n_max) {
             __syncwarp();
+            const int k1 = (gl - first) & (EL - 1);  // entry k has the number first + k
 #pragma unroll 1
-            for (int k = gl; k < k_max + gl; k += EL)
-                if (k < n_in) {
-                    const float2 h = q[k];
-                    const int a = __float_as_int(h.y);
-                    e += ca_pair_sum(b, bhb, S.ca_atom[a], S.ca_hb[a], h.x);
-                }
+            for (int k0 = 0; k0 < k_max; k0 += EL) {
+                if (k0 + k1 >= n_in) continue;
+                const float2 h = q[k0 + k1];
+                const int a = __float_as_int(h.y);
+                e += ca_pair_sum(b, bhb, S.ca_atom[a], S.ca_hb[a], h.x);
+            }
             __syncwarp();
+            first += n_in;
             n_in = 0;
         }
     }
 #pragma unroll
     for (int o = EL / 2; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-#pragma unroll 1
-    for (unsigned m = __ballot_sync(0xffffffffu, live && !ok && gl == 0); m; m &= m - 1) {
-        const int src = __ffs(m) - 1;
-        const F3 c = {__shfl_sync(0xffffffffu, ca.x, src), __shfl_sync(0xffffffffu, ca.y, src),
-                      __shfl_sync(0xffffffffu, ca.z, src)};
-        const double v = warp_scan_energy<L>(c, __shfl_sync(0xffffffffu, aa, src), hits);
-        if ((lane & ~(EL - 1)) == src) e += v;
-    }
     return e;
 }
 
@@ -857,10 +875,9 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
     const bool cells_staged = staged && ncell <= C;
 #pragma unroll 2
     for (int i = tid; staged && i < nag; i += NT) {
-        const float4 prm = A.ca_prm[i];
         s_cgq[i] = A.ca_pq[i];
-        s_cgp[i] = prm;
-        s_aa[i] = A.res_aa[__float_as_int(prm.w)];  // w: residue of the i-th Calpha in grid order
+        s_cgp[i] = A.ca_prm[i];
+        s_aa[i] = A.ca_aa[i];
         if (F32) {
             const float4 q = A.ca_atom[i];
             s_agq[i] = q;
@@ -907,10 +924,8 @@ __global__ void __launch_bounds__(L::W * 32, (L::W == 8 && L::RT == 32 && !L::LR
         }
     }
     if (tid == 0) {
-        S.env.lpos = staged ? s_cgq : A.ca_pq;
-        S.env.pos = staged ? s_cgq : A.ca_atom;
-        S.env.aa = staged ? s_aa : A.res_aa;
-        S.env.map = staged ? nullptr : A.ca_prm;
+        S.env.pos = staged ? s_cgq : A.ca_pq;
+        S.env.aa = staged ? s_aa : A.ca_aa;
         S.env.n = nag;
         S.env.np = np;
         S.iscal[IS_NTASK] = S.iscal[IS_CYSMV] = 0;

@@ -49,7 +49,8 @@ void launch_gather_atoms(cudaStream_t s, const int* sorted_idx, int n, const flo
                          const float* z, const float* q, const float* rmh, const float* eps, const uint8_t* hyd,
                          const uint8_t* type, float4* pq, float4* prm, float4* box);
 void launch_gather_ca(cudaStream_t s, const int* sorted_idx, int n, const float* x, const float* y, const float* z,
-                      const uint8_t* aa, const float4* res_tab, float inv, float4* pq, float4* prm, int4* cells);
+                      const uint8_t* aa, const float4* res_tab, float inv, float4* pq, float4* prm, int4* cells,
+                      uint8_t* sorted_aa);
 void launch_nb_count(cudaStream_t s, const GridView& g, const float* px, const float* py, const float* pz, int n_q,
                      long long* counts);
 void launch_nb_fill(cudaStream_t s, const GridView& g, const int* sorted_idx, const float* px, const float* py,
