@@ -182,6 +182,7 @@ _SIGS = {
     "binder_mlp_take_log": (C.c_int, [C.c_void_p, C.POINTER(C.c_size_t)]),
     "binder_set_proposal": (C.c_int, [C.c_void_p, C.c_int, C.c_float, C.c_float]),
     "binder_selftest_wait": (C.c_int, [C.c_void_p, C.c_uint32]),
+    "binder_selftest_div": (C.c_int, [C.c_void_p, C.POINTER(C.c_int64)]),
     "binder_debug_fail_alloc": (C.c_int, [C.c_int64]),
     "binder_minimize": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p]),
     "binder_validate": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),

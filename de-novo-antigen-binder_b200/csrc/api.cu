@@ -2913,6 +2913,21 @@ int binder_debug_fail_alloc(int64_t n) {
     return BINDER_OK;
 }
 
+int binder_selftest_div(binder_ctx* ctx, int64_t* out_wrong) {
+    int s = enter(ctx);
+    if (s) return s;
+    if (!out_wrong) return fail(ctx, BINDER_ERR_ARG, "NULL out");
+    CK(ctx->pairs.ensure(1), "alloc");
+    CK(cudaMemsetAsync(ctx->pairs.p, 0, sizeof(long long), ctx->stream), "memset");
+    launch_div_selftest(ctx->stream, ctx->pairs.p, ctx->num_sms * 8);
+    LAUNCHED("division self-test");
+    long long h = 0;
+    CK(cudaMemcpyAsync(&h, ctx->pairs.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream), "D2H");
+    CK(cudaStreamSynchronize(ctx->stream), "synchronize");
+    *out_wrong = h;
+    return BINDER_OK;
+}
+
 int binder_selftest_wait(binder_ctx* ctx, uint32_t max_polls) {
     int s = enter(ctx);
     if (s) return s;

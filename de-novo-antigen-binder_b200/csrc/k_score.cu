@@ -694,6 +694,28 @@ int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, i
     return count ? 1 : 2;  // launches issued
 }
 
+// div_by (score.cuh) against the IEEE quotient for every float of its range, both signs and
+// 0, and every divisor it is used with: the EEF1 lambdas of the table and the H-bond sigma.
+__global__ void k_div_selftest(unsigned long long* __restrict__ wrong) {
+    unsigned long long bad = 0;
+    const unsigned lo = (127 - 60) << 23, hi = (127 + 4) << 23;  // 2^-60 .. 16
+#pragma unroll 1
+    for (int t = 0; t <= 16; ++t) {
+        const float d = t < 16 ? c_eef1[t].z : HB_SIGMA, y = __frcp_rn(d);
+        for (unsigned u = lo + blockIdx.x * blockDim.x + threadIdx.x; u < hi; u += gridDim.x * blockDim.x) {
+            const float r = __uint_as_float(u);
+            bad += div_by(r, d, y) != __fdiv_rn(r, d);
+            bad += div_by(-r, d, y) != __fdiv_rn(-r, d);
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) bad += div_by(0.0f, d, y) != 0.0f;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) bad += 1.0f / HB_SIGMA != __frcp_rn(HB_SIGMA);
+    if (bad) atomicAdd(wrong, bad);
+}
+void launch_div_selftest(cudaStream_t s, long long* wrong, int ctas) {
+    k_div_selftest<<<ctas, 256, 0, s>>>((unsigned long long*)wrong);
+}
+
 void launch_score_state_count(cudaStream_t s, const StateView& st, const AgView* ags, long long* pairs,
                               uint32_t* err, const StateScoreScratch& scr, int grid_ctas) {
     if (st.n_cand <= 0) return;

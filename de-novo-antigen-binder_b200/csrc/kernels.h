@@ -99,6 +99,8 @@ void launch_sum_select(cudaStream_t s, const StateView& st, const double* res_e,
 int launch_score_state(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, int full,
                        const ScoreOut& out, const StateScoreScratch& scr, int grid_ctas, int warps_per_cta,
                        const SumTopk* tk = nullptr);
+// counts the quotients of div_by (score.cuh) that differ from IEEE division over its range
+void launch_div_selftest(cudaStream_t s, long long* wrong, int ctas);
 // the full residue energies only (res_e)
 void launch_score_full_residues(cudaStream_t s, const StateView& st, const AgView* ags, int accumulate, uint32_t* err,
                                 const StateScoreScratch& scr, int grid_ctas, int warps_per_cta);

@@ -145,8 +145,8 @@ struct GroupFull {
 // exact remainder (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990).  For the five divisors this is used with (the EEF1
 // lambdas 3.15, 3.5, 3.7, 3.9 and the H-bond sigma 0.35) it equals the IEEE quotient for
-// every float |r| in [2^-60, 16) and 0 (checked exhaustively); three operations instead
-// of a division's dozen.
+// every float |r| in [2^-60, 16) and 0 (k_div_selftest compares all of them); three
+// operations instead of a division's dozen.
 __device__ __forceinline__ float div_by(float r, float d, float y) {
     const float q = __fmul_rn(r, y);
     return __fmaf_rn(__fmaf_rn(-d, q, r), y, q);
