@@ -151,11 +151,22 @@ struct FlatAtoms {
 // chain's tip to the next backbone), so that its sphere, and with it the antigen atoms it
 // queues, stays small -- groups of eight consecutive atoms straddled residues tens of
 // Angstroms apart and queued most of the antigen (1024 candidates x 170 atoms against
-// 2500: 337 us, 67 us now).  Warps take groups as they come free; each group's FP64 energy
-// has its own slot and the slots are added in order, so sums do not depend on the order
-// the groups were taken in.
+// 2500: 337 us, 67 us now).  Two more rules, whole calls of 1024 candidates x 160 atoms:
+//  * A group with an atom further than FLAT_LONG from its first, longer than any residue
+//    (Calphas in a row have no gap), is cut in two: against 6700 atoms 495 us whole, 271 in
+//    two (291 in eights), 210 in fours, which short chains and small antigens pay for
+//    (random walks of Calphas 308 in fours, 302 in two; against 130 atoms 171 and 160).
+//  * Where gaps leave fewer than four atoms a group on average (atoms in no spatial order)
+//    and the antigen is small, gaps end no group: the whole antigen is in every group's
+//    reach anyway (against 130 atoms 234 us with gaps, 173 without, in eights 181; 590
+//    atoms 270 and 247; 1000 atoms 283 and 270, but 295 and 356 when spread over a shell).
+// Warps take groups as they come free; each group's FP64 energy has its own slot and the
+// slots are added in order, so sums do not depend on the order the groups were taken in.
 constexpr int FLAT_GROUP = 14;       // atoms of the largest residue
+constexpr int FLAT_PART = 7;         // atoms of a long group's parts
 constexpr float FLAT_GAP = 4.5f;     // A between consecutive atoms of a group
+constexpr float FLAT_LONG = 12.0f;   // A from a group's first atom
+constexpr int FLAT_SMALL = 640;      // antigen atoms
 constexpr int FLAT_CHUNK = 256;      // atoms cut into groups at once
 template <int NW, bool KAHAN, bool ABS, bool COUNT>
 __global__ void __launch_bounds__(NW * 32) k_score_grouped(FlatAtoms src, int n_cand, const AgView* __restrict__ ags,
@@ -167,6 +178,7 @@ __global__ void __launch_bounds__(NW * 32) k_score_grouped(FlatAtoms src, int n_
     __shared__ GroupSmem gs[NW];
     __shared__ double s_e[FLAT_CHUNK], s_a[ABS ? FLAT_CHUNK : 1];
     __shared__ short s_start[FLAT_CHUNK + 1];
+    __shared__ bool s_long[FLAT_CHUNK];
     __shared__ int s_warp[NW], s_groups, s_next;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -178,27 +190,33 @@ __global__ void __launch_bounds__(NW * 32) k_score_grouped(FlatAtoms src, int n_
         double e = 0.0, ea = 0.0;  // thread 0
         for (long long base = a0; base < a1; base += FLAT_CHUNK) {
             const int m = (int)min((long long)FLAT_CHUNK, a1 - base);
-            // group starts: atoms far from their predecessor, and every FLAT_GROUP-th after one
+            // group starts: atoms far from their predecessor, every FLAT_GROUP-th after one,
+            // and the middles of long groups
             bool brk = false;
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto apart = [&](int i, float d) {  // atom i of the chunk further than d from this one
+                const float4 q = __ldg(&src.atoms[2 * (base + i)]);
+                const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+                return !(dx * dx + dy * dy + dz * dz <= d * d);
+            };
             if (tid < m) {
-                const float4 p = __ldg(&src.atoms[2 * (base + tid)]);
-                brk = tid == 0;
-                if (tid > 0) {
-                    const float4 q = __ldg(&src.atoms[2 * (base + tid - 1)]);
-                    const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-                    brk = !(dx * dx + dy * dy + dz * dz <= FLAT_GAP * FLAT_GAP);
-                }
+                p = __ldg(&src.atoms[2 * (base + tid)]);
+                brk = tid == 0 || apart(tid - 1, FLAT_GAP);
             }
             const unsigned mb = __ballot_sync(0xffffffffu, brk);
             if (lane == 0) s_warp[warp] = mb ? warp * 32 + 31 - __clz(mb) : -1;  // the warp's last break
+            if (tid < FLAT_CHUNK) s_long[tid] = false;
             if (tid == 0) s_next = 0;
-            __syncthreads();
+            const bool scattered = __syncthreads_count(brk) * 4 > m && Ap->n_atoms <= FLAT_SMALL;
             const unsigned below = mb & (lt | 1u << lane);
             int run = below ? warp * 32 + 31 - __clz(below) : -1;
             for (int w = warp - 1; run < 0 && w >= 0; --w) run = s_warp[w];
-            const bool start = tid < m && (tid - run) % FLAT_GROUP == 0;
-            const unsigned ms = __ballot_sync(0xffffffffu, start);
+            if (scattered) run = 0;
+            const int k = (tid - run) % FLAT_GROUP;
+            if (tid < m && k >= FLAT_PART && !scattered && apart(tid - k, FLAT_LONG)) s_long[tid - k] = true;
             __syncthreads();
+            const bool start = tid < m && (k == 0 || (k == FLAT_PART && s_long[tid - k]));
+            const unsigned ms = __ballot_sync(0xffffffffu, start);
             if (lane == 0) s_warp[warp] = __popc(ms);
             __syncthreads();
             int at = __popc(ms & lt);
