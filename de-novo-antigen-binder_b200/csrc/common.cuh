@@ -89,6 +89,11 @@ __device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
 }
 __device__ __forceinline__ float f2_lo(uint64_t v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float f2_hi(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
+// the reference's r^2 of both elements of packed differences (scalar, never fused)
+__device__ __forceinline__ void f2_dist2(uint64_t dx, uint64_t dy, uint64_t dz, float& lo, float& hi) {
+    lo = xdist2(f2_lo(dx), f2_lo(dy), f2_lo(dz));
+    hi = xdist2(f2_hi(dx), f2_hi(dy), f2_hi(dz));
+}
 // The same in packed arithmetic: a product rounded on its own is fma(d, d, -0) with a -0
 // that the code generator cannot see (it comes from memory), which no add can be fused into.
 __device__ __forceinline__ void f2_dist2(uint64_t dx, uint64_t dy, uint64_t dz, uint64_t neg0, float& lo, float& hi) {
@@ -96,18 +101,13 @@ __device__ __forceinline__ void f2_dist2(uint64_t dx, uint64_t dy, uint64_t dz, 
     lo = f2_lo(d);
     hi = f2_hi(d);
 }
-// 1 / sqrt(x) of a normal x: the instruction of rsqrtf without the scaling around it that
-// only denormal x needs (three operations each).  Every r^2 whose result is used is at
-// least MIN_R_SQ.
+// 1 / sqrt(x) of a normal x: PTX rsqrt.approx.f32 with .ftz, which by the PTX ISA differs
+// from the plain form in reading subnormal inputs as zero only.  Every r^2 whose result is
+// used is at least MIN_R_SQ.
 __device__ __forceinline__ float rsqrt_normal(float x) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-// the reference's r^2 of both elements of packed differences (scalar, never fused)
-__device__ __forceinline__ void f2_dist2(uint64_t dx, uint64_t dy, uint64_t dz, float& lo, float& hi) {
-    lo = xdist2(f2_lo(dx), f2_lo(dy), f2_lo(dz));
-    hi = xdist2(f2_hi(dx), f2_hi(dy), f2_hi(dz));
 }
 
 // Transcendentals of the Metropolis path (acceptance exp, H-bond and disulfide

@@ -138,13 +138,6 @@ __device__ __forceinline__ ChiTrig zero_trig() {
     for (int i = 0; i < 4; ++i) c.t[i] = make_float2(0.f, 1.f);
     return c;
 }
-// packed per-residue form: two float4 {sin chi1, cos chi1, sin chi2, cos chi2}, {..chi3, ..chi4}
-__device__ __forceinline__ ChiTrig unpack_trig(float4 a, float4 b) {
-    ChiTrig c;
-    c.t[0] = make_float2(a.x, a.y); c.t[1] = make_float2(a.z, a.w);
-    c.t[2] = make_float2(b.x, b.y); c.t[3] = make_float2(b.z, b.w);
-    return c;
-}
 
 // build_side_chain (rotamer.rs:439-462): atoms[0..n_bb) hold the backbone; side-chain
 // atoms are appended at n_bb.. in program order (= topology order).

@@ -29,21 +29,23 @@
 //     move follows in the same step.
 //
 // What bounds it: the chain of dependent latencies of a step (one candidate's work is
-// tiny), so every phase is arranged to be short and few (three barriers a step, four
-// more per backbone move) and many candidates share an SM.  64 x 20 residues, 300-residue
+// tiny), so every phase is arranged to be short and few (four barriers a step -- the
+// second among the energy warps only unless a Cys moves -- four more per backbone move and
+// one after a rejected one) and many candidates share an SM.  64 x 20 residues, 300-residue
 // antigen, 600 steps: 13.4 ms before (42 k cycles a step: lane-0 FP64 folds of every
 // energy, one thread scanning for Cys pairs, side chains built from divergent constant
 // tables and local memory, nine barriers), 9.5 ms so arranged, 9.1 ms with the lists kept
 // between launches and the skins below; 1024 x 20 residues, 60 steps: 7.9, 4.2, 4.1 ms.
-// What is left is about 6.5 cycles per dependent instruction (2.5 of fixed latency, 1 of shared memory, 0.8 of branches, 0.6-0.9 of instruction
-// fetch): the code is kept small -- one copy of each exponential, pair term and scan, no
+// What is left is about 6.5 cycles per dependent instruction (2.5 of fixed latency, 1 of
+// shared memory, 0.8 of branches, 0.7 of instruction fetch) and the other warps' waits for
+// the one that decides: the code is kept small -- one copy of each exponential, pair term and scan, no
 // unrolling (178 -> 122 KB) -- because several warps in different phases of unrolled code
 // waited for instructions more than for anything else (a 1024-candidate launch 5.5 -> 4.3 ms).
 //
 // Accumulation: ACC = float reproduces the reference's f32 sums bit for bit (terms
 // staged and added in antigen order by one lane); ACC = double sums the same f32 pair
-// terms in double over the lanes of a group and a fixed butterfly, and takes the
-// Metropolis test on the double energy difference.
+// terms in double in one fixed order (EL below) and takes the Metropolis test on the
+// double energy difference.
 #include <type_traits>
 
 #include "cg_list.cuh"

@@ -1,13 +1,13 @@
 // k_mlp.cu — the learned mutation / rotamer proposal network on sm_100a.
 //
-// Network: 180 environment features -> 128 (SiLU) -> 128 (SiLU) -> 25 outputs
+// Network: 180 environment features -> 256 (SiLU) -> 256 (SiLU) -> 25 outputs
 // (predicted Metropolis energy change of a mutation to each of the 20 amino acids
 // and of each of the 5 rotamers).  Weights and activations are BF16, every sum is
 // FP32.  The dense layers of training and of batched inference run on the 5th-gen
 // tensor cores: one kernel, k_gemm_tc, computes C = A * B^T for K-major BF16
 // operands with tcgen05.mma (one elected thread issues, the FP32 accumulator
 // lives in tensor memory), operands staged in shared memory in the canonical
-// no-swizzle core-matrix layout by 16-byte cp.async copies through a two-stage
+// no-swizzle core-matrix layout by 16-byte cp.async copies through a four-stage
 // ring, and the epilogue (bias, SiLU, SiLU', BF16 packing, transposed copies for
 // the weight-gradient GEMMs, split-K partials) fused on the tcgen05.ld path.
 //

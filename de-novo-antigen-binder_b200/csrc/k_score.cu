@@ -4,10 +4,12 @@
 // Replaces GpuContext::score_batch (gpu.rs:166-267) and its shader
 // (energy.wgsl:47-118), whose pair math is the LJ/Coulomb/hydrophobic part of
 // interaction_energy_atoms_breakdown (energy.rs:261-314).  The shader is brute
-// force over every antigen atom; here each candidate atom visits only the grid
-// columns whose cells can hold an antigen atom within the 10 A cutoff, so the
-// pair set is exactly the reference's (0.25 <= r^2 <= 100 with the reference's
-// f32 rounding of r^2) at a fraction of the pair tests.
+// force over every antigen atom.  Here the energy kernels take groups of nearby
+// candidate atoms (a residue, or consecutive atoms of a flat candidate) against the
+// blocks of 32 antigen atoms whose boxes come near the group (score.cuh); the force
+// kernel takes one candidate atom at a time against the grid columns in reach.  The
+// pair set is exactly the reference's (0.25 <= r^2 <= 100 with the reference's f32
+// rounding of r^2) at a fraction of the pair tests.
 //
 // Precision: f32 pair terms, per-lane compensated (Kahan) sums, FP64 warp-shuffle and
 // fixed-order FP64 sums above them (deterministic).

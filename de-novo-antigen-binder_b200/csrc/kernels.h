@@ -24,11 +24,18 @@ struct LaunchCfg {
 };
 
 // The shapes of a state of total_res residues when the caller neither set nor tuned them.
-// Gradient steps (10, us): the flat form with work-balanced tasks beats the lane groups at
-// every size -- 1280 residues 50 (4 a warp; 8 a warp 54) against 72, 9000 66 (8) against
-// 113, 20480 73 against 133, 81 k residues of 8 antigens 226 with 8 warps on the work queue
-// (297 with 4 warps static) against 376.  Scores in residue order: the cell order's better
-// locality (68 against 73 us at 20480) does not pay for its three sorting launches (17 us).
+// Gradient steps: the flat form with work-balanced tasks beats the lane groups at every
+// size, also in a first launch, whose work bands are still empty, and in long ones.  Whole
+// binder_diffuse calls of 10 / 200 steps after an upload, us:
+//   residues            4 a warp      8 a warp      8 a warp, 8 warps, queue   lane groups
+//   1280                72 / 856      72 / 1078     83 / 1112                  97 / 1017
+//   4080                81 / 1039     81 / 1003     85 / 1040                  118 / 1202
+//   9000                90 / 1215     86 / 1169     86 / 1168                  123 / 1286
+//   20480               148 / 1941    96 / 1316     98 / 1328                  147 / 1884
+//   32760               158 / 2482    147 / 2187    127 / 2045                 172 / 2463
+//   81 k, 8 antigens    540 / 9537    344 / 6096    264 / 4881                 406 / 6272
+// Scores in residue order: the cell order's better locality (68 against 73 us at 20480)
+// does not pay for its three sorting launches (17 us).
 inline LaunchCfg default_launch_cfg(int total_res) {
     LaunchCfg c;
     if (total_res < 4096) c.cg_flat = 4;

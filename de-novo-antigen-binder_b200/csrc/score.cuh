@@ -55,7 +55,6 @@ static cudaError_t score_tables_init() {
 
 struct AtomIn {
     float x, y, z, qs, rmh, se, h;
-    int type;
 };
 
 struct Acc {
