@@ -1932,12 +1932,13 @@ int binder_block(binder_ctx* ctx, int n_steps, uint32_t step0, int k, double* ou
     // the device error word accumulates over a run of enqueued blocks until fetched
     if (!ctx->async_pending && (s = clear_err(ctx))) return s;
     ctx->async_pending = async;
-    CK(ctx->energy.ensure(S.n_cand), "alloc");
-    if (k > 0) CK(ctx->topk.ensure((size_t)S.n_segments * k), "alloc");
     const bool tm = ctx->timing && ctx->ev_blocks < TIMING_RING;
     const bool pipe = async && !tm && (ctx->params.flags & BINDER_FLAG_GRAPH) && k > 0 && S.n_segments > 0 &&
                       sum_topk_fits(k, S.max_segment);
+    // (before the top-k buffer can be replaced, which a failed allocation leaves empty)
     if (ctx->sel_pending && (!pipe || ctx->sel_k != k) && (s = flush_select(ctx))) return s;
+    CK(ctx->energy.ensure(S.n_cand), "alloc");
+    if (k > 0) CK(ctx->topk.ensure((size_t)S.n_segments * k), "alloc");
     if (tm) {
         // per-phase events: the launches are issued one by one
         if ((s = enqueue_block(ctx, n_steps, k, &ctx->ev[4 * ctx->ev_blocks]))) return s;
